@@ -91,9 +91,13 @@ awq_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
   constexpr int STAGES = RST;  // name used by the shared epilogue text
   (void)STAGES;
   // Row-per-thread dequantisation (template flag ROW; decode-sized token tiles with SUBS == 4 k-blocks per raw stage):
-  // a thread owns one weight row and two whole k-blocks (128 values = one AWQ group) of every raw stage, so it
-  // waits for the raw stage once, fetches one scale / zero point per 64..128 values and touches a barrier once
-  // per 64 values: about half the per-value overhead of the half-k-block scheme used for larger token tiles.
+  // a thread owns one weight row and two whole k-blocks of every raw stage, so it waits for the raw stage once,
+  // fetches one scale / zero point per 32..64 values and touches a barrier once per 64 values: about half the
+  // per-value overhead of the half-k-block scheme used for larger token tiles.  The two halves of the warps take
+  // the k-blocks in turn (even, odd): a warp then comes back to an A stage at most AST + 2 k-blocks after the last
+  // one it knows to be read, and the parity of the stage's barrier tells that apart from a stage one round older
+  // for any AST >= 2.  Two neighbouring k-blocks per half would skip two, and with AST == 2 a warp that ran ahead
+  // could take an unread stage for a free one.
   constexpr bool kRowScheme = ROW && (SUBS == 4);
 
   extern __shared__ uint8_t smem_raw[];
@@ -258,7 +262,7 @@ awq_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
       for (int u = 0; u < 2; ++u)
 #pragma unroll
         for (int h = 0; h < 2; ++h)
-          ld_off[u][h] = SUBS * B_BYTES + row * QROW + raw_swizzle_chunk<SUBS>(row, (half * 2 + u) * 2 + h) * 16;
+          ld_off[u][h] = SUBS * B_BYTES + row * QROW + raw_swizzle_chunk<SUBS>(row, (u * 2 + half) * 2 + h) * 16;
       size_t srow[NA];
       bool rvalid[NA];
 #pragma unroll
@@ -273,7 +277,7 @@ awq_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
       auto fetch = [&](int rs) {
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-          const int kb = kb_begin + rs * SUBS + half * 2 + u;
+          const int kb = kb_begin + rs * SUBS + u * 2 + half;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int k = kb * BK + h * 32;
@@ -318,7 +322,7 @@ awq_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
         }
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-          const int sub = half * 2 + u;
+          const int sub = u * 2 + half;
           const int kb = kb_begin + rs * SUBS + sub;
           if (kb >= kb_end) break;                                       // ragged last raw stage (uniform per warp)
           const int it = rs * SUBS + sub;                                // k-blocks use the A stages round robin
