@@ -22,6 +22,7 @@
 #include "../common/tensormap.h"
 #include "comm_desc.h"
 #include "epilogue.cuh"
+#include "skinny_gemm.h"
 
 using namespace fi;
 
@@ -570,6 +571,15 @@ static int fi_awq_gemm_impl(const void* X, const void* qw, const void* scales, c
   if ((K % 64) != 0 || (ldc % 8) != 0 || (reinterpret_cast<uintptr_t>(C) & 15) != 0) return -10;
   if (group != 32 && group != 64 && group != 128 && !(group > 128 && group % 64 == 0)) return -13;
   if (dual_rows > 0 && N != dual_rows) return -11;
+  if (skinny_takes(true, false, T, K) && bn == 0 && splits == 0 && comm == nullptr && grp == nullptr && (ldx % 8) == 0 &&
+      (reinterpret_cast<uintptr_t>(X) & 15) == 0 && (reinterpret_cast<uintptr_t>(qw) & 15) == 0) {
+    SkinnyParams q = {};
+    q.x = X; q.w = qw; q.scales = scales; q.zeros = reinterpret_cast<const uint8_t*>(zeros); q.group = group;
+    q.rows_total = dual_rows > 0 ? 2 * dual_rows : N;
+    q.C = C; q.bias = bias; q.residual = residual; q.T = T; q.N = N; q.K = K; q.ldx = ldx; q.ldc = ldc;
+    q.act = act; q.dual_rows = dual_rows; q.out_fp32 = out_fp32; q.is_fp16 = dtype == 1; q.int4 = 1;
+    return skinny_gemm(q, reinterpret_cast<cudaStream_t>(stream));
+  }
   if (bn == 0) bn = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : 128;
   int w_rows = dual_rows > 0 ? 2 * dual_rows : N;
   if (grp != nullptr) w_rows = grp->num_experts * grp->expert_rows;

@@ -17,6 +17,7 @@
 #include "../common/tensormap.h"
 #include "comm_desc.h"
 #include "epilogue.cuh"
+#include "skinny_gemm.h"
 
 using namespace fi;
 
@@ -353,6 +354,11 @@ extern "C" int fi_dense_gemm_pick_bn(int T) {
   return 128;
 }
 
+static bool rope_fits(const FiRope& r, int N, int dual_rows, int out_fp32, const void* residual, int act) {
+  return (r.head_dim == 64 || r.head_dim == 128) && N == (r.num_heads + 2 * r.num_kv_heads) * r.head_dim && dual_rows == 0 &&
+         !out_fp32 && residual == nullptr && act == 0 && r.block_size > 0;
+}
+
 // C = X W^T with optional epilogue.  All pointers are device pointers; nothing is allocated.
 //   dtype: 0 = bf16, 1 = fp16 (X, W, bias; C/residual too unless out_fp32)
 //   dual_rows > 0: gated mode, W holds [gate rows; up rows], N must equal dual_rows
@@ -370,6 +376,21 @@ static int fi_dense_gemm_impl(const void* X, const void* W, void* C, const void*
   if ((K % 8) != 0 || (ldc % 8) != 0 || (reinterpret_cast<uintptr_t>(C) & 15) != 0) return -10;
   if (dual_rows > 0 && N != dual_rows) return -11;
   if (act == kActClippedSwiglu && (dual_rows <= 0 || !(act_limit > 0.f))) return -12;
+  if (skinny_takes(false, rms_eps > 0.f, T, K) && bn == 0 && splits == 0 && comm == nullptr && grp == nullptr && !w_dynamic && g_plain_trace == nullptr &&
+      (reinterpret_cast<uintptr_t>(X) & 15) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0 && (ldx % 8) == 0 && (ldw % 8) == 0) {
+    SkinnyParams q = {};
+    q.x = X; q.w = W; q.C = C; q.bias = bias; q.residual = residual;
+    q.T = T; q.N = N; q.K = K; q.ldx = ldx; q.ldw = ldw; q.ldc = ldc;
+    q.act = act; q.act_limit = act_limit; q.dual_rows = dual_rows; q.out_fp32 = out_fp32; q.is_fp16 = dtype == 1;
+    q.rms_eps = rms_eps;
+    if (rope != nullptr) {
+      if (!rope_fits(*rope, N, dual_rows, out_fp32, residual, act)) return -23;
+      q.rope_cs = rope->cos_sin; q.rope_pos = rope->positions; q.rope_slots = rope->slot_mapping;
+      q.k_cache = rope->k_cache; q.v_cache = rope->v_cache;
+      q.rope_nh = rope->num_heads; q.rope_nkv = rope->num_kv_heads; q.rope_hd = rope->head_dim; q.rope_bs = rope->block_size;
+    }
+    return skinny_gemm(q, reinterpret_cast<cudaStream_t>(stream));
+  }
   if (bn == 0) bn = fi_dense_gemm_pick_bn(T);
   const uint64_t w_rows = grp != nullptr ? static_cast<uint64_t>(grp->num_experts) * grp->expert_rows
                                          : static_cast<uint64_t>(dual_rows > 0 ? 2 * dual_rows : N);
@@ -420,9 +441,7 @@ static int fi_dense_gemm_impl(const void* X, const void* W, void* C, const void*
   p.rope_nh = p.rope_nkv = p.rope_hd = p.rope_bs = 0;
   if (rope != nullptr) {
     const int hd = rope->head_dim;
-    if ((hd != 64 && hd != 128) || N != (rope->num_heads + 2 * rope->num_kv_heads) * hd || dual_rows > 0 ||
-        out_fp32 || residual != nullptr || comm != nullptr || act != 0 || rope->block_size <= 0)
-      return -23;
+    if (comm != nullptr || !rope_fits(*rope, N, dual_rows, out_fp32, residual, act)) return -23;
     p.rope_cs = rope->cos_sin; p.rope_pos = rope->positions; p.rope_slots = rope->slot_mapping;
     p.k_cache = rope->k_cache; p.v_cache = rope->v_cache;
     p.rope_nh = rope->num_heads; p.rope_nkv = rope->num_kv_heads; p.rope_hd = hd; p.rope_bs = rope->block_size;

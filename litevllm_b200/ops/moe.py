@@ -277,7 +277,9 @@ def fused_experts(x: torch.Tensor, w_gate_up: Int4Weight, w_down: Int4Weight, id
     if w_gate_up.qw is None or w_down.qw is None:
         raise RuntimeError("expert weights are not in the device runtime layout (were they loaded on the CPU?)")
     n = T * K
-    bn = 16 if n // max(num_experts_local, 1) < 16 else 32 if n // num_experts_local < 48 else 64
+    mean = n // max(num_experts_local, 1)
+    few = mean < 16          # decode steps: an expert sees a few rows, its product streams weights (skinny_gemm.cu)
+    bn = 8 if mean < 4 else 16 if few else 32 if mean < 48 else 64
     max_tiles = min(n, num_experts_local + (n + bn - 1) // bn)
     dev = x.device
     ints = scratch("moe_ints", (2 * n + num_experts_local + 1 + 3 * max_tiles + 8) * 4, dev).view(torch.int32)
@@ -299,21 +301,30 @@ def fused_experts(x: torch.Tensor, w_gate_up: Int4Weight, w_down: Int4Weight, id
     x_sorted = acts[: n * H * esz].view(x.dtype).view(n, H)
     a_sorted = acts[n * H * esz: n * (H + inter) * esz].view(x.dtype).view(n, inter)
     y_sorted = acts[n * (H + inter) * esz: n * (2 * H + inter) * esz].view(x.dtype).view(n, H)
-    rc = lib.fi_moe_gather(_p(x), _p(sorted_route), _p(offsets), num_experts_local, n, K, H, _p(x_sorted),
-                           _DT[x.dtype], st)
-    _lib.check(rc, "fi_moe_gather")
     g = FiGrouped(_p(tile_expert), _p(tile_row0), _p(tile_rows), _p(n_tiles), max_tiles, num_experts_local,
                   2 * inter, 0)
-    sw = _p(status_word(dev))
-    rc = lib.fi_awq_gemm_grouped(_p(x_sorted), _p(w_gate_up.qw), _p(w_gate_up.scales_t), _p(w_gate_up.zeros_t),
-                                 _p(a_sorted), None, None, n, inter, H, w_gate_up.group, H, inter, _ACT[act], inter,
-                                 0, _DT[x.dtype], 1, bn, sw, st, ctypes.byref(g))
-    _lib.check(rc, "fi_awq_gemm_grouped(gate_up)")
     g2 = FiGrouped(_p(tile_expert), _p(tile_row0), _p(tile_rows), _p(n_tiles), max_tiles, num_experts_local, H, 0)
-    rc = lib.fi_awq_gemm_grouped(_p(a_sorted), _p(w_down.qw), _p(w_down.scales_t), _p(w_down.zeros_t), _p(y_sorted),
-                                 None, None, n, H, inter, w_down.group, inter, H, 0, 0, 0, _DT[x.dtype], 1, bn, sw,
-                                 st, ctypes.byref(g2))
-    _lib.check(rc, "fi_awq_gemm_grouped(down)")
+    sw = _p(status_word(dev))
+    dt = _DT[x.dtype]
+    if few and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0:
+        rc = lib.fi_awq_gemm_grouped_rows(_p(x), _p(sorted_route), K, _p(w_gate_up.qw), _p(w_gate_up.scales_t),
+                                          _p(w_gate_up.zeros_t), _p(a_sorted), n, inter, H, w_gate_up.group, x.stride(0), inter,
+                                          _ACT[act], inter, dt, bn, ctypes.byref(g), st)
+        _lib.check(rc, "fi_awq_gemm_grouped_rows(gate_up)")
+        rc = lib.fi_awq_gemm_grouped_rows(_p(a_sorted), None, 1, _p(w_down.qw), _p(w_down.scales_t), _p(w_down.zeros_t),
+                                          _p(y_sorted), n, H, inter, w_down.group, inter, H, 0, 0, dt, bn, ctypes.byref(g2), st)
+        _lib.check(rc, "fi_awq_gemm_grouped_rows(down)")
+    else:
+        rc = lib.fi_moe_gather(_p(x), _p(sorted_route), _p(offsets), num_experts_local, n, K, H, _p(x_sorted), dt, st)
+        _lib.check(rc, "fi_moe_gather")
+        rc = lib.fi_awq_gemm_grouped(_p(x_sorted), _p(w_gate_up.qw), _p(w_gate_up.scales_t), _p(w_gate_up.zeros_t),
+                                     _p(a_sorted), None, None, n, inter, H, w_gate_up.group, H, inter, _ACT[act], inter,
+                                     0, dt, 1, bn, sw, st, ctypes.byref(g))
+        _lib.check(rc, "fi_awq_gemm_grouped(gate_up)")
+        rc = lib.fi_awq_gemm_grouped(_p(a_sorted), _p(w_down.qw), _p(w_down.scales_t), _p(w_down.zeros_t), _p(y_sorted),
+                                     None, None, n, H, inter, w_down.group, inter, H, 0, 0, 0, dt, 1, bn, sw,
+                                     st, ctypes.byref(g2))
+        _lib.check(rc, "fi_awq_gemm_grouped(down)")
     out = torch.empty(T, H, dtype=x.dtype, device=dev)
     if ep_heap is not None and ep_heap.fits_low_latency(T, H):
         # expert parallel: the combine also sums the ranks' partial outputs (one kernel, peer stores)
