@@ -14,8 +14,7 @@
 // Warp roles (320 threads): warp 0 TMA producer, warp 1 MMA issuer and TMEM owner, warps 2..9 epilogue (two per TMEM
 // quarter, each draining half of the tile's tokens: with short K the epilogue is the longer half of a tile's time).
 // Barriers: full/empty per pipeline stage (running across tiles), acc_full/acc_empty per accumulator.
-// Tile order: consecutive CTAs take different weight tiles of the same 128 tokens, so the token tile
-// is shared through L2 and the weights (a few MB per layer) stay L2-resident across token tiles.
+// Tile order: see tile_at.
 // Grouped mode (mixture of experts): token tiles come from a table built on the device (expert, first row, rows) over
 // activations sorted by expert, and a tile's weights are those of its expert.
 // Every wait is bounded; a timeout records a status code and the kernel winds down normally.
@@ -37,7 +36,6 @@ using namespace fi;
 namespace {
 
 constexpr int BM = 128;   // weight rows per tile (UMMA M)
-constexpr int BN = 128;   // tokens per tile (UMMA N)
 constexpr int BK = 64;    // k-block: 64 16-bit values = one 128-byte swizzled row
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = 64 + 32 * kEpiWarps;
@@ -49,9 +47,10 @@ struct PParams {
   int T, N, K, ldc;
   int dual_rows, act, is_fp16, out_fp32;
   float act_limit;     // act 4
-  int second_off;   // weight rows between the two A tiles of a CTA: dual_rows (gated) or 128 (plain, 256-row tile)
-  int rows_per_tile;   // output rows (of N) one tile covers: 128 (gated or single) or 256
+  int second_off;   // weight rows between the two A tiles of a CTA: dual_rows (gated) or 128 (grouped plain form, 256-row tile)
+  int rows_per_tile;   // output rows (of N) one tile covers: 128, or 256 in the grouped plain form
   int n_tiles_n, n_tiles;
+  int n_group;         // weight tiles that are worked on together over all token tiles (grouped mode: all of them)
   int* status;
   // grouped mode (tile_expert != null): n_tiles is the grid's upper bound, the true number of token tiles is *tiles
   const int* tile_expert;
@@ -85,12 +84,19 @@ __device__ __forceinline__ float ld16(const void* p, size_t i, int is_fp16) {
   if (is_fp16) return __half2float(reinterpret_cast<const __half*>(p)[i]);
   return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]);
 }
-__device__ __forceinline__ void st16(void* p, size_t i, float v, int is_fp16) {
-  if (is_fp16) reinterpret_cast<__half*>(p)[i] = __float2half_rn(v);
-  else reinterpret_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16_rn(v);
+
+// Weight tile and token tile of a place in the order of work.  The tiles in flight at a time form a block of n_group weight tiles
+// by as many token tiles as there are CTAs for, so that what they share stays in L2 and matrices larger than L2 leave HBM once
+// (gated 2 x 12288 x 4096 at 2048 tokens, 201 MB of weights: 426 us a row of weight tiles at a time, 304 us in groups of 8).
+__device__ __forceinline__ void tile_at(const PParams& p, int tile, int n_token_tiles, int* n, int* tt) {
+  const int per = p.n_group * n_token_tiles;
+  const int g = tile / per, at = tile - g * per;
+  const int width = min(p.n_group, p.n_tiles_n - g * p.n_group);      // the last group may be narrower
+  *tt = at / width;
+  *n = g * p.n_group + (at - *tt * width);
 }
 
-template <int STAGES, bool DUAL>
+template <int STAGES, bool DUAL, int BN>      // BN: tokens per tile (UMMA N)
 __global__ void __launch_bounds__(kThreads)
 dense_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                              const PParams p) {
@@ -98,7 +104,8 @@ dense_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
   constexpr int B_BYTES = BN * 128;
   constexpr int STAGE_BYTES = A_BYTES * (DUAL ? 2 : 1) + B_BYTES;
   constexpr int ACC_COLS = DUAL ? 2 * BN : BN;          // TMEM columns of one accumulator (gate | up)
-  constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;          // two accumulators: 256 or 512 columns
+  constexpr uint32_t TMEM_COLS = 2 * ACC_COLS <= 128 ? 128 : 2 * ACC_COLS <= 256 ? 256 : 512;     // two accumulators
+  static_assert(2 * ACC_COLS <= 512 && BN % 32 == 0, "accumulators fit, epilogue halves are whole batches of 16 tokens");
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -130,6 +137,7 @@ dense_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
   const int kb_total = (p.K + BK - 1) / BK;
   const bool grouped = p.tile_expert != nullptr;
   const int n_tiles = grouped ? *p.tiles * p.n_tiles_n : p.n_tiles;
+  const int n_token_tiles = n_tiles / p.n_tiles_n;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -138,8 +146,9 @@ dense_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
       tma_prefetch_desc(&tmap_x);
       long it = 0;
       for (int tile = blockIdx.x; tile < n_tiles && !*aborted; tile += gridDim.x) {
-        const int tt = tile / p.n_tiles_n;
-        const int n0 = (tile % p.n_tiles_n) * p.rows_per_tile + (grouped ? p.tile_expert[tt] * p.expert_rows : 0);
+        int nt, tt;
+        tile_at(p, tile, n_token_tiles, &nt, &tt);
+        const int n0 = nt * p.rows_per_tile + (grouped ? p.tile_expert[tt] * p.expert_rows : 0);
         const int t0 = grouped ? p.tile_row0[tt] : tt * BN;
         for (int kb = 0; kb < kb_total; ++kb, ++it) {
           const int s = static_cast<int>(it % STAGES);
@@ -217,9 +226,11 @@ dense_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
         break;
       }
       tc_fence_after();
-      const int n0 = (tile % p.n_tiles_n) * p.rows_per_tile;
-      const int t0 = grouped ? p.tile_row0[tile / p.n_tiles_n] : (tile / p.n_tiles_n) * BN;
-      const int t_end = grouped ? t0 + p.tile_rows[tile / p.n_tiles_n] : p.T;
+      int nt, tt;
+      tile_at(p, tile, n_token_tiles, &nt, &tt);
+      const int n0 = nt * p.rows_per_tile;
+      const int t0 = grouped ? p.tile_row0[tt] : tt * BN;
+      const int t_end = grouped ? t0 + p.tile_rows[tt] : p.T;
       const bool gated = p.dual_rows > 0;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(b * ACC_COLS);
       // Each thread owns one weight row of the accumulator (a TMEM lane) but the output is
@@ -323,23 +334,49 @@ dense_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
   }
 }
 
-template <int STAGES, bool DUAL>
+inline int sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v > 0 ? v : 148;
+  }();
+  return n;
+}
+
+template <int STAGES, bool DUAL, int BN>
 int launch(const CUtensorMap& tw, const CUtensorMap& tx, const PParams& p, cudaStream_t stream) {
-  auto kern = dense_gemm_persistent_kernel<STAGES, DUAL>;
+  auto kern = dense_gemm_persistent_kernel<STAGES, DUAL, BN>;
   constexpr int smem = STAGES * (BM * 128 * (DUAL ? 2 : 1) + BN * 128) + (2 * STAGES + 4) * 8 + 16 + kEpiWarps * 16 * 32 * 4 + 1024;
+  static_assert(smem <= 227 * 1024, "shared memory of one SM");
   {
     cudaError_t e = fi::ensure_dynamic_smem(kern, smem);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 148;
-  }
-  const int grid = p.n_tiles < sms ? p.n_tiles : sms;
+  const int grid = p.n_tiles < sm_count() ? p.n_tiles : sm_count();
   return static_cast<int>(launch_kernel(kern, dim3(grid), dim3(kThreads), smem, stream, 0, tw, tx, p));
+}
+
+// Tile of a product: 128 output rows x `tokens`, whichever costs least over the waves of tiles that the SMs need: waves x tokens
+// x relative time per row and token.  The times are from full waves (N = 6144, K = 4096, 4096 tokens: 0.81 us per 1000 rows and
+// tokens of a wave with 256 tokens, 0.82 with 192, 0.89 with 160, 0.94 with 128, 1.06 with 96, 1.27 with 64; one tile of 256 x 128
+// took 0.85).  us before (256 x 128 always) and now: N = 2560, K = 2048: 25.2 -> 19.1 at 1135 tokens, 38.5 -> 25.1 at 2048;
+// N = 2048, K = 5632: 42.8 -> 25.6 at 1135, 44.2 -> 42.3 at 2048; N = 6144, K = 4096: 62.2 -> 48.2, 88.7 -> 84.2.
+struct TileChoice { int tokens; float cost; };
+constexpr TileChoice kPlainTiles[] = {{256, 0.94f}, {192, 0.93f}, {160, 0.96f}, {128, 1.f}, {96, 1.13f}, {64, 1.35f}};
+constexpr TileChoice kGatedTiles[] = {{128, 1.f}, {96, 1.1f}};       // a gate and an up row for each output
+
+template <int COUNT>
+int pick_tokens(const TileChoice (&choices)[COUNT], int T, int N) {
+  int best = choices[0].tokens;
+  float best_cost = 0.f;
+  for (const TileChoice& c : choices) {
+    const long tiles = static_cast<long>((N + BM - 1) / BM) * ((T + c.tokens - 1) / c.tokens);
+    const long waves = (tiles + sm_count() - 1) / sm_count();
+    const float cost = static_cast<float>(waves * c.tokens) * c.cost;
+    if (best_cost == 0.f || cost < best_cost) { best = c.tokens; best_cost = cost; }
+  }
+  return best;
 }
 
 }  // namespace
@@ -359,26 +396,34 @@ extern "C" int fi_dense_gemm_persistent(const void* X, const void* W, void* C, c
   if (act == 4 && (dual_rows <= 0 || !(act_limit > 0.f))) return -12;
   if (out_fp32 && residual != nullptr) return -13;
   const int w_rows = dual_rows > 0 ? 2 * dual_rows : N;
+  const int tokens = dual_rows > 0 ? pick_tokens(kGatedTiles, T, N) : pick_tokens(kPlainTiles, T, N);
   CUtensorMap tw, tx;
   int r = make_tmap_2d_16bit_sw128(&tw, W, w_rows, K, ldw, BM);
   if (r != 0) return r * 100 - 1;
-  r = make_tmap_2d_16bit_sw128(&tx, X, T, K, ldx, BN);
+  r = make_tmap_2d_16bit_sw128(&tx, X, T, K, ldx, tokens);
   if (r != 0) return r * 100 - 2;
   PParams p = {};
   p.C = C; p.bias = bias; p.residual = residual;
   p.T = T; p.N = N; p.K = K; p.ldc = ldc;
   p.dual_rows = dual_rows; p.act = act; p.act_limit = act_limit; p.is_fp16 = dtype == 1; p.out_fp32 = out_fp32;
-  // plain products use a 256-row tile (two A tiles per stage against one token tile), which halves the
-  // L2 -> shared-memory traffic per FLOP; 128 x 128 tiles were L2-bandwidth-bound at ~55 % of peak
-  const bool wide = dual_rows == 0 && N > BM;
-  p.second_off = dual_rows > 0 ? dual_rows : BM;
-  p.rows_per_tile = wide ? 2 * BM : BM;
-  p.n_tiles_n = (N + p.rows_per_tile - 1) / p.rows_per_tile;
-  p.n_tiles = p.n_tiles_n * ((T + BN - 1) / BN);
+  p.second_off = dual_rows;
+  p.rows_per_tile = BM;
+  p.n_tiles_n = (N + BM - 1) / BM;
+  p.n_tiles = p.n_tiles_n * ((T + tokens - 1) / tokens);
+  // about as many weight rows as tokens in the block of tiles in flight
+  p.n_group = dual_rows > 0 ? 8 : 16;
+  if (p.n_group > p.n_tiles_n) p.n_group = p.n_tiles_n;
   p.status = status;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (dual_rows > 0 || wide) return launch<4, true>(tw, tx, p, s);
-  return launch<6, false>(tw, tx, p, s);
+  if (dual_rows > 0) return tokens == 96 ? launch<4, true, 96>(tw, tx, p, s) : launch<4, true, 128>(tw, tx, p, s);
+  switch (tokens) {
+    case 256: return launch<4, false, 256>(tw, tx, p, s);
+    case 192: return launch<5, false, 192>(tw, tx, p, s);
+    case 160: return launch<5, false, 160>(tw, tx, p, s);
+    case 128: return launch<6, false, 128>(tw, tx, p, s);
+    case 96: return launch<7, false, 96>(tw, tx, p, s);
+    default: return launch<8, false, 64>(tw, tx, p, s);
+  }
 }
 
 // Grouped form over activations sorted by expert: rows of X [n_rows, K] (pitch ldx) belong to the experts of g's tile
@@ -394,7 +439,7 @@ extern "C" int fi_dense_gemm_persistent_grouped(const void* X, const void* W, vo
   CUtensorMap tw, tx;
   int r = make_tmap_2d_16bit_sw128(&tw, W, static_cast<uint64_t>(g->num_experts) * g->expert_rows, K, K, BM);
   if (r != 0) return r * 100 - 1;
-  r = make_tmap_2d_16bit_sw128(&tx, X, n_rows, K, ldx, BN);
+  r = make_tmap_2d_16bit_sw128(&tx, X, n_rows, K, ldx, 128);
   if (r != 0) return r * 100 - 2;
   PParams p = {};
   p.C = C; p.T = n_rows; p.N = N; p.K = K; p.ldc = ldc; p.dual_rows = dual_rows; p.act = act; p.act_limit = act_limit; p.is_fp16 = dtype == 1;
@@ -403,9 +448,10 @@ extern "C" int fi_dense_gemm_persistent_grouped(const void* X, const void* W, vo
   p.rows_per_tile = wide ? 2 * BM : BM;
   p.n_tiles_n = (N + p.rows_per_tile - 1) / p.rows_per_tile;
   p.n_tiles = p.n_tiles_n * g->max_tiles;
+  p.n_group = p.n_tiles_n;
   p.tile_expert = g->tile_expert; p.tile_row0 = g->tile_row0; p.tile_rows = g->tile_rows; p.tiles = g->n_tiles;
   p.expert_rows = g->expert_rows; p.status = status;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (dual_rows > 0 || wide) return launch<4, true>(tw, tx, p, s);
-  return launch<6, false>(tw, tx, p, s);
+  if (dual_rows > 0 || wide) return launch<4, true, 128>(tw, tx, p, s);
+  return launch<6, false, 128>(tw, tx, p, s);
 }

@@ -131,8 +131,11 @@ def scratch(name: str, nbytes: int, device: torch.device) -> torch.Tensor:
 # ---------------------------------------------------------------------------- GEMM
 # prefill-sized GEMMs take the persistent kernel (FI_PERSISTENT_GEMM=0 keeps the one-tile-per-CTA kernel)
 _PERSISTENT_GEMM = os.environ.get("FI_PERSISTENT_GEMM", "1") != "0"
-_PERSISTENT_MIN_T = int(os.environ.get("FI_PERSISTENT_MIN_T", "1024"))
-# Plain (non-gated) products use it too, with 256-row tiles (FI_PERSISTENT_PLAIN=0 keeps the one-tile kernel)
+# From which number of tokens on (us, one tile per CTA / persistent): plain 2048 x 5632 16 / 19 at 128 tokens, 24 / 19 at 200, 37 / 22
+# at 600, 45 / 43 at 2048; 6144 x 4096 21 / 18, 30 / 20, 35 / 36, 104 / 86; gated 2 x 5632 x 2048 41 / 22 at 70, 45 / 36 at 600.
+_PERSISTENT_MIN_T = int(os.environ.get("FI_PERSISTENT_MIN_T", "129"))
+_PERSISTENT_MIN_T_GATED = int(os.environ.get("FI_PERSISTENT_MIN_T", "65"))
+# Plain (non-gated) products use it too, (FI_PERSISTENT_PLAIN=0 keeps the one-tile kernel)
 _PERSISTENT_PLAIN = _PERSISTENT_GEMM and os.environ.get("FI_PERSISTENT_PLAIN", "1") != "0"
 
 
@@ -208,7 +211,7 @@ def linear(x, w, bias=None, residual=None, act=None, out=None, out_dtype=None, s
         return out
     wide_out = out.dtype == torch.float32
     if _PERSISTENT_PLAIN and T >= _PERSISTENT_MIN_T and splits == 0 and bn == 0 and N % 8 == 0 \
-            and (not wide_out or residual is None):
+            and (residual is None or (not wide_out and residual.data_ptr() % 16 == 0)):
         # prefill-sized: persistent CTAs with two TMEM accumulators (epilogue overlaps the next main loop)
         rc = _lib.kernels().fi_dense_gemm_persistent(
             _p(x), _p(w), _p(out), _p(bias), _p(residual), T, N, K, x.stride(0), w.stride(0), out.stride(0),
@@ -282,7 +285,7 @@ def gated_linear(x, w_gate_up, act="silu", out=None, splits=0, bn=0, rms_eps=0.0
             y = y + bias.float()
         out.copy_(reference.apply_gated(y[:, :inter], y[:, inter:], act, act_limit))
         return out
-    if rms_eps <= 0 and _PERSISTENT_GEMM and T >= _PERSISTENT_MIN_T and splits == 0 and bn == 0 and inter % 8 == 0:
+    if rms_eps <= 0 and _PERSISTENT_GEMM and T >= _PERSISTENT_MIN_T_GATED and splits == 0 and bn == 0 and inter % 8 == 0:
         rc = _lib.kernels().fi_dense_gemm_persistent(
             _p(x), _p(w_gate_up), _p(out), _p(bias), None, T, inter, K, x.stride(0), w_gate_up.stride(0), out.stride(0),
             _ACT[act], act_limit, inter, 0, _DT[x.dtype], _p(status_word(x.device)), _stream())

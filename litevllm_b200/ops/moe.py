@@ -135,7 +135,7 @@ def stacked_linear(x: torch.Tensor, w: torch.Tensor):
             or x.stride(0) != T * x.stride(1) or x.data_ptr() % 16 or not w.is_contiguous():
         return [ops.linear(x[e], w[e]) for e in range(E)]
     out = torch.empty(E, T, N, dtype=x.dtype, device=x.device)
-    many = T >= ops._PERSISTENT_MIN_T
+    many = T >= max(1024, ops._PERSISTENT_MIN_T)
     bn = 128 if many else 16 if T <= 16 else 32 if T <= 32 else 64
     t, n = _stacked_tile_table(E, T, bn, x.device)
     at = t.data_ptr()
