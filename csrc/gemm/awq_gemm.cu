@@ -557,7 +557,64 @@ inline int make_tmap_packed(CUtensorMap* out, const void* base, uint64_t rows, u
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 
+// The weights in 16 bits, [rows, K]: the values that the dequantisers above hand to the tensor core.  A warp takes 128
+// words (1024 values) of one row; lanes read neighbouring words, so both streams are whole lines.
+template <typename T>
+__global__ void __launch_bounds__(256) int4_expand_kernel(const uint32_t* __restrict__ qw, const uint16_t* __restrict__ scales,
+                                                          const uint8_t* __restrict__ zeros, uint4* __restrict__ out, int rows,
+                                                          int words, int group) {
+  pdl_launch_dependents();
+  pdl_wait();       // the buffer may still be read by the product in front
+  const int per_row = (words + 127) / 128;
+  const long unit = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  const int row = static_cast<int>(unit / per_row);
+  if (row >= rows) return;
+  const int w0 = static_cast<int>(unit % per_row) * 128 + (threadIdx.x & 31);
+  uint32_t w[4], s[4], z[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int at = w0 + 32 * i;
+    w[i] = 0u; s[i] = 0u; z[i] = 8u;
+    if (at < words) {
+      w[i] = qw[static_cast<size_t>(row) * words + at];
+      const size_t g = static_cast<size_t>(at * 8 / group) * rows + row;
+      s[i] = scales[g];
+      if (zeros != nullptr) z[i] = zeros[g];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int at = w0 + 32 * i;
+    if (at >= words) continue;
+    const uint32_t s2 = s[i] * 0x00010001u, z2 = Pack<T>::kMagic2 + z[i] * 0x00010001u;
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      o[e] = Pack<T>::sub_mul(((w[i] >> (4 * e)) & 0x000F000Fu) | Pack<T>::kMagic2, *reinterpret_cast<const typename Pack<T>::v2*>(&z2),
+                              *reinterpret_cast<const typename Pack<T>::v2*>(&s2));
+    out[static_cast<size_t>(row) * words + at] = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
 }  // namespace
+
+// out [rows, K] (16-bit, dtype 0 bf16 / 1 fp16) = the int4 weights as 16-bit numbers.
+extern "C" int fi_int4_expand(const void* qw, const void* scales, const void* zeros, void* out, int rows, int K, int group, int dtype,
+                              void* stream) {
+  if (rows <= 0 || K <= 0) return 0;
+  if ((K % 64) != 0 || (reinterpret_cast<uintptr_t>(out) & 15) != 0) return -10;
+  if (group != 32 && group != 64 && group != 128 && !(group > 128 && group % 64 == 0)) return -13;
+  const int words = K / 8;
+  const long units = static_cast<long>(rows) * ((words + 127) / 128);
+  const dim3 grid(static_cast<unsigned>((units + 7) / 8));
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  const uint32_t* q = reinterpret_cast<const uint32_t*>(qw);
+  const uint16_t* sc = reinterpret_cast<const uint16_t*>(scales);
+  const uint8_t* z = reinterpret_cast<const uint8_t*>(zeros);
+  uint4* o = reinterpret_cast<uint4*>(out);
+  return static_cast<int>(dtype == 1 ? launch_kernel(int4_expand_kernel<__half>, grid, dim3(256), 0, s, 0, q, sc, z, o, rows, words, group)
+                                     : launch_kernel(int4_expand_kernel<__nv_bfloat16>, grid, dim3(256), 0, s, 0, q, sc, z, o, rows, words, group));
+}
 
 // C = X dequant(Wq)^T with optional epilogue.  qw/scales/zeros in the runtime layout described at
 // the top of this file.  dtype: 0 bf16, 1 fp16 (X, scales, bias, C unless out_fp32).

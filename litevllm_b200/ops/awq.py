@@ -108,6 +108,23 @@ class Int4Weight:
         return dequantize(nib, self.scales_t.t().contiguous(), zeros, self.group)
 
 
+# From this many tokens on the weights are expanded to 16 bits once per call: the fused kernel expands a tile of weights again
+# for every 128 tokens, and with two of them does little else.  us per call, fused / expanded (one B200): gated 2 x 12288 rows,
+# K = 4096: 76 / 97 at 128 tokens, 141 / 109 at 192, 778 / 357 at 2048; plain 6144 rows: 26 / 27, 42 / 28, 157 / 97; 4096 rows,
+# K = 12288: 42 / 65, 72 / 66, 268 / 201; 8192 rows, K = 2816, group 32: 23 / 28, 36 / 30, 139 / 93.
+_EXPAND_MIN_T = 129
+_EXPAND_MAX_BYTES = 1 << 30
+
+
+def _expands(T: int, w: Int4Weight, x, out, residual) -> bool:
+    """Whether a product of T tokens goes through an expanded copy: enough tokens, and operands the persistent kernel takes."""
+    return (T >= _EXPAND_MIN_T and 2 * w.N * w.K <= _EXPAND_MAX_BYTES
+            and out.shape[1] % 8 == 0 and out.stride(0) % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
+            and out.data_ptr() % 16 == 0
+            and (residual is None or (out.dtype != torch.float32 and residual.stride(0) == out.stride(0)
+                                      and residual.data_ptr() % 16 == 0)))
+
+
 def int4_linear(x: torch.Tensor, w: Int4Weight, bias=None, residual=None, act=None, gated_act=None,
                 out=None, out_dtype=None, splits: int = 0, bn: int = 0) -> torch.Tensor:
     """``x @ dequant(w).T`` (+bias, +residual) or, with ``gated_act``, ``act(x Wg^T) * (x Wu^T)`` for
@@ -130,6 +147,19 @@ def int4_linear(x: torch.Tensor, w: Int4Weight, bias=None, residual=None, act=No
     if out is None:
         out = torch.empty(T, N, dtype=out_dtype, device=x.device)
     if T == 0:
+        return out
+    if splits == 0 and bn == 0 and _expands(T, w, x, out, residual):
+        # a copy in 16 bits that this call alone uses, then the persistent product
+        dense = torch.empty(w.N, K, dtype=x.dtype, device=x.device)
+        rc = _lib.kernels().fi_int4_expand(_p(w.qw), _p(w.scales_t), _p(w.zeros_t), _p(dense), w.N, K, w.group, _DT[x.dtype],
+                                           _stream())
+        _lib.check(rc, "fi_int4_expand")
+        rc = _lib.kernels().fi_dense_gemm_persistent(
+            _p(x), _p(dense), _p(out), _p(bias), _p(residual), T, N, K, x.stride(0), K, out.stride(0),
+            _ACT[gated_act if gated_act else act], 0.0, N if gated_act else 0, 1 if out.dtype == torch.float32 else 0,
+            _DT[x.dtype], _p(status_word(x.device)), _stream())
+        _lib.check(rc, "fi_dense_gemm_persistent(int4)")
+        _count(2)
         return out
     rc = _lib.kernels().fi_awq_gemm(
         _p(x), _p(w.qw), _p(w.scales_t), _p(w.zeros_t), _p(out), _p(bias), _p(residual), T, N, K, w.group,
