@@ -20,6 +20,7 @@ from .. import ops
 from ..layers.linear import LiteLinear
 from ..layers.rope import get_cos_sin
 from ..ops import moe as moe_ops
+from ..ops import stream_norms as sn
 from ..ops.awq import Int4Weight, unpack_nibbles
 from ..parallel import state as pstate
 from ..utils.profiling import stage
@@ -111,7 +112,9 @@ class Gemma4Router(nn.Module):
 
     def forward(self, residual):
         # scale-free RMSNorm x learned scale x hidden^-0.5, then the router projection in fp32
-        x = ops.rmsnorm(residual, self.scale, self.eps, w_mode=0, out_scale=self.H ** -0.5)
+        return self.route(ops.rmsnorm(residual, self.scale, self.eps, w_mode=0, out_scale=self.H ** -0.5))
+
+    def route(self, x):
         logits = ops.linear(x, self.proj, out_dtype=torch.float32)
         return moe_ops.route(logits, self.top_k, "softmax", None, self.per_expert_scale, True, 1.0)
 
@@ -148,6 +151,11 @@ class Gemma4Experts(nn.Module):
             return Int4Weight(unpack_nibbles(q), s, None, self.group, dt)
         self.w_gate_up = build("gate_up", 2 * self.I, self.H)
         self.w_down = build("down", self.H, self.I)
+
+    def rows(self, x, ids, weights):
+        """The chosen experts' outputs before their weighted sum (one rank, CUDA)."""
+        self.finalize()
+        return moe_ops.fused_expert_rows(x, self.w_gate_up, self.w_down, ids, weights, self.e_local, self.e_lo, "gelu_tanh")
 
     def forward(self, x, ids, weights):
         self.finalize()
@@ -192,9 +200,40 @@ class Gemma4DecoderLayer(nn.Module):
         else:
             self.mlp = Gemma4MLP(arch, arch.intermediate_size, dtype, qc, p + ".mlp")
 
-    def forward(self, h, batch, kv, max_pos):
+    def _forward_fused(self, h, a, batch, carry, next_norm):
+        """Behind the attention on one GPU: the norms around the stream run in one kernel per place, and the next layer's
+        input (``carry["x"]``) leaves with the last one."""
+        eps, outs = self.input_layernorm.eps, [(self.pre_feedforward_layernorm.weight, 1.0)]
+        if self.use_moe:
+            outs += [(self.router.scale, self.router.H ** -0.5), (self.pre_feedforward_layernorm_2.weight, 1.0)]
+        h, normed = sn.stream_norms(h, eps, self.post_attention_layernorm.weight, outs, y=a)
+        nexts = [] if next_norm is None else [(next_norm, 1.0)]
+        if self.use_moe:
+            with stage("layer.moe.shared"):
+                dense = self.shared_mlp(normed[0], batch)
+            with stage("layer.moe.router"):
+                ids, w = self.router.route(normed[1])
+            with stage("layer.moe.experts"):
+                routed = self.experts.rows(normed[2], ids, w)
+            h, normed = sn.stream_norms(h, eps, self.post_feedforward_layernorm.weight, nexts,
+                                        branches=(routed, self.post_feedforward_layernorm_2.weight, dense,
+                                                  self.post_feedforward_layernorm_1.weight))
+        else:
+            with stage("layer.mlp"):
+                y = self.mlp(normed[0], batch)
+            h, normed = sn.stream_norms(h, eps, self.post_feedforward_layernorm.weight, nexts, y=y)
+        if normed:
+            carry["x"] = normed[0]
+        return h
+
+    def forward(self, h, batch, kv, max_pos, carry=None, next_norm=None):
+        """``carry``: what travels beside the stream from layer to layer (the normed input of this one, if it is there)."""
+        x = carry.pop("x", None) if carry is not None else None
         with stage("layer.attention"):
-            a = self.self_attn(self.input_layernorm(h), batch, kv, max_pos)
+            a = self.self_attn(self.input_layernorm(h) if x is None else x, batch, kv, max_pos)
+            if carry is not None and self._scalar == 1.0 and sn.takes(h) and (not self.use_moe or pstate.ep_size() == 1) \
+                    and not any(m._forward_hooks or m._forward_pre_hooks for m in self.children()):
+                return self._forward_fused(h, a, batch, carry, next_norm)
             h = ops.rmsnorm(a, self.post_attention_layernorm.weight, self.post_attention_layernorm.eps, addend=h)
         x = self.pre_feedforward_layernorm(h)
         if self.use_moe:
@@ -252,8 +291,10 @@ class Gemma4ForCausalLM(nn.Module):
 
     def forward(self, batch, kv_caches, inputs_embeds=None):
         h = inputs_embeds if inputs_embeds is not None else self.embed(batch.input_ids)
+        carry: dict = {}
         for i, layer in enumerate(self.layers):
-            h = layer(h, batch, kv_caches[i], self.max_pos)
+            following = self.layers[i + 1].input_layernorm.weight if i + 1 < len(self.layers) else None
+            h = layer(h, batch, kv_caches[i], self.max_pos, carry, following)
         last = h if batch.logits_indices is None else h.index_select(0, batch.logits_indices)
         x = self.norm(last)
         if self.tie:

@@ -259,27 +259,20 @@ def _reference_experts(x, w_gate_up: Int4Weight, w_down: Int4Weight, ids, weight
     return out.to(x.dtype)
 
 
-def fused_experts(x: torch.Tensor, w_gate_up: Int4Weight, w_down: Int4Weight, ids: torch.Tensor,
-                  weights: torch.Tensor, num_experts_local: int, e_lo: int, act: str = "gelu_tanh",
-                  residual: torch.Tensor | None = None, ep_heap=None) -> torch.Tensor:
-    """x [T, H]; stacked int4 experts (``w_gate_up``: [E_local * 2I, H], ``w_down``: [E_local * H, I]);
-    ids/weights from :func:`route` (global expert ids).  Returns sum_k w * expert(x) [+ residual]
-    over the local experts ``[e_lo, e_lo + num_experts_local)``.  With ``ep_heap`` (the symmetric
-    heap of an expert-parallel group, GPU only) the result is also summed over the ranks."""
+def fused_expert_rows(x: torch.Tensor, w_gate_up: Int4Weight, w_down: Int4Weight, ids: torch.Tensor, weights: torch.Tensor,
+                      num_experts_local: int, e_lo: int, act: str = "gelu_tanh") -> RoutedRows:
+    """:func:`fused_experts` before its sum (CUDA): the rows live in scratch until the next call on the stream."""
     T, H = x.shape
     K = ids.shape[1]
     e_hi = e_lo + num_experts_local
     inter = w_gate_up.N // (num_experts_local * 2)
-    if not x.is_cuda:
-        local = ids - e_lo
-        out = _reference_experts(x, w_gate_up, w_down, local, weights, num_experts_local, 0, num_experts_local, act)
-        return out if residual is None else (out.float() + residual.float()).to(x.dtype)
     if w_gate_up.qw is None or w_down.qw is None:
         raise RuntimeError("expert weights are not in the device runtime layout (were they loaded on the CPU?)")
     n = T * K
     mean = n // max(num_experts_local, 1)
-    few = mean < 16          # decode steps: an expert sees a few rows, its product streams weights (skinny_gemm.cu)
-    bn = 8 if mean < 4 else 16 if few else 32 if mean < 48 else 64
+    # decode steps: an expert sees a few rows, its product streams weights (skinny_gemm.cu)
+    few = mean < 16 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
+    bn = 8 if few and mean < 4 else 16 if mean < 16 else 32 if mean < 48 else 64
     max_tiles = min(n, num_experts_local + (n + bn - 1) // bn)
     dev = x.device
     ints = scratch("moe_ints", (2 * n + num_experts_local + 1 + 3 * max_tiles + 8) * 4, dev).view(torch.int32)
@@ -306,7 +299,7 @@ def fused_experts(x: torch.Tensor, w_gate_up: Int4Weight, w_down: Int4Weight, id
     g2 = FiGrouped(_p(tile_expert), _p(tile_row0), _p(tile_rows), _p(n_tiles), max_tiles, num_experts_local, H, 0)
     sw = _p(status_word(dev))
     dt = _DT[x.dtype]
-    if few and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0:
+    if few:
         rc = lib.fi_awq_gemm_grouped_rows(_p(x), _p(sorted_route), K, _p(w_gate_up.qw), _p(w_gate_up.scales_t),
                                           _p(w_gate_up.zeros_t), _p(a_sorted), n, inter, H, w_gate_up.group, x.stride(0), inter,
                                           _ACT[act], inter, dt, bn, ctypes.byref(g), st)
@@ -325,6 +318,26 @@ def fused_experts(x: torch.Tensor, w_gate_up: Int4Weight, w_down: Int4Weight, id
                                      None, None, n, H, inter, w_down.group, inter, H, 0, 0, 0, dt, 1, bn, sw,
                                      st, ctypes.byref(g2))
         _lib.check(rc, "fi_awq_gemm_grouped(down)")
+    _count(3 if few else 4)
+    return RoutedRows(y_sorted, weights, slot_of.view(T, K))
+
+
+def fused_experts(x: torch.Tensor, w_gate_up: Int4Weight, w_down: Int4Weight, ids: torch.Tensor,
+                  weights: torch.Tensor, num_experts_local: int, e_lo: int, act: str = "gelu_tanh",
+                  residual: torch.Tensor | None = None, ep_heap=None) -> torch.Tensor:
+    """x [T, H]; stacked int4 experts (``w_gate_up``: [E_local * 2I, H], ``w_down``: [E_local * H, I]);
+    ids/weights from :func:`route` (global expert ids).  Returns sum_k w * expert(x) [+ residual]
+    over the local experts ``[e_lo, e_lo + num_experts_local)``.  With ``ep_heap`` (the symmetric
+    heap of an expert-parallel group, GPU only) the result is also summed over the ranks."""
+    T, H = x.shape
+    K = ids.shape[1]
+    if not x.is_cuda:
+        local = ids - e_lo
+        out = _reference_experts(x, w_gate_up, w_down, local, weights, num_experts_local, 0, num_experts_local, act)
+        return out if residual is None else (out.float() + residual.float()).to(x.dtype)
+    routed = fused_expert_rows(x, w_gate_up, w_down, ids, weights, num_experts_local, e_lo, act)
+    y_sorted, slot_of, lib, st, sw = routed.rows, routed.slot_of, _lib.kernels(), _stream(), _p(status_word(x.device))
+    dev = x.device
     out = torch.empty(T, H, dtype=x.dtype, device=dev)
     if ep_heap is not None and ep_heap.fits_low_latency(T, H):
         # expert parallel: the combine also sums the ranks' partial outputs (one kernel, peer stores)
@@ -332,11 +345,11 @@ def fused_experts(x: torch.Tensor, w_gate_up: Int4Weight, w_down: Int4Weight, id
         rc = lib.fi_moe_combine_allreduce(_p(y_sorted), _p(slot_of), _p(weights), _p(residual), _p(out), T, K, H,
                                           _DT[x.dtype], sw, st, ctypes.byref(comm))
         _lib.check(rc, "fi_moe_combine_allreduce")
-        _count(5)
+        _count()
         return out
     rc = lib.fi_moe_combine(_p(y_sorted), _p(slot_of), _p(weights), _p(residual), _p(out), T, K, H, _DT[x.dtype], st)
     _lib.check(rc, "fi_moe_combine")
-    _count(5)
+    _count()
     if ep_heap is not None:       # too large for the low-latency slabs: library collective
         from ..parallel import state as pstate
         pstate.all_reduce(out)
