@@ -428,12 +428,18 @@ _PREFILL_TC = os.environ.get("FI_PREFILL_TC", "auto")
 _PREFILL_TC_MIN_Q = int(os.environ.get("FI_PREFILL_TC_MIN_Q", "64"))
 
 
-def pick_decode_splits(B: int, nkv: int, max_kv_len: int, sm_count: int = 148) -> int:
+def pick_decode_splits(B: int, nkv: int, max_kv_len: int, sm_count: int = 148, cluster_head: int = 0) -> int:
+    """``cluster_head``: head size of a call whose splits can form one cluster (up to eight, merged in the same launch)."""
     if _DECODE_SPLITS > 0:
         return _DECODE_SPLITS
     chunks = max(1, (max_kv_len + 63) // 64)
     ctas = max(1, B * nkv)
     want = max(1, (2 * sm_count + ctas - 1) // ctas)
+    # Few sequences: eight splits of a few more keys cost less than a second launch per layer.  us per step, more splits and a
+    # merge kernel / eight (contexts of 100 to 2040 tokens): TinyLlama 1 sequence 1161 / 932 to 1170 / 1021, 4 (19 wanted) 1126 / 1074
+    # to 1183 / 1136; 8 heads of 128 at 4 sequences (10 wanted) lose 1 to 3 %.  Heads of 256: 1 sequence (37) 832 / 805, 2 (19) lose up to 4 %.
+    if cluster_head > 0 and want >= (19 if cluster_head <= 128 else 37) and max_kv_len <= 8 * 320:
+        want = 8
     return int(max(1, min(want, chunks, 32)))
 
 
@@ -516,7 +522,8 @@ def paged_attention_decode(q, k_cache, v_cache, block_tables, seq_lens, nh, nkv,
         eff = min(max_kv_len, window) if window and window > 0 else max_kv_len
         if sigmoid is not None and sigmoid.chunk > 0:
             eff = min(eff, sigmoid.chunk)
-        splits = pick_decode_splits(B, nkv, eff)
+        splits = pick_decode_splits(B, nkv, eff, cluster_head=hd if _DECODE_MERGE == "cluster" and k_cache.shape[2] % 16 == 0
+                                    and reference.kv_mode(k_cache) < 2 else 0)
     mode = reference.kv_mode(k_cache)
     assert mode < 2 or plain, "row-scaled caches take no sinks, gates, narrow outputs or two maps"
     if mode >= 2:
