@@ -1,8 +1,10 @@
 """Decode attention with the number of splits left to the op: few sequences take one cluster of eight splits, down to contexts
 shorter than a split."""
 import pytest
+import torch
 
 from litevllm_b200 import ops
+from litevllm_b200.ops import reference
 
 
 @pytest.mark.parametrize("B,nkv,hd,context,want", [(1, 4, 64, 2112, 8), (4, 4, 64, 2112, 8), (5, 4, 64, 2112, 15), (2, 8, 128, 2112, 8),
@@ -11,3 +13,26 @@ from litevllm_b200 import ops
 def test_rule(B, nkv, hd, context, want):
     assert ops.pick_decode_splits(B, nkv, context, cluster_head=hd) == want
     assert ops.pick_decode_splits(B, nkv, context) == min(max(1, -(-296 // (B * nkv))), -(-context // 64), 32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,nh,nkv,hd", [(1, 32, 4, 64), (2, 32, 8, 128), (1, 16, 8, 256)])
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("window", [0, 1024])
+def test_few_sequences(B, nh, nkv, hd, fp8, window):
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    bs, blocks = 16, 160
+    dt = torch.float8_e4m3fn if fp8 else torch.bfloat16
+    k, v = (torch.randn(1 + B * blocks, nkv, bs, hd, generator=g, device="cuda").to(torch.bfloat16).to(dt) for _ in range(2))
+    table = (1 + torch.randperm(B * blocks, generator=g, device="cuda")).int().view(B, blocks)
+    for lens in ([1], [63], [320], [321], [2560]):
+        seq = torch.tensor((lens * B)[:B], device="cuda", dtype=torch.int32)
+        if B > 1:
+            seq[1] = 131
+        q = torch.randn(B, nh * hd, generator=g, device="cuda").to(torch.bfloat16)
+        got = ops.paged_attention_decode(q, k, v, table, seq, nh, nkv, hd, hd ** -0.5, window, 0.0, max_kv_len=2560)
+        cu = torch.arange(B + 1, dtype=torch.int32)
+        ref = reference.paged_attention(q.cpu().float(), k.cpu().float(), v.cpu().float(), table.cpu(), seq.cpu(), cu, nh, nkv, hd,
+                                        hd ** -0.5, window, 0.0)
+        # probabilities and the result are rounded to 16 bits: 2^-8 of values that average around one each
+        assert torch.all((got.float().cpu() - ref.float()).abs() <= 2.0 ** -6 * (ref.float().abs() + ref.float().abs().mean()))
