@@ -58,8 +58,9 @@ __device__ __forceinline__ float to_float(__half v) { return __half2float(v); }
 // RST raw stages (packed weights + tokens via TMA), AST dequantised A stages.
 // Packed weights are fetched SUBS k-blocks (of 64) at a time so that every weight row contributes
 // 32 * SUBS contiguous bytes per TMA box: 32-byte fragments (one k-block) kept HBM at a fraction of
-// its rate.  Decode-sized token tiles take 4 k-blocks (128 bytes per row), 64 tokens 2, larger 1.
-__host__ __device__ constexpr int raw_subs(int bn) { return bn <= 32 ? 4 : (bn <= 64 ? 2 : 1); }
+// its rate.  Token tiles of 16 and 32 take 4 k-blocks (128 bytes per row), 64 tokens 4
+// or (experts) 2, larger 1.
+__host__ __device__ constexpr int raw_subs(int bn, bool row) { return bn <= 32 || (bn <= 64 && row) ? 4 : (bn <= 64 ? 2 : 1); }
 // 16-byte chunk of row `row` where logical chunk c of the packed tile lives: the TMA swizzle mode
 // that matches the row pitch (128 B: 128B swizzle, 64 B: 64B swizzle, 32 B: none).
 template <int SUBS>
@@ -79,7 +80,7 @@ __global__ void __launch_bounds__(kAwqThreads)
 awq_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
                 const __grid_constant__ TokenMaps tmaps_x, const GemmParams p) {
   constexpr int NA = DUAL ? 2 : 1;
-  constexpr int SUBS = raw_subs(BN);          // 64-wide k-blocks per raw stage
+  constexpr int SUBS = raw_subs(BN, ROW);          // 64-wide k-blocks per raw stage
   constexpr int A_BYTES = BM * 128;           // dequantised tile of one k-block
   constexpr int QROW = 32 * SUBS;             // packed bytes per weight row and raw stage
   constexpr int Q_BYTES = BM * QROW;          // packed tile: 128 rows x 8*SUBS int32
@@ -463,20 +464,20 @@ awq_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
   }
 }
 
-template <int BN, int RST, int AST, bool DUAL>
+template <int BN, int RST, int AST, bool DUAL, bool ROW>
 constexpr int ring_bytes() {
-  return AST * (DUAL ? 2 : 1) * BM * 128 + RST * raw_subs(BN) * (BM * 32 * (DUAL ? 2 : 1) + BN * 128);
+  return AST * (DUAL ? 2 : 1) * BM * 128 + RST * raw_subs(BN, ROW) * (BM * 32 * (DUAL ? 2 : 1) + BN * 128);
 }
-template <int BN, int RST, int AST, bool DUAL>
+template <int BN, int RST, int AST, bool DUAL, bool ROW>
 constexpr int smem_bytes() {
-  return ring_bytes<BN, RST, AST, DUAL>() + (2 * RST + 2 * AST + 1) * 8 + 16 + 1024;
+  return ring_bytes<BN, RST, AST, DUAL, ROW>() + (2 * RST + 2 * AST + 1) * 8 + 16 + 1024;
 }
 
 template <typename T, int BN, int RST, int AST, bool DUAL, bool ROW = false>
 int launch(const CUtensorMap& tw, const TokenMaps& tx, GemmParams p, cudaStream_t stream) {
   auto kern = awq_gemm_kernel<T, BN, RST, AST, DUAL, ROW>;
-  constexpr int smem = smem_bytes<BN, RST, AST, DUAL>();
-  constexpr int ring = ring_bytes<BN, RST, AST, DUAL>();
+  constexpr int smem = smem_bytes<BN, RST, AST, DUAL, ROW>();
+  constexpr int ring = ring_bytes<BN, RST, AST, DUAL, ROW>();
   static_assert(BN * BM * 4 <= ring, "fp32 staging tile must fit inside the rings");
   static int max_active[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   {
@@ -528,6 +529,8 @@ inline bool row_scheme() {
   return on;
 }
 
+inline bool row64(bool grouped) { return !grouped && row_scheme(); }
+
 template <typename T, bool DUAL>
 int dispatch(int bn, const CUtensorMap& tw, const TokenMaps& tx, const GemmParams& p, cudaStream_t s) {
   switch (bn) {
@@ -535,7 +538,9 @@ int dispatch(int bn, const CUtensorMap& tw, const TokenMaps& tx, const GemmParam
     // decode-sized tiles: row-per-thread dequantisers (FI_AWQ_ROW_SCHEME=0: the older half-k-block dequantisers)
     case 16: return row_scheme() ? launch<T, 16, 2, DUAL ? 2 : 3, DUAL, true>(tw, tx, p, s) : launch<T, 16, 2, DUAL ? 2 : 3, DUAL>(tw, tx, p, s);
     case 32: return row_scheme() ? launch<T, 32, 2, DUAL ? 2 : 3, DUAL, true>(tw, tx, p, s) : launch<T, 32, 2, DUAL ? 2 : 3, DUAL>(tw, tx, p, s);
-    case 64: return launch<T, 64, 2, DUAL ? 2 : 3, DUAL>(tw, tx, p, s);
+    // 33 to 64 tokens (us before / now: 6144 x 4096 24.7 / 20.0, gated 2 x 12288 x 4096 67 / 56, 4096 x 12288 37 / 28); experts keep the
+    // smaller stages, two CTAs of which share an SM (128 experts, 768 tokens: 463 / 496)
+    case 64: return row64(p.tile_expert != nullptr) ? launch<T, 64, 2, DUAL ? 2 : 3, DUAL, true>(tw, tx, p, s) : launch<T, 64, 2, DUAL ? 2 : 3, DUAL>(tw, tx, p, s);
     default: return launch<T, 128, 3, DUAL ? 2 : 3, DUAL>(tw, tx, p, s);
   }
 }
@@ -642,7 +647,7 @@ static int fi_awq_gemm_impl(const void* X, const void* qw, const void* scales, c
   if (grp != nullptr) w_rows = grp->num_experts * grp->expert_rows;
   CUtensorMap tw;
   TokenMaps tx;
-  int r = make_tmap_packed(&tw, qw, w_rows, K / 8, raw_subs(bn));
+  int r = make_tmap_packed(&tw, qw, w_rows, K / 8, raw_subs(bn, row64(grp != nullptr)));
   if (r != 0) return r * 100 - 1;
   if (comm != nullptr && comm->ag_world > 1) {
     if (comm->ag_rows_per_rank % bn != 0) return -14;

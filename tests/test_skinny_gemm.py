@@ -39,7 +39,7 @@ def test_16_bit_with_norm(T, N, K, dtype):
         _close(ops.gated_linear(x, w, "silu", rms_eps=1e-5), y, dtype, 4.0)
 
 
-@pytest.mark.parametrize("T", [1, 5, 8, 9, 16])
+@pytest.mark.parametrize("T", [1, 5, 8, 9, 16, 33, 64])
 @pytest.mark.parametrize("N,K,group,zero", [(16, 64, 32, False), (48, 192, 64, True), (5136, 704, 32, False), (4096, 4096, 128, True),
                                             (64, 384, 128, True), (32, 576, 192, True), (48, 12288, 256, False)])
 @pytest.mark.parametrize("gated", [False, True])
