@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import torch
 from torch import nn
+from torch.nn.modules.module import _has_any_global_hook
 
 from .. import ops
 from ..layers.linear import LiteLinear
@@ -176,6 +177,19 @@ class Gemma4Experts(nn.Module):
         return out
 
 
+_NORMS_BEHIND_ATTENTION = ("post_attention_layernorm", "pre_feedforward_layernorm", "post_feedforward_layernorm",
+                           "pre_feedforward_layernorm_2", "post_feedforward_layernorm_1", "post_feedforward_layernorm_2")
+
+
+def _watched(*modules) -> bool:
+    """Whether a hook or a replaced ``forward`` hangs on the call of one of the modules."""
+    return bool(_has_any_global_hook()) or any(m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__ for m in modules)
+
+
+def _plain_norm(m, eps: float) -> bool:
+    return type(m) is RMSNormWeight and m.eps == eps and m.w_mode == 0 and not m.folded and not _watched(m)
+
+
 class Gemma4DecoderLayer(nn.Module):
     def __init__(self, arch: ModelArch, i: int, dtype, qc):
         super().__init__()
@@ -200,14 +214,30 @@ class Gemma4DecoderLayer(nn.Module):
         else:
             self.mlp = Gemma4MLP(arch, arch.intermediate_size, dtype, qc, p + ".mlp")
 
+    def _fuses(self, h) -> bool:
+        """Whether the part behind the attention may run in its fused form, which calls neither the norms nor the router and
+        the experts as modules."""
+        m = self._modules
+        norms = [m[n] for n in _NORMS_BEHIND_ATTENTION if n in m]
+        return (self._scalar == 1.0 and (not self.use_moe or (pstate.ep_size() == 1 and not _watched(m["router"], m["experts"])))
+                and all(_plain_norm(n, norms[0].eps) for n in norms)
+                and sn.takes(h, *[n.weight for n in norms], *([m["router"].scale] if self.use_moe else [])))
+
+    def norm_ahead(self, following) -> torch.Tensor | None:
+        """Weight of the first norm of the layer that follows, if that norm may run ahead of it: nobody sees or changes the
+        stream between the two layers, and nobody waits for the norm to be called."""
+        if following is None or _watched(self, following) or not _plain_norm(following.input_layernorm, self.post_feedforward_layernorm.eps):
+            return None
+        return following.input_layernorm.weight
+
     def _forward_fused(self, h, a, batch, carry, next_norm):
         """Behind the attention on one GPU: the norms around the stream run in one kernel per place, and the next layer's
-        input (``carry["x"]``) leaves with the last one."""
-        eps, outs = self.input_layernorm.eps, [(self.pre_feedforward_layernorm.weight, 1.0)]
+        input leaves with the last one, beside the stream that it was taken from (``carry``)."""
+        eps, outs = self.post_attention_layernorm.eps, [(self.pre_feedforward_layernorm.weight, 1.0)]
         if self.use_moe:
             outs += [(self.router.scale, self.router.H ** -0.5), (self.pre_feedforward_layernorm_2.weight, 1.0)]
         h, normed = sn.stream_norms(h, eps, self.post_attention_layernorm.weight, outs, y=a)
-        nexts = [] if next_norm is None else [(next_norm, 1.0)]
+        nexts = [(next_norm, 1.0)] if next_norm is not None and sn.takes(h, next_norm) else []
         if self.use_moe:
             with stage("layer.moe.shared"):
                 dense = self.shared_mlp(normed[0], batch)
@@ -223,16 +253,16 @@ class Gemma4DecoderLayer(nn.Module):
                 y = self.mlp(normed[0], batch)
             h, normed = sn.stream_norms(h, eps, self.post_feedforward_layernorm.weight, nexts, y=y)
         if normed:
-            carry["x"] = normed[0]
+            carry["from"], carry["x"] = h, normed[0]
         return h
 
     def forward(self, h, batch, kv, max_pos, carry=None, next_norm=None):
-        """``carry``: what travels beside the stream from layer to layer (the normed input of this one, if it is there)."""
-        x = carry.pop("x", None) if carry is not None else None
+        """``carry``: what travels beside the stream from layer to layer (the normed input of this one, if it is there).  It is
+        used only with the very stream that it belongs to.  ``next_norm``: weight of the norm it shall be made with."""
+        known, x = (carry.pop("from", None), carry.pop("x", None)) if carry is not None else (None, None)
         with stage("layer.attention"):
-            a = self.self_attn(self.input_layernorm(h) if x is None else x, batch, kv, max_pos)
-            if carry is not None and self._scalar == 1.0 and sn.takes(h) and (not self.use_moe or pstate.ep_size() == 1) \
-                    and not any(m._forward_hooks or m._forward_pre_hooks for m in self.children()):
+            a = self.self_attn(x if x is not None and known is h else self.input_layernorm(h), batch, kv, max_pos)
+            if carry is not None and self._fuses(h):
                 return self._forward_fused(h, a, batch, carry, next_norm)
             h = ops.rmsnorm(a, self.post_attention_layernorm.weight, self.post_attention_layernorm.eps, addend=h)
         x = self.pre_feedforward_layernorm(h)
@@ -293,8 +323,8 @@ class Gemma4ForCausalLM(nn.Module):
         h = inputs_embeds if inputs_embeds is not None else self.embed(batch.input_ids)
         carry: dict = {}
         for i, layer in enumerate(self.layers):
-            following = self.layers[i + 1].input_layernorm.weight if i + 1 < len(self.layers) else None
-            h = layer(h, batch, kv_caches[i], self.max_pos, carry, following)
+            following = self.layers[i + 1] if i + 1 < len(self.layers) else None
+            h = layer(h, batch, kv_caches[i], self.max_pos, carry, layer.norm_ahead(following))
         last = h if batch.logits_indices is None else h.index_select(0, batch.logits_indices)
         x = self.norm(last)
         if self.tie:

@@ -14,9 +14,10 @@ from . import _count, _p, _stream, _DT
 from .moe import RoutedRows
 
 
-def takes(h: torch.Tensor) -> bool:
+def takes(h: torch.Tensor, *weights: torch.Tensor) -> bool:
     return (h.is_cuda and h.dtype in (torch.bfloat16, torch.float16) and h.is_contiguous() and h.shape[1] % 8 == 0
-            and h.shape[1] <= 16384 and h.data_ptr() % 16 == 0)
+            and h.shape[1] <= 16384 and h.data_ptr() % 16 == 0
+            and all(w.dtype == h.dtype and w.is_contiguous() and w.data_ptr() % 16 == 0 for w in weights))
 
 
 def stream_norms(h: torch.Tensor, eps: float, post: torch.Tensor, outs: list[tuple[torch.Tensor, float]],
