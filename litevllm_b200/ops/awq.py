@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import torch
 
+from .. import ops
 from . import _lib, reference
 from . import _count, _p, _stream, status_word, _ACT, _DT  # noqa: F401  (shared helpers)
 
@@ -116,9 +117,11 @@ _EXPAND_MIN_T = 129
 _EXPAND_MAX_BYTES = 1 << 30
 
 
-def _expands(T: int, w: Int4Weight, x, out, residual) -> bool:
-    """Whether a product of T tokens goes through an expanded copy: enough tokens, and operands the persistent kernel takes."""
-    return (T >= _EXPAND_MIN_T and 2 * w.N * w.K <= _EXPAND_MAX_BYTES
+def _expands(T: int, w: Int4Weight, x, out, residual, gated: bool = False) -> bool:
+    """Whether a product of T tokens goes through an expanded copy: enough tokens, and operands the persistent kernel takes,
+    where the switches of that kernel (FI_PERSISTENT_*) leave it on."""
+    return (T >= max(_EXPAND_MIN_T, ops._PERSISTENT_MIN_T) and (ops._PERSISTENT_GEMM if gated else ops._PERSISTENT_PLAIN)
+            and 2 * w.N * w.K <= _EXPAND_MAX_BYTES
             and out.shape[1] % 8 == 0 and out.stride(0) % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
             and out.data_ptr() % 16 == 0
             and (residual is None or (out.dtype != torch.float32 and residual.stride(0) == out.stride(0)
@@ -148,7 +151,7 @@ def int4_linear(x: torch.Tensor, w: Int4Weight, bias=None, residual=None, act=No
         out = torch.empty(T, N, dtype=out_dtype, device=x.device)
     if T == 0:
         return out
-    if splits == 0 and bn == 0 and _expands(T, w, x, out, residual):
+    if splits == 0 and bn == 0 and _expands(T, w, x, out, residual, bool(gated_act)):
         # a copy in 16 bits that this call alone uses, then the persistent product
         dense = torch.empty(w.N, K, dtype=x.dtype, device=x.device)
         rc = _lib.kernels().fi_int4_expand(_p(w.qw), _p(w.scales_t), _p(w.zeros_t), _p(dense), w.N, K, w.group, _DT[x.dtype],
