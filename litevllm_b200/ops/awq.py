@@ -73,11 +73,12 @@ def to_runtime_layout(nib: torch.Tensor, scales: torch.Tensor, zeros: torch.Tens
 
 class Int4Weight:
     """Runtime int4 weight of one (possibly merged) linear layer."""
-    __slots__ = ("qw", "scales_t", "zeros_t", "group", "N", "K", "nib", "scales", "zeros")
+    __slots__ = ("qw", "scales_t", "zeros_t", "group", "N", "K", "nib", "scales", "zeros", "copy_fits")
 
     def __init__(self, nib, scales, zeros, group: int, dtype: torch.dtype, keep_reference: bool = False):
         self.N, self.K = nib.shape
         self.group = group
+        self.copy_fits = True       # until a copy in 16 bits found no memory (int4_linear)
         if nib.is_cuda:
             self.qw, self.scales_t, self.zeros_t = to_runtime_layout(nib, scales, zeros, dtype)
             self.nib = self.scales = self.zeros = None
@@ -91,7 +92,7 @@ class Int4Weight:
     def from_runtime(cls, qw, scales_t, zeros_t, N: int, K: int, group: int) -> "Int4Weight":
         """Wrap tensors that already are in the kernel's layout (the on-disk repack cache)."""
         w = cls.__new__(cls)
-        w.N, w.K, w.group = int(N), int(K), int(group)
+        w.N, w.K, w.group, w.copy_fits = int(N), int(K), int(group), True
         w.qw, w.scales_t, w.zeros_t = qw, scales_t, zeros_t
         w.nib = w.scales = w.zeros = None
         return w
@@ -117,11 +118,22 @@ _EXPAND_MIN_T = 129
 _EXPAND_MAX_BYTES = 1 << 30
 
 
+def _copy_of(w: Int4Weight, dtype, device) -> torch.Tensor | None:
+    """Room for the weights in 16 bits, or None where the device has none left (a cache pool that takes all of its memory):
+    such a product runs in the fused kernel, which needs no room, and so do the later ones of this weight, so that the
+    allocator does not give back all that it holds for every product of a prompt."""
+    try:
+        return torch.empty(w.N, w.K, dtype=dtype, device=device)
+    except torch.OutOfMemoryError:
+        w.copy_fits = False
+        return None
+
+
 def _expands(T: int, w: Int4Weight, x, out, residual, gated: bool = False) -> bool:
     """Whether a product of T tokens goes through an expanded copy: enough tokens, and operands the persistent kernel takes,
     where the switches of that kernel (FI_PERSISTENT_*) leave it on."""
     return (T >= max(_EXPAND_MIN_T, ops._PERSISTENT_MIN_T) and (ops._PERSISTENT_GEMM if gated else ops._PERSISTENT_PLAIN)
-            and 2 * w.N * w.K <= _EXPAND_MAX_BYTES
+            and 2 * w.N * w.K <= _EXPAND_MAX_BYTES and w.copy_fits
             and out.shape[1] % 8 == 0 and out.stride(0) % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
             and out.data_ptr() % 16 == 0
             and (residual is None or (out.dtype != torch.float32 and residual.stride(0) == out.stride(0)
@@ -151,9 +163,11 @@ def int4_linear(x: torch.Tensor, w: Int4Weight, bias=None, residual=None, act=No
         out = torch.empty(T, N, dtype=out_dtype, device=x.device)
     if T == 0:
         return out
+    dense = None
     if splits == 0 and bn == 0 and _expands(T, w, x, out, residual, bool(gated_act)):
+        dense = _copy_of(w, x.dtype, x.device)
+    if dense is not None:
         # a copy in 16 bits that this call alone uses, then the persistent product
-        dense = torch.empty(w.N, K, dtype=x.dtype, device=x.device)
         rc = _lib.kernels().fi_int4_expand(_p(w.qw), _p(w.scales_t), _p(w.zeros_t), _p(dense), w.N, K, w.group, _DT[x.dtype],
                                            _stream())
         _lib.check(rc, "fi_int4_expand")
