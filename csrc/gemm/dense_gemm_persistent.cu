@@ -30,6 +30,7 @@
 #include "../common/ptx.cuh"
 #include "../common/tensormap.h"
 #include "comm_desc.h"
+#include "routes.h"
 
 using namespace fi;
 
@@ -357,28 +358,6 @@ int launch(const CUtensorMap& tw, const CUtensorMap& tx, const PParams& p, cudaS
   return static_cast<int>(launch_kernel(kern, dim3(grid), dim3(kThreads), smem, stream, 0, tw, tx, p));
 }
 
-// Tile of a product: 128 output rows x `tokens`, whichever costs least over the waves of tiles that the SMs need: waves x tokens
-// x relative time per row and token.  The times are from full waves (N = 6144, K = 4096, 4096 tokens: 0.81 us per 1000 rows and
-// tokens of a wave with 256 tokens, 0.82 with 192, 0.89 with 160, 0.94 with 128, 1.06 with 96, 1.27 with 64; one tile of 256 x 128
-// took 0.85).  us before (256 x 128 always) and now: N = 2560, K = 2048: 25.2 -> 19.1 at 1135 tokens, 38.5 -> 25.1 at 2048;
-// N = 2048, K = 5632: 42.8 -> 25.6 at 1135, 44.2 -> 42.3 at 2048; N = 6144, K = 4096: 62.2 -> 48.2, 88.7 -> 84.2.
-struct TileChoice { int tokens; float cost; };
-constexpr TileChoice kPlainTiles[] = {{256, 0.94f}, {192, 0.93f}, {160, 0.96f}, {128, 1.f}, {96, 1.13f}, {64, 1.35f}};
-constexpr TileChoice kGatedTiles[] = {{128, 1.f}, {96, 1.1f}};       // a gate and an up row for each output
-
-template <int COUNT>
-int pick_tokens(const TileChoice (&choices)[COUNT], int T, int N) {
-  int best = choices[0].tokens;
-  float best_cost = 0.f;
-  for (const TileChoice& c : choices) {
-    const long tiles = static_cast<long>((N + BM - 1) / BM) * ((T + c.tokens - 1) / c.tokens);
-    const long waves = (tiles + sm_count() - 1) / sm_count();
-    const float cost = static_cast<float>(waves * c.tokens) * c.cost;
-    if (best_cost == 0.f || cost < best_cost) { best = c.tokens; best_cost = cost; }
-  }
-  return best;
-}
-
 }  // namespace
 
 // Prefill-sized dense GEMM (see the top of the file).  dtype: 0 bf16, 1 fp16 for X, W, bias, residual and
@@ -396,7 +375,7 @@ extern "C" int fi_dense_gemm_persistent(const void* X, const void* W, void* C, c
   if (act == 4 && (dual_rows <= 0 || !(act_limit > 0.f))) return -12;
   if (out_fp32 && residual != nullptr) return -13;
   const int w_rows = dual_rows > 0 ? 2 * dual_rows : N;
-  const int tokens = dual_rows > 0 ? pick_tokens(kGatedTiles, T, N) : pick_tokens(kPlainTiles, T, N);
+  const int tokens = persistent_tile(T, N, dual_rows > 0, sm_count()).tokens;
   CUtensorMap tw, tx;
   int r = make_tmap_2d_16bit_sw128(&tw, W, w_rows, K, ldw, BM);
   if (r != 0) return r * 100 - 1;
@@ -424,6 +403,14 @@ extern "C" int fi_dense_gemm_persistent(const void* X, const void* W, void* C, c
     case 96: return launch<7, false, 96>(tw, tx, p, s);
     default: return launch<8, false, 64>(tw, tx, p, s);
   }
+}
+
+// Whether a plain product of fewer than about a thousand tokens is faster here than in dense_gemm.cu, which splits long K over a
+// cluster where there are few tiles, and runs the tiles of a little more than one wave side by side (routes.h).  us there / here:
+// N = 128, K = 4096: 10.8 / 14.1 at 129 tokens, 14.8 / 13.9 at 768; N = 512, K = 8192: 14.6 / 22.8, 22.9 / 22.7; N = 4096, K = 512, 1000
+// tokens: 11.7 / 15.7; N = 6144, K = 2048, 640 tokens: 21.6 / 24.9; N = 2048, K = 5632: 24 / 19 at 200, 37 / 22 at 600.
+extern "C" int fi_dense_gemm_persistent_pays(int T, int N, int K) {
+  return persistent_us(T, N, K, false, sm_count()) <= one_tile_us(T, N, K, sm_count()) ? 1 : 0;
 }
 
 // Grouped form over activations sorted by expert: rows of X [n_rows, K] (pitch ldx) belong to the experts of g's tile

@@ -1,0 +1,64 @@
+// Estimates, in us, of the time that a product of many tokens takes in either of two kernels: which of them a call takes, and with
+// which tile, follows from the smaller one.  Plain host arithmetic.
+//
+// The forms follow the kernels (waves of tiles, a main loop that hides the epilogue of the tile in front, K split over a
+// cluster where there are few tiles); their numbers are fitted to one B200, products of 129 to 1000 tokens, K = 128 to 12288,
+// 64 to 32000 rows, weights cold.  Over 1485 of them choosing by the estimates takes 0.3 % longer than the better kernel each time;
+// against one_tile_us's kernel alone the products take 0.79 of the time on average, 8 of them more than 3 % longer (at most 10 %).
+// Persistent alone: 0.86, 305 of them longer, up to twice as long.
+#pragma once
+
+namespace fi {
+
+inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
+inline float larger(float a, float b) { return a > b ? a : b; }
+
+// Tile of a product in the persistent kernel: 128 output rows x `tokens`, whichever costs least over the waves of tiles that the
+// SMs need: waves x tokens x relative time per row and token.  The times are from full waves (N = 6144, K = 4096, 4096 tokens:
+// 0.81 us per 1000 rows and tokens of a wave with 256 tokens, 0.82 with 192, 0.89 with 160, 0.94 with 128, 1.06 with 96, 1.27 with
+// 64; one tile of 256 x 128 took 0.85).  us before (256 x 128 always) and now: N = 2560, K = 2048: 25.2 -> 19.1 at 1135 tokens,
+// 38.5 -> 25.1 at 2048; N = 2048, K = 5632: 42.8 -> 25.6 at 1135, 44.2 -> 42.3 at 2048; N = 6144, K = 4096: 62.2 -> 48.2,
+// 88.7 -> 84.2.
+struct TileChoice { int tokens; float cost; };
+struct PersistentTile { int tokens; float cost; int waves; };
+
+inline PersistentTile persistent_tile(int T, int N, bool gated, int sms) {
+  constexpr TileChoice kPlain[] = {{256, 0.94f}, {192, 0.93f}, {160, 0.96f}, {128, 1.f}, {96, 1.13f}, {64, 1.35f}};
+  constexpr TileChoice kGated[] = {{128, 1.f}, {96, 1.1f}};       // a gate and an up row for each output
+  const TileChoice* choices = gated ? kGated : kPlain;
+  const int count = gated ? 2 : 6;
+  PersistentTile best = {0, 0.f, 0};
+  float best_cost = 0.f;
+  for (int i = 0; i < count; ++i) {
+    const long tiles = static_cast<long>(ceil_div(N, 128)) * ceil_div(T, choices[i].tokens);
+    const long waves = (tiles + sms - 1) / sms;
+    const float cost = static_cast<float>(waves * choices[i].tokens) * choices[i].cost;
+    if (best.tokens == 0 || cost < best_cost) {
+      best = {choices[i].tokens, choices[i].cost, static_cast<int>(waves)};
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
+// dense_gemm_persistent.cu.  A lone tile is bound by its chain of k-blocks, the last epilogue is not hidden.
+inline float persistent_us(int T, int N, int K, bool gated, int sms) {
+  const PersistentTile t = persistent_tile(T, N, gated, sms);
+  const float loop = 2.2e-5f * t.tokens * t.cost * K * (gated ? 2 : 1), epilogue = 0.035f * t.tokens;
+  return 3.9f + larger(loop, 0.0021f * K) + (t.waves - 1) * larger(loop, epilogue) + epilogue;
+}
+
+// dense_gemm.cu, token tiles of 128: up to two CTAs per SM, few tiles split K over clusters of up to eight.  (Between one tile per
+// SM and the last split the persistent kernel was the faster one at every size tried.)
+inline float one_tile_us(int T, int N, int K, int sms) {
+  const int tiles = ceil_div(N, 128) * ceil_div(T, 128);
+  int split = 108 / tiles;
+  if (split > 8) split = 8;
+  if (split > K / 128) split = K / 128;
+  if (split > 1) return 6.9f + (N > 64 ? 1.6f : 0.f) + 0.175f * (tiles < 12 ? tiles : 12) + 0.0052f * K / split;
+  if (tiles <= sms) return 1e9f;
+  const float rounds = tiles <= 4 * sms ? static_cast<float>(ceil_div(tiles, 2 * sms)) : tiles / (2.f * sms);
+  return rounds * (6.8f + 0.0068f * K);
+}
+
+}  // namespace fi

@@ -9,6 +9,7 @@ from __future__ import annotations
 import math
 
 import ctypes
+import functools
 import os
 from dataclasses import dataclass
 
@@ -131,12 +132,19 @@ def scratch(name: str, nbytes: int, device: torch.device) -> torch.Tensor:
 # ---------------------------------------------------------------------------- GEMM
 # prefill-sized GEMMs take the persistent kernel (FI_PERSISTENT_GEMM=0 keeps the one-tile-per-CTA kernel)
 _PERSISTENT_GEMM = os.environ.get("FI_PERSISTENT_GEMM", "1") != "0"
-# From which number of tokens on (us, one tile per CTA / persistent): plain 2048 x 5632 16 / 19 at 128 tokens, 24 / 19 at 200, 37 / 22
-# at 600, 45 / 43 at 2048; 6144 x 4096 21 / 18, 30 / 20, 35 / 36, 104 / 86; gated 2 x 5632 x 2048 41 / 22 at 70, 45 / 36 at 600.
+# From which number of tokens on: gated products always (us, one tile per CTA / persistent: 2 x 5632 x 2048 41 / 22 at 70, 45 / 36 at
+# 600, 2.0 to 2.1 times as fast at every width from 64 to 2112 and K from 512 to 4096), plain ones from 129 tokens to 1023 where the
+# estimates of csrc/gemm/routes.h say so, and above.  A number given by FI_PERSISTENT_MIN_T holds for all sizes.
+_PERSISTENT_BY_SIZE = "FI_PERSISTENT_MIN_T" not in os.environ
 _PERSISTENT_MIN_T = int(os.environ.get("FI_PERSISTENT_MIN_T", "129"))
 _PERSISTENT_MIN_T_GATED = int(os.environ.get("FI_PERSISTENT_MIN_T", "65"))
-# Plain (non-gated) products use it too, (FI_PERSISTENT_PLAIN=0 keeps the one-tile kernel)
+# Plain (non-gated) products use it too (FI_PERSISTENT_PLAIN=0 keeps the one-tile kernel)
 _PERSISTENT_PLAIN = _PERSISTENT_GEMM and os.environ.get("FI_PERSISTENT_PLAIN", "1") != "0"
+
+
+@functools.lru_cache(maxsize=4096)
+def _persistent_pays(T: int, N: int, K: int) -> bool:
+    return T >= 1024 or not _PERSISTENT_BY_SIZE or bool(_lib.kernels().fi_dense_gemm_persistent_pays(T, N, K))
 
 
 def _rms_scaled(x, eps):
@@ -211,7 +219,7 @@ def linear(x, w, bias=None, residual=None, act=None, out=None, out_dtype=None, s
         return out
     wide_out = out.dtype == torch.float32
     if _PERSISTENT_PLAIN and T >= _PERSISTENT_MIN_T and splits == 0 and bn == 0 and N % 8 == 0 \
-            and (residual is None or (not wide_out and residual.data_ptr() % 16 == 0)):
+            and (residual is None or (not wide_out and residual.data_ptr() % 16 == 0)) and _persistent_pays(T, N, K):
         # prefill-sized: persistent CTAs with two TMEM accumulators (epilogue overlaps the next main loop)
         rc = _lib.kernels().fi_dense_gemm_persistent(
             _p(x), _p(w), _p(out), _p(bias), _p(residual), T, N, K, x.stride(0), w.stride(0), out.stride(0),
