@@ -22,6 +22,7 @@
 #include "../common/tensormap.h"
 #include "comm_desc.h"
 #include "epilogue.cuh"
+#include "routes.h"
 #include "skinny_gemm.h"
 
 using namespace fi;
@@ -619,6 +620,17 @@ extern "C" int fi_int4_expand(const void* qw, const void* scales, const void* ze
   uint4* o = reinterpret_cast<uint4*>(out);
   return static_cast<int>(dtype == 1 ? launch_kernel(int4_expand_kernel<__half>, grid, dim3(256), 0, s, 0, q, sc, z, o, rows, words, group)
                                      : launch_kernel(int4_expand_kernel<__nv_bfloat16>, grid, dim3(256), 0, s, 0, q, sc, z, o, rows, words, group));
+}
+
+// Whether a product of more than 128 tokens is faster through the copy above than in the fused kernel below (routes.h; N counts
+// outputs, of a gate and an up row each in gated mode).  us fused / expanded: gated 2 x 12288 rows, K = 4096: 76 / 97 at 128
+// tokens, 141 / 109 at 192, 778 / 357 at 2048; plain 6144 rows, K = 4096: 26 / 27, 42 / 28, 157 / 97; 256 rows, K = 8192: 18 / 24 at 129,
+// 32 / 25 at 1000; 4096 rows, K = 512: 12 / 10, 14 / 19; 12288 rows, K = 8192: 95 / 110 at 200 tokens.
+extern "C" int fi_int4_expand_pays(int T, int N, int K, int group, int gated) {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+    sms = 148;
+  return persistent_us(T, N, K, gated != 0, sms) + int4_expand_us(gated ? 2 * N : N, K, group) <= int4_fused_us(T, N, K, gated != 0, sms) ? 1 : 0;
 }
 
 // C = X dequant(Wq)^T with optional epilogue.  qw/scales/zeros in the runtime layout described at

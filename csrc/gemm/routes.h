@@ -5,7 +5,8 @@
 // cluster where there are few tiles); their numbers are fitted to one B200, products of 129 to 1000 tokens, K = 128 to 12288,
 // 64 to 32000 rows, weights cold.  Over 1485 of them choosing by the estimates takes 0.3 % longer than the better kernel each time;
 // against one_tile_us's kernel alone the products take 0.79 of the time on average, 8 of them more than 3 % longer (at most 10 %).
-// Persistent alone: 0.86, 305 of them longer, up to twice as long.
+// Persistent alone: 0.86, 305 of them longer, up to twice as long.  The int4 forms: 129 to 3000 tokens, groups of 32 and 128, gated
+// and plain, K = 256 to 16384, 64 to 12288 rows.
 #pragma once
 
 namespace fi {
@@ -60,5 +61,20 @@ inline float one_tile_us(int T, int N, int K, int sms) {
   const float rounds = tiles <= 4 * sms ? static_cast<float>(ceil_div(tiles, 2 * sms)) : tiles / (2.f * sms);
   return rounds * (6.8f + 0.0068f * K);
 }
+
+// awq_gemm.cu, token tiles of 128: each tile expands its weights again; gated tiles have an SM to themselves.
+inline float int4_fused_us(int T, int N, int K, bool gated, int sms) {
+  const int tiles = ceil_div(N, 128) * ceil_div(T, 128);
+  if (gated) return ceil_div(tiles, sms) * (18.5f + 0.0113f * K);
+  int split = 82 / tiles;
+  if (split > 8) split = 8;
+  if (split > K / 128) split = K / 128;
+  if (split > 1) return 5.9f + (N > 64 ? 3.1f : 0.f) + 0.0116f * K / split;
+  const int rounds = ceil_div(tiles, 2 * sms);
+  return 7.1f * rounds + K * (0.0059f * rounds + 0.0022f * tiles / sms);
+}
+
+// The copy in 16 bits: half a byte and the scales of each value read, two written.
+inline float int4_expand_us(int rows, int K, int group) { return 0.5f + 3.9e-7f * rows * K * (1.f + 10.f / group); }
 
 }  // namespace fi

@@ -13,6 +13,8 @@ Runtime layout (csrc/gemm/awq_gemm.cu): ``qw int32 [N, K/8]`` with pair-friendly
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from .. import ops
@@ -110,12 +112,15 @@ class Int4Weight:
         return dequantize(nib, self.scales_t.t().contiguous(), zeros, self.group)
 
 
-# From this many tokens on the weights are expanded to 16 bits once per call: the fused kernel expands a tile of weights again
-# for every 128 tokens, and with two of them does little else.  us per call, fused / expanded (one B200): gated 2 x 12288 rows,
-# K = 4096: 76 / 97 at 128 tokens, 141 / 109 at 192, 778 / 357 at 2048; plain 6144 rows: 26 / 27, 42 / 28, 157 / 97; 4096 rows,
-# K = 12288: 42 / 65, 72 / 66, 268 / 201; 8192 rows, K = 2816, group 32: 23 / 28, 36 / 30, 139 / 93.
+# From this many tokens on the weights may be expanded to 16 bits once per call: the fused kernel expands a tile of weights again
+# for every 128 tokens, and with two of them does little else.  Which sizes do: fi_int4_expand_pays, measured on both sides.
 _EXPAND_MIN_T = 129
 _EXPAND_MAX_BYTES = 1 << 30
+
+
+@functools.lru_cache(maxsize=4096)
+def _expand_pays(T: int, N: int, K: int, group: int, gated: bool) -> bool:
+    return bool(_lib.kernels().fi_int4_expand_pays(T, N, K, group, 1 if gated else 0))
 
 
 def _copy_of(w: Int4Weight, dtype, device) -> torch.Tensor | None:
@@ -137,7 +142,8 @@ def _expands(T: int, w: Int4Weight, x, out, residual, gated: bool = False) -> bo
             and out.shape[1] % 8 == 0 and out.stride(0) % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
             and out.data_ptr() % 16 == 0
             and (residual is None or (out.dtype != torch.float32 and residual.stride(0) == out.stride(0)
-                                      and residual.data_ptr() % 16 == 0)))
+                                      and residual.data_ptr() % 16 == 0))
+            and _expand_pays(T, out.shape[1], w.K, w.group, gated))
 
 
 def int4_linear(x: torch.Tensor, w: Int4Weight, bias=None, residual=None, act=None, gated_act=None,
