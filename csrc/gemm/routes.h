@@ -3,8 +3,8 @@
 //
 // The forms follow the kernels (waves of tiles, a main loop that hides the epilogue of the tile in front, K split over a
 // cluster where there are few tiles); their numbers are fitted to one B200, products of 129 to 1000 tokens, K = 128 to 12288,
-// 64 to 32000 rows, weights cold.  Over 1485 of them choosing by the estimates takes 0.3 % longer than the better kernel each time;
-// against one_tile_us's kernel alone the products take 0.79 of the time on average, 8 of them more than 3 % longer (at most 10 %).
+// 64 to 32000 rows, weights cold.  Over 1485 of them choosing by the estimates takes 0.2 % longer than the better kernel each time;
+// against one_tile_us's kernel alone the products take 0.79 of the time on average, 12 of them more than 3 % longer (at most 11 %).
 // Persistent alone: 0.86, 305 of them longer, up to twice as long.  The int4 forms: 129 to 3000 tokens, groups of 32 and 128, gated
 // and plain, K = 256 to 16384, 64 to 12288 rows.
 #pragma once
@@ -56,7 +56,10 @@ inline float one_tile_us(int T, int N, int K, int sms) {
   int split = 108 / tiles;
   if (split > 8) split = 8;
   if (split > K / 128) split = K / 128;
-  if (split > 1) return 6.9f + (N > 64 ? 1.6f : 0.f) + 0.175f * (tiles < 12 ? tiles : 12) + 0.0052f * K / split;
+  // tiles in other numbers than powers of two were 2 to 3 us slower from five on (N = 128, K = 2816: 10.6 us with 4 tiles, 13.9 with
+  // 6, 11.5 with 8)
+  const float odd = tiles > 4 && (tiles & (tiles - 1)) != 0 ? 2.f : 0.f;
+  if (split > 1) return 6.9f + (N > 64 ? 1.6f : 0.f) + 0.175f * (tiles < 12 ? tiles : 12) + odd + 0.0052f * K / split;
   if (tiles <= sms) return 1e9f;
   const float rounds = tiles <= 4 * sms ? static_cast<float>(ceil_div(tiles, 2 * sms)) : tiles / (2.f * sms);
   return rounds * (6.8f + 0.0068f * K);
