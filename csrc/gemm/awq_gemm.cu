@@ -645,8 +645,9 @@ static int fi_awq_gemm_impl(const void* X, const void* qw, const void* scales, c
   if ((K % 64) != 0 || (ldc % 8) != 0 || (reinterpret_cast<uintptr_t>(C) & 15) != 0) return -10;
   if (group != 32 && group != 64 && group != 128 && !(group > 128 && group % 64 == 0)) return -13;
   if (dual_rows > 0 && N != dual_rows) return -11;
-  if (skinny_takes(true, false, T, K) && bn == 0 && splits == 0 && comm == nullptr && grp == nullptr && (ldx % 8) == 0 &&
-      (reinterpret_cast<uintptr_t>(X) & 15) == 0 && (reinterpret_cast<uintptr_t>(qw) & 15) == 0) {
+  if (bn == 0 && splits == 0 && comm == nullptr && grp == nullptr && (ldx % 8) == 0 &&
+      (reinterpret_cast<uintptr_t>(X) & 15) == 0 && (reinterpret_cast<uintptr_t>(qw) & 15) == 0 &&
+      skinny_takes(true, false, T, N, K, dual_rows > 0)) {
     SkinnyParams q = {};
     q.x = X; q.w = qw; q.scales = scales; q.zeros = reinterpret_cast<const uint8_t*>(zeros); q.group = group;
     q.rows_total = dual_rows > 0 ? 2 * dual_rows : N;

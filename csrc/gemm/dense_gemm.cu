@@ -376,8 +376,9 @@ static int fi_dense_gemm_impl(const void* X, const void* W, void* C, const void*
   if ((K % 8) != 0 || (ldc % 8) != 0 || (reinterpret_cast<uintptr_t>(C) & 15) != 0) return -10;
   if (dual_rows > 0 && N != dual_rows) return -11;
   if (act == kActClippedSwiglu && (dual_rows <= 0 || !(act_limit > 0.f))) return -12;
-  if (skinny_takes(false, rms_eps > 0.f, T, K) && bn == 0 && splits == 0 && comm == nullptr && grp == nullptr && !w_dynamic && g_plain_trace == nullptr &&
-      (reinterpret_cast<uintptr_t>(X) & 15) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0 && (ldx % 8) == 0 && (ldw % 8) == 0) {
+  if (bn == 0 && splits == 0 && comm == nullptr && grp == nullptr && !w_dynamic && g_plain_trace == nullptr &&
+      (reinterpret_cast<uintptr_t>(X) & 15) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0 && (ldx % 8) == 0 && (ldw % 8) == 0 &&
+      skinny_takes(false, rms_eps > 0.f, T, N, K, dual_rows > 0)) {
     SkinnyParams q = {};
     q.x = X; q.w = W; q.C = C; q.bias = bias; q.residual = residual;
     q.T = T; q.N = N; q.K = K; q.ldx = ldx; q.ldw = ldw; q.ldc = ldc;

@@ -466,32 +466,42 @@ inline int sm_count() {
   return n;
 }
 
+// What a launch needs by its sizes: tokens in one piece up to kMostBytes of shared memory, beyond in segments of K that every round
+// stages again; kernels of few accumulators run two CTAs per SM where their tokens leave room.
+struct Shape { int seg, segs, smem, per_sm, blocks; };
+
+template <bool INT4, int KS, int MT, int NT, int DW>
+Shape shape_of(int tokens, int K, int tiles) {
+  constexpr int CH = INT4 ? 128 : 64, kMostBytes = 200 * 1024;
+  constexpr int fixed = (2 * kWarps * MT * NT * 8 * kRedPitch + kWarps * NT * 8) * 4;
+  const int chunks = (K + CH - 1) / CH;
+  int seg = (chunks + KS * DW - 1) / (KS * DW) * (KS * DW);
+  while (seg > KS * DW && fixed + tokens * row_units(INT4, (seg < chunks ? seg : chunks) * CH) * 16 > kMostBytes) seg -= KS * DW;
+  Shape s;
+  s.seg = seg;
+  s.segs = (chunks + seg - 1) / seg;
+  s.smem = fixed + tokens * row_units(INT4, (seg < chunks ? seg : chunks) * CH) * 16;
+  s.per_sm = MT * NT <= 2 && s.smem <= 113 * 1024 ? 2 : 1;
+  s.blocks = ((tiles + MT - 1) / MT + kWarps / KS - 1) / (kWarps / KS);
+  return s;
+}
+
 template <typename T, bool INT4, bool POST, bool RMS, int KS, int MT, int NT, int DW>
 int launch(const SkinnyParams& p, int tiles, cudaStream_t s) {
-  constexpr int CH = INT4 ? 128 : 64, GP = kWarps / KS;
   auto kern = skinny_kernel<T, INT4, POST, RMS, KS, MT, NT, DW>;
   const bool grouped = p.tile_expert != nullptr;
-  const int tokens = grouped ? p.tile_tokens : p.T;
-  constexpr int fixed = (2 * kWarps * MT * NT * 8 * kRedPitch + kWarps * NT * 8) * 4;
-  const int chunks = (p.K + CH - 1) / CH;
-  // tokens in one piece where they leave room for a neighbour on the SM, or at least fit; otherwise in segments
-  constexpr int kMost = 200 * 1024;
-  int seg = (chunks + KS * DW - 1) / (KS * DW) * (KS * DW);
-  while (seg > KS * DW && fixed + tokens * row_units(INT4, (seg < chunks ? seg : chunks) * CH) * 16 > kMost) seg -= KS * DW;
-  const int smem = fixed + tokens * row_units(INT4, (seg < chunks ? seg : chunks) * CH) * 16;
-  if (smem > 227 * 1024) return -31;
-  cudaError_t e = ensure_dynamic_smem(kern, smem > 48 * 1024 ? smem : 48 * 1024);
+  const Shape f = shape_of<INT4, KS, MT, NT, DW>(grouped ? p.tile_tokens : p.T, p.K, tiles);
+  if (f.smem > 227 * 1024) return -31;
+  cudaError_t e = ensure_dynamic_smem(kern, f.smem > 48 * 1024 ? f.smem : 48 * 1024);
   if (e != cudaSuccess) return static_cast<int>(e);
-  const int per_sm = MT * NT <= 2 && smem <= 113 * 1024 ? 2 : 1;
-  const int units = (tiles + MT - 1) / MT, blocks = (units + GP - 1) / GP;
-  int gx = blocks;
+  int gx = f.blocks;
   if (grouped) {        // about four CTAs per place over the experts that can occur
-    const int want = (4 * per_sm * sm_count() + p.max_tiles - 1) / p.max_tiles;
+    const int want = (4 * f.per_sm * sm_count() + p.max_tiles - 1) / p.max_tiles;
     if (gx > want) gx = want;
-  } else if (gx > per_sm * sm_count()) {
-    gx = per_sm * sm_count();
+  } else if (gx > f.per_sm * sm_count()) {
+    gx = f.per_sm * sm_count();
   }
-  return static_cast<int>(launch_kernel(kern, dim3(gx, grouped ? p.max_tiles : 1, 1), dim3(kSkinnyThreads), smem, s, 0, p, tiles, seg));
+  return static_cast<int>(launch_kernel(kern, dim3(gx, grouped ? p.max_tiles : 1, 1), dim3(kSkinnyThreads), f.smem, s, 0, p, tiles, f.seg));
 }
 
 // Which split of the warps.  Measured on one B200, us per launch in a captured chain, weights cold (512 tiles: N = 8192):
@@ -509,6 +519,32 @@ int int4_by_size(const SkinnyParams& p, cudaStream_t s) {
   return tiles >= 320 ? launch<T, true, POST, false, 8, 2, 1, 2>(p, tiles, s) : launch<T, true, POST, false, 8, 1, 1, 4>(p, tiles, s);
 }
 
+// Int4 layers of up to 16 tokens: against awq_gemm.cu, which splits K over clusters and stages the tokens with the weights.
+// Up to 8 tokens in one piece this kernel is 1.2 to 3 times as fast at every size tried but the shortest K under the most rows (K =
+// 256, 12288 rows: 5.8 / 6.3 us).  More tokens, and pieces, cost what follows: estimates in us of both, fitted to 1660 products
+// of 9 to 16 tokens (K = 256 to 16384, 64 to 12288 outputs).  Over 3100 products of 1 to 16 tokens choosing by them takes 0.2 % longer
+// than the better kernel each time and 0.67 of awq_gemm.cu's time; 33 are more than 3 % longer than there (at most 17 %), with
+// this kernel always 259 (up to 1.7 times).  us there / here: 1024 x 12288 15 / 18 at 9 tokens, 15 / 22 at 16; 4096 x 12288 29 / 25
+// at 16; gated 2 x 8192 x 12288 71 / 91 at 16.
+bool int4_pays(int T, int N, int K, bool gated) {
+  const int tiles = gated ? (N + 7) / 8 : (N + 15) / 16;
+  const Shape f = T > 8 ? shape_of<true, 8, 2, 2, 2>(T, K, tiles) : tiles >= 320 ? shape_of<true, 8, 2, 1, 2>(T, K, tiles)
+                                                                             : shape_of<true, 8, 1, 1, 4>(T, K, tiles);
+  if (T <= 8 && f.segs == 1) return true;
+  const int rounds = (f.blocks + f.per_sm * sm_count() - 1) / (f.per_sm * sm_count());
+  const float tk = static_cast<float>(T) * K;
+  const float piece = f.segs == 1 ? 0.f : T > 8 ? 5.8e-5f : 2.4e-5f;        // of a token's value, staged again in each round
+  const float here = 1.63f + (f.segs == 1 ? 6.8e-6f * tk : 0.f) + rounds * (1.86f + f.per_sm * K * (5.2e-4f + 1.22e-5f * T) + piece * tk);
+  const int rows = (N + 127) / 128, most = (gated ? 1 : 2) * sm_count() * 19 / 20;      // clusters leave some SMs over
+  int split = (107 + rows - 1) / rows;
+  if (split > 8) split = 8;
+  if (split > K / 128) split = K / 128 > 0 ? K / 128 : 1;
+  while (split > 1 && rows * split > most) --split;
+  const float k = static_cast<float>(K) / split;
+  const float there = gated ? 8.3f + 0.0084f * k + rows * (1.67e-5f * K + 0.0011f) : 4.36f + 0.0061f * k + rows * (2.7e-5f * K + 0.0011f);
+  return here <= there;
+}
+
 template <typename T>
 int by_kind(const SkinnyParams& p, cudaStream_t s) {
   if (p.int4) return p.group % 128 == 0 ? int4_by_size<T, true>(p, s) : int4_by_size<T, false>(p, s);
@@ -517,10 +553,16 @@ int by_kind(const SkinnyParams& p, cudaStream_t s) {
 
 }  // namespace
 
+bool skinny_takes(bool int4, bool norm, int T, int N, int K, bool gated) {
+  if (static_cast<double>(N) * K * (gated ? 2 : 1) >= 3.e10) return false;      // rows are counted in 32 bits (skinny_gemm)
+  if (int4) return !norm && T > 0 && T <= 16 && int4_pays(T, N, K, gated);
+  return norm && T <= 8 && static_cast<long>(T) * K <= 20000;
+}
+
 int skinny_gemm(const SkinnyParams& p, cudaStream_t stream) {
   if (p.T <= 0 || p.N <= 0) return 0;
   const bool norm = p.rms_eps > 0.f;
-  if (p.tile_expert == nullptr && !skinny_takes(p.int4 != 0, norm, p.T, p.K)) return -30;
+  if (p.tile_expert == nullptr && !skinny_takes(p.int4 != 0, norm, p.T, p.N, p.K, p.dual_rows > 0)) return -30;
   if (p.int4 ? norm : p.tile_expert != nullptr) return -30;
   // rows are counted in 16-byte words of 32 bits, scales in elements of 32 bits
   const uint64_t rows = p.int4 ? p.rows_total : p.dual_rows > 0 ? 2ull * p.dual_rows : p.N;
@@ -529,6 +571,11 @@ int skinny_gemm(const SkinnyParams& p, cudaStream_t stream) {
 }
 
 }  // namespace fi
+
+// skinny_takes, for whoever wants to know the route of a product.
+extern "C" int fi_skinny_takes(int int4, int norm, int T, int N, int K, int gated) {
+  return fi::skinny_takes(int4 != 0, norm != 0, T, N, K, gated != 0) ? 1 : 0;
+}
 
 // Routed int4 experts of few rows each: the rows of X that the sorted routes name (x_rows[r] / x_div; null: row r itself)
 // meet the weights of their expert; C [n_rows, ldc] in the order of the routes.  g: table of tiles of `bn` (8 or 16) rows.

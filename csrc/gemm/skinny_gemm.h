@@ -7,14 +7,11 @@
 
 namespace fi {
 
-// Whether skinny_gemm is the better kernel for T tokens.  int4 weights: up to 16 tokens (at 32 the operands from registers
-// lose to tensor memory: N = 8192, K = 2816 in 20.6 us against 14.6).  16-bit weights: products with a fused RMSNorm of few staged
-// tokens (a TinyLlama step of one token: 1.200 ms without, 1.183 with the gated one alone, 1.181 with q|k|v alone).  The others
-// are faster alone too, but not in a step, where their predecessors' rings hide the start of dense_gemm.cu's stream (o 1.264 ms,
-// down 1.246, logits of 151936 rows at three tokens 160 us slower).
-inline bool skinny_takes(bool int4, bool norm, int T, int K) {
-  return int4 ? T <= 16 : norm && T <= 8 && static_cast<long>(T) * K <= 20000;
-}
+// Whether skinny_gemm is the better kernel for T tokens and N outputs (gated: of two weight rows each).  16-bit weights: products
+// with a fused RMSNorm of few staged tokens (a TinyLlama step of one token: 1.200 ms without, 1.183 with the gated one alone, 1.181
+// with q|k|v alone).  The others are faster alone too, but not in a step, where their predecessors' rings hide the start of
+// dense_gemm.cu's stream (o 1.264 ms, down 1.246, logits of 151936 rows at three tokens 160 us slower).
+bool skinny_takes(bool int4, bool norm, int T, int N, int K, bool gated);
 
 struct SkinnyParams {
   const void* x;            // [T, K] rows of pitch ldx, 16-bit

@@ -26,3 +26,22 @@ def test_from_1024_tokens_on_and_by_the_switch(monkeypatch):
     monkeypatch.setattr(ops, "_PERSISTENT_BY_SIZE", False)
     assert ops._persistent_pays(129, 64, 8192)
     ops._persistent_pays.cache_clear()
+
+
+# (tokens, outputs, K, gated, us awq_gemm.cu, us skinny_gemm.cu)
+@pytest.mark.parametrize("T,N,K,gated,there,here", [
+    (16, 64, 6144, False, 8.9, 11.5), (14, 256, 6144, False, 9.4, 11.6), (12, 512, 8192, False, 11.1, 13.5), (9, 1024, 12288, False, 15.1, 17.5),
+    (16, 1024, 12288, False, 15.4, 22.1), (16, 2560, 12288, False, 22.1, 23.8), (16, 6144, 16384, False, 53.2, 60.3),
+    (16, 2560, 8192, True, 23.7, 30.0), (12, 2560, 12288, True, 30.2, 37.9), (16, 8192, 12288, True, 71.1, 90.6), (16, 12288, 512, False, 8.0, 9.0),
+    (16, 12288, 512, True, 11.6, 13.2),
+    (1, 64, 512, False, 6.1, 2.9), (8, 4096, 12288, False, 29.0, 24.1), (8, 12288, 4096, True, 49.3, 22.5), (9, 64, 512, False, 6.1, 3.7),
+    (16, 6144, 4096, False, 20.2, 13.3), (16, 4096, 4096, False, 13.4, 9.8), (16, 12288, 4096, True, 49.7, 30.9), (16, 4096, 12288, False, 29.2, 24.9),
+    (16, 8192, 2816, False, 17.0, 11.8), (16, 2112, 2816, True, 13.3, 8.2), (12, 2048, 8192, True, 23.0, 15.6)])
+def test_int4_products_of_few_tokens(T, N, K, gated, there, here):
+    assert bool(_lib.kernels().fi_skinny_takes(1, 0, T, N, K, gated)) == (here < there)
+
+
+def test_int4_products_of_more_tokens_or_more_weights_than_the_registers_take():
+    takes = _lib.kernels().fi_skinny_takes
+    assert takes(1, 0, 16, 4096, 4096, 0) and not takes(1, 0, 17, 4096, 4096, 0)
+    assert not takes(1, 0, 1, 1 << 20, 1 << 18, 0)
