@@ -378,6 +378,7 @@ static int fi_dense_gemm_impl(const void* X, const void* W, void* C, const void*
   if (act == kActClippedSwiglu && (dual_rows <= 0 || !(act_limit > 0.f))) return -12;
   if (bn == 0 && splits == 0 && comm == nullptr && grp == nullptr && !w_dynamic && g_plain_trace == nullptr &&
       (reinterpret_cast<uintptr_t>(X) & 15) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0 && (ldx % 8) == 0 && (ldw % 8) == 0 &&
+      static_cast<double>(dual_rows > 0 ? 2 * dual_rows : N) * ldw < 3.e10 &&      // rows are counted in 32 bits there
       skinny_takes(false, rms_eps > 0.f, T, N, K, dual_rows > 0)) {
     SkinnyParams q = {};
     q.x = X; q.w = W; q.C = C; q.bias = bias; q.residual = residual;

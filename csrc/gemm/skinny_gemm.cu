@@ -545,6 +545,19 @@ bool int4_pays(int T, int N, int K, bool gated) {
   return here <= there;
 }
 
+// 16-bit products with a fused norm: against dense_gemm.cu, whose rings stream long rows better (us there / here, one token: 6144 x
+// 8192 22 / 24, 256 x 12288 7.6 / 10.5, gated 2 x 2560 x 12288 30 / 34) and which has no rounds of CTAs to fill (K = 256: 10240 rows 4.2 /
+// 6.4; a third round that is nearly empty: 10240 x 2560 at 6 tokens 13.5 / 14.8).  Up to the lines below: 2560 x 2048 7.0 / 5.2, 6144 x
+// 4096 14.4 / 13.6, gated 2 x 5632 x 2048 15.3 / 11.0, 2 x 704 x 4096 8.8 / 5.5.  Over 832 products of 1 to 8 tokens (K = 256 to 19968,
+// 64 to 32000 outputs) 0.84 of the time there, 0.4 % over the better one each time; 4 are more than 3 % longer (at most 4 %).
+bool norm_pays(int T, int N, int K, bool gated) {
+  const int tiles = gated ? (N + 7) / 8 : (N + 15) / 16, round = 2 * sm_count();
+  if (K < 512) return gated ? tiles <= 512 : tiles <= 160 && T <= 5;
+  if (gated) return K <= 6144 || (K <= 8192 && tiles <= round);
+  if (K > 4096) return K <= 6144 && tiles >= 64 && tiles <= round;
+  return T <= 2 || tiles <= 2 * round || (tiles + round - 1) / round * round <= 1.3f * tiles;
+}
+
 template <typename T>
 int by_kind(const SkinnyParams& p, cudaStream_t s) {
   if (p.int4) return p.group % 128 == 0 ? int4_by_size<T, true>(p, s) : int4_by_size<T, false>(p, s);
@@ -556,7 +569,7 @@ int by_kind(const SkinnyParams& p, cudaStream_t s) {
 bool skinny_takes(bool int4, bool norm, int T, int N, int K, bool gated) {
   if (static_cast<double>(N) * K * (gated ? 2 : 1) >= 3.e10) return false;      // rows are counted in 32 bits (skinny_gemm)
   if (int4) return !norm && T > 0 && T <= 16 && int4_pays(T, N, K, gated);
-  return norm && T <= 8 && static_cast<long>(T) * K <= 20000;
+  return norm && T > 0 && T <= 8 && static_cast<long>(T) * K <= 20000 && norm_pays(T, N, K, gated);
 }
 
 int skinny_gemm(const SkinnyParams& p, cudaStream_t stream) {

@@ -45,3 +45,19 @@ def test_int4_products_of_more_tokens_or_more_weights_than_the_registers_take():
     takes = _lib.kernels().fi_skinny_takes
     assert takes(1, 0, 16, 4096, 4096, 0) and not takes(1, 0, 17, 4096, 4096, 0)
     assert not takes(1, 0, 1, 1 << 20, 1 << 18, 0)
+
+
+# (tokens, outputs, K, gated, us dense_gemm.cu, us skinny_gemm.cu)
+@pytest.mark.parametrize("T,N,K,gated,there,here", [
+    (1, 64, 8192, False, 6.1, 7.1), (1, 6144, 8192, False, 21.9, 24.4), (1, 256, 12288, False, 7.6, 10.5), (1, 1024, 16384, False, 12.3, 16.2),
+    (2, 256, 6144, False, 5.7, 6.3), (7, 10240, 2560, False, 13.8, 15.3), (3, 10240, 256, False, 4.2, 6.7), (8, 256, 256, False, 3.3, 3.8),
+    (1, 2560, 12288, True, 29.7, 33.8), (1, 1024, 19968, True, 22.1, 24.6), (1, 2560, 8192, True, 22.0, 22.9), (4, 10240, 256, True, 7.0, 9.6),
+    (1, 2560, 2048, False, 6.9, 5.0), (8, 2560, 2048, False, 7.2, 6.0), (1, 6144, 4096, False, 14.4, 13.6), (3, 32000, 4096, False, 47.9, 42.7),
+    (8, 6144, 2048, False, 9.7, 8.7), (1, 5632, 2048, True, 15.3, 10.9), (8, 5632, 2048, True, 15.9, 12.3), (4, 704, 4096, True, 9.0, 6.0),
+    (1, 704, 8192, True, 12.3, 9.4)])
+def test_products_of_few_tokens_with_a_norm(T, N, K, gated, there, here):
+    assert bool(_lib.kernels().fi_skinny_takes(0, 1, T, N, K, gated)) == (here < there)
+
+
+def test_products_of_few_tokens_without_a_norm_stay():
+    assert not any(_lib.kernels().fi_skinny_takes(0, 0, T, 2560, 2048, gated) for T in (1, 8) for gated in (0, 1))
