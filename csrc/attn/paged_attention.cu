@@ -461,7 +461,11 @@ __global__ void __launch_bounds__(128) paged_decode_kernel(const AttnParams p) {
 // multi-stage cp.async pipeline over 16-token groups (one KV block slice each), so the main loop has
 // no CTA-wide barrier and each SM keeps tens of KB of KV reads in flight.  Block-table entries are
 // fetched 32 groups at a time into registers and handed out by shuffle.  Needs block_size % 16 == 0.
-template <typename T, int HD, int NST, bool SIG>
+// OWN: the weights of a group are relative to the group's own maximum and meet the sums by a factor in 32 bits.  Rounded to 16 bits
+// the largest weight of every group is then exact, so a warp may take four groups as accurately as one (relative to the running
+// maximum, eight splits of 2040 keys are 3 to 5 % further from 64-bit results than 32).  It costs a multiplication per sum and group:
+// calls of few sequences take it, which are bound by latency (launch_decode_as); a step of 32 requests would take 1448 -> 1466 us.
+template <typename T, int HD, int NST, bool SIG, bool OWN>
 __global__ void __launch_bounds__(128) paged_decode_v2_kernel(const AttnParams p) {
   fi::pdl_launch_dependents();
   fi::pdl_wait();
@@ -597,6 +601,7 @@ __global__ void __launch_bounds__(128) paged_decode_v2_kernel(const AttnParams p
       MmaT<T>::mma(s[0], a, kb);
       MmaT<T>::mma(s[1], a, kb + 2);
     }
+    [[maybe_unused]] float a0, a1, b0 = 1.f, b1 = 1.f;      // what the sums so far, and this group's, are multiplied by
     if constexpr (SIG) {
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
@@ -625,23 +630,29 @@ __global__ void __launch_bounds__(128) paged_decode_v2_kernel(const AttnParams p
       mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
       mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
       const float nm0 = fmaxf(m0, mx0), nm1 = fmaxf(m1, mx1);
-      const float a0 = nm0 == -CUDART_INF_F ? 1.f : exp2f((m0 - nm0) * kLog2e);
-      const float a1 = nm1 == -CUDART_INF_F ? 1.f : exp2f((m1 - nm1) * kLog2e);
+      a0 = nm0 == -CUDART_INF_F ? 1.f : exp2f((m0 - nm0) * kLog2e);
+      a1 = nm1 == -CUDART_INF_F ? 1.f : exp2f((m1 - nm1) * kLog2e);
+      if constexpr (OWN) {
+        b0 = mx0 == -CUDART_INF_F ? 0.f : exp2f((mx0 - nm0) * kLog2e);
+        b1 = mx1 == -CUDART_INF_F ? 0.f : exp2f((mx1 - nm1) * kLog2e);
+      }
       float rs0 = 0.f, rs1 = 0.f;
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float nm = e < 2 ? nm0 : nm1;
+          const float mx = OWN ? (e < 2 ? mx0 : mx1) : (e < 2 ? nm0 : nm1);
           // tokens past seq_len inside a valid block hold stale cache data: their weight is exactly 0
-          const float pv = nm == -CUDART_INF_F ? 0.f : exp2f((s[j][e] - nm) * kLog2e);
+          const float pv = mx == -CUDART_INF_F ? 0.f : exp2f((s[j][e] - mx) * kLog2e);
           s[j][e] = pv;
           if (e < 2) rs0 += pv; else rs1 += pv;
         }
       }
-      l0 = l0 * a0 + rs0; l1 = l1 * a1 + rs1; m0 = nm0; m1 = nm1;
+      l0 = l0 * a0 + (OWN ? rs0 * b0 : rs0); l1 = l1 * a1 + (OWN ? rs1 * b1 : rs1); m0 = nm0; m1 = nm1;
+      if constexpr (!OWN) {
 #pragma unroll
-      for (int i = 0; i < HD / 8; ++i) { o[i][0] *= a0; o[i][1] *= a0; o[i][2] *= a1; o[i][3] *= a1; }
+        for (int i = 0; i < HD / 8; ++i) { o[i][0] *= a0; o[i][1] *= a0; o[i][2] *= a1; o[i][3] *= a1; }
+      }
     }
     uint32_t pa[4] = {MmaT<T>::pack(s[0][0], s[0][1]), MmaT<T>::pack(s[0][2], s[0][3]),
                       MmaT<T>::pack(s[1][0], s[1][1]), MmaT<T>::pack(s[1][2], s[1][3])};
@@ -649,8 +660,18 @@ __global__ void __launch_bounds__(128) paged_decode_v2_kernel(const AttnParams p
     for (int dp = 0; dp < HD / 16; ++dp) {
       uint32_t vb[4];
       ldsm_x4_t(vb, smem_addr(V + tile_off<HD>((lane & 7) + ((lane >> 3) & 1) * 8, dp * 2 + (lane >> 4))));
-      MmaT<T>::mma(o[2 * dp], pa, vb);
-      MmaT<T>::mma(o[2 * dp + 1], pa, vb + 2);
+      if constexpr (!OWN) {
+        MmaT<T>::mma(o[2 * dp], pa, vb);
+        MmaT<T>::mma(o[2 * dp + 1], pa, vb + 2);
+      } else {
+        float g[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        MmaT<T>::mma(g[0], pa, vb);
+        MmaT<T>::mma(g[1], pa, vb + 2);
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o[2 * dp + j][e] = fmaf(g[j][e], e < 2 ? b0 : b1, o[2 * dp + j][e] * (e < 2 ? a0 : a1));
+      }
     }
     __syncwarp();
   }
@@ -1059,7 +1080,9 @@ int launch_decode_as(const AttnParams& p, int B, cudaStream_t s) {
       pc.cluster_off = (smem + 127) & ~127;
       smem = pc.cluster_off + (16 * HD + 32) * 4;
     }
-    auto kern = paged_decode_v2_kernel<T, HD, NST, SIG>;
+    // few sequences: the calls that take eight splits in one cluster where they would fill the chip with many (pick_decode_splits)
+    const bool own = !SIG && pc.cluster_off > 0 && B * p.nkv <= (HD <= 128 ? 16 : 8);
+    auto kern = own ? paged_decode_v2_kernel<T, HD, NST, SIG, !SIG> : paged_decode_v2_kernel<T, HD, NST, SIG, false>;
     cudaError_t ce = fi::ensure_dynamic_smem(kern, smem);
     if (ce != cudaSuccess) return static_cast<int>(ce);
     if (pc.cluster_off > 0) {

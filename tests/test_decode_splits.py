@@ -36,3 +36,26 @@ def test_few_sequences(B, nh, nkv, hd, fp8, window):
                                         hd ** -0.5, window, 0.0)
         # probabilities and the result are rounded to 16 bits: 2^-8 of values that average around one each
         assert torch.all((got.float().cpu() - ref.float()).abs() <= 2.0 ** -6 * (ref.float().abs() + ref.float().abs().mean()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nkv,group,hd", [(4, 8, 64), (8, 4, 128), (8, 2, 256)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_eight_splits_are_as_accurate_as_many(nkv, group, hd, dtype):
+    """Distances from 64-bit results over several inputs, eight splits against one per 64 keys.  Both round the same weights, so
+    they differ by the order of 32-bit sums alone; 1 % covers results that fall on the other side of a rounding."""
+    few = many = 0.0
+    nh, blocks, context = nkv * group, 132, 2040
+    for seed in range(8):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        k, v = (torch.randn(1 + blocks, nkv, 16, hd, generator=g, device="cuda").to(dtype) for _ in range(2))
+        q = torch.randn(1, nh * hd, generator=g, device="cuda").to(dtype)
+        table = (1 + torch.randperm(blocks, generator=g, device="cuda")).int().view(1, -1)
+        seq = torch.tensor([context], device="cuda", dtype=torch.int32)
+        keys, values = (c[table[0].long()].permute(1, 0, 2, 3).reshape(nkv, -1, hd)[:, :context].double() for c in (k, v))
+        ref = (torch.softmax(q.double().view(nkv, group, hd) @ keys.transpose(1, 2) * hd ** -0.5, -1) @ values).reshape(1, -1)
+        for splits in (8, 32):
+            got = ops.paged_attention_decode(q, k, v, table, seq, nh, nkv, hd, hd ** -0.5, splits=splits, max_kv_len=2112)
+            err = float((got.double() - ref).norm() / ref.norm())
+            few, many = (few + err, many) if splits == 8 else (few, many + err)
+    assert few <= 1.01 * many
