@@ -22,6 +22,7 @@
 #include "../common/tensormap.h"
 #include "comm_desc.h"
 #include "epilogue.cuh"
+#include "int4_stages.h"
 #include "routes.h"
 #include "skinny_gemm.h"
 
@@ -73,7 +74,6 @@ __device__ __forceinline__ int raw_swizzle_chunk(int row, int c) {
 
 // Threads: warp 0 TMA producer, warp 1 MMA issuer, warps 2..9 dequantisers (warps 2..5 also run the
 // TMEM -> shared-memory part of the epilogue, every thread the final reduce/store).
-constexpr int kDequantWarps = 8;
 constexpr int kAwqThreads = 64 + kDequantWarps * 32;
 
 template <typename T, int BN, int RST, int AST, bool DUAL, bool ROW = false>
@@ -96,12 +96,8 @@ awq_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
   // Row-per-thread dequantisation (template flag ROW; decode-sized token tiles with SUBS == 4 k-blocks per raw stage):
   // a thread owns one weight row and two whole k-blocks of every raw stage, so it waits for the raw stage once,
   // fetches one scale / zero point per 32..64 values and touches a barrier once per 64 values: about half the
-  // per-value overhead of the half-k-block scheme used for larger token tiles.  The two halves of the warps take
-  // the k-blocks in turn (even, odd): a warp then comes back to an A stage at most AST + 2 k-blocks after the last
-  // one it knows to be read, and the parity of the stage's barrier tells that apart from a stage one round older
-  // for any AST >= 2.  Two neighbouring k-blocks per half would skip two, and with AST == 2 a warp that ran ahead
-  // could take an unread stage for a free one.
-  constexpr bool kRowScheme = ROW && (SUBS == 4);
+  // per-value overhead of the half-k-block scheme used for larger token tiles.  Which half writes which k-block: int4_stages.h.
+  constexpr bool kRowScheme = ROW && (SUBS == kRowBlocks);
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -141,9 +137,7 @@ awq_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
       mbar_init(&raw_empty[s], 1 + kDequantWarps);   // MMA commit (token tile) + one arrival per dequant warp
     }
     for (int s = 0; s < AST; ++s) {
-      // one arrival per dequant warp that writes the stage: all eight in the half-k-block scheme, the four
-      // that own the k-block in the row-per-thread scheme (SUBS == 4)
-      mbar_init(&a_full[s], kRowScheme ? kDequantWarps / 2 : kDequantWarps);
+      mbar_init(&a_full[s], a_full_arrivals(kRowScheme));   // one per dequant warp that writes the stage
       mbar_init(&a_empty[s], 1);
     }
     mbar_init(accum_bar, 1);
@@ -265,7 +259,7 @@ awq_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
       for (int u = 0; u < 2; ++u)
 #pragma unroll
         for (int h = 0; h < 2; ++h)
-          ld_off[u][h] = SUBS * B_BYTES + row * QROW + raw_swizzle_chunk<SUBS>(row, (u * 2 + half) * 2 + h) * 16;
+          ld_off[u][h] = SUBS * B_BYTES + row * QROW + raw_swizzle_chunk<SUBS>(row, row_block(u, half) * 2 + h) * 16;
       size_t srow[NA];
       bool rvalid[NA];
 #pragma unroll
@@ -280,7 +274,7 @@ awq_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
       auto fetch = [&](int rs) {
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-          const int kb = kb_begin + rs * SUBS + u * 2 + half;
+          const int kb = kb_begin + rs * SUBS + row_block(u, half);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int k = kb * BK + h * 32;
@@ -325,7 +319,7 @@ awq_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
         }
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-          const int sub = u * 2 + half;
+          const int sub = row_block(u, half);
           const int kb = kb_begin + rs * SUBS + sub;
           if (kb >= kb_end) break;                                       // ragged last raw stage (uniform per warp)
           const int it = rs * SUBS + sub;                                // k-blocks use the A stages round robin
@@ -537,12 +531,12 @@ int dispatch(int bn, const CUtensorMap& tw, const TokenMaps& tx, const GemmParam
   switch (bn) {
     // raw stages hold raw_subs(BN) k-blocks each; sizes keep two CTAs per SM where possible
     // decode-sized tiles: row-per-thread dequantisers (FI_AWQ_ROW_SCHEME=0: the older half-k-block dequantisers)
-    case 16: return row_scheme() ? launch<T, 16, 2, DUAL ? 2 : 3, DUAL, true>(tw, tx, p, s) : launch<T, 16, 2, DUAL ? 2 : 3, DUAL>(tw, tx, p, s);
-    case 32: return row_scheme() ? launch<T, 32, 2, DUAL ? 2 : 3, DUAL, true>(tw, tx, p, s) : launch<T, 32, 2, DUAL ? 2 : 3, DUAL>(tw, tx, p, s);
+    case 16: return row_scheme() ? launch<T, 16, 2, a_stages(DUAL), DUAL, true>(tw, tx, p, s) : launch<T, 16, 2, a_stages(DUAL), DUAL>(tw, tx, p, s);
+    case 32: return row_scheme() ? launch<T, 32, 2, a_stages(DUAL), DUAL, true>(tw, tx, p, s) : launch<T, 32, 2, a_stages(DUAL), DUAL>(tw, tx, p, s);
     // 33 to 64 tokens (us before / now: 6144 x 4096 24.7 / 20.0, gated 2 x 12288 x 4096 67 / 56, 4096 x 12288 37 / 28); experts keep the
     // smaller stages, two CTAs of which share an SM (128 experts, 768 tokens: 463 / 496)
-    case 64: return row64(p.tile_expert != nullptr) ? launch<T, 64, 2, DUAL ? 2 : 3, DUAL, true>(tw, tx, p, s) : launch<T, 64, 2, DUAL ? 2 : 3, DUAL>(tw, tx, p, s);
-    default: return launch<T, 128, 3, DUAL ? 2 : 3, DUAL>(tw, tx, p, s);
+    case 64: return row64(p.tile_expert != nullptr) ? launch<T, 64, 2, a_stages(DUAL), DUAL, true>(tw, tx, p, s) : launch<T, 64, 2, a_stages(DUAL), DUAL>(tw, tx, p, s);
+    default: return launch<T, 128, 3, a_stages(DUAL), DUAL>(tw, tx, p, s);
   }
 }
 

@@ -3,16 +3,35 @@
 Two halves of the dequantising warps write k-blocks into a ring of AST stages; the tensor core reads the blocks in order.
 A writer waits for the parity of its stage's "empty" barrier.  A parity tells only neighbouring rounds apart, so the split of
 the k-blocks over the halves has to keep a writer from coming back to a stage two rounds early.  The CPU test walks every
-interleaving of a model of the barriers with the split that the kernel's source states; the GPU test repeats products with few
-k-blocks, where a half can run furthest ahead, and wants the same bits every time.
+interleaving of a model of the barriers with the split, stages and arrivals that the kernel takes from its header
+(csrc/gemm/int4_stages.h, compiled here for the host).  The model's own part is the rest: one wait for a stage's "empty" parity and
+one set of arrivals per k-block, reads in order.  The GPU test repeats products with few k-blocks, where a half can run furthest
+ahead, through each of the kernel's token tiles that work this way, and wants the same bits every time.
 """
-import re
+import ctypes
+import subprocess
 from pathlib import Path
 
 import pytest
 import torch
 
-SOURCE = Path(__file__).resolve().parents[1] / "csrc" / "gemm" / "awq_gemm.cu"
+HEADER = Path(__file__).resolve().parents[1] / "csrc" / "gemm" / "int4_stages.h"
+
+
+@pytest.fixture(scope="module")
+def kernel_side(tmp_path_factory):
+    """The header's numbers as functions of a host library."""
+    d = tmp_path_factory.mktemp("stages")
+    (d / "s.cpp").write_text(f'''#include "{HEADER}"
+extern "C" {{
+int row_block(int u, int half) {{ return fi::row_block(u, half); }}
+int row_blocks() {{ return fi::kRowBlocks; }}
+int warps() {{ return fi::kDequantWarps; }}
+int a_stages(int gated) {{ return fi::a_stages(gated != 0); }}
+int a_full_arrivals(int row) {{ return fi::a_full_arrivals(row != 0); }}
+}}''')
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-o", str(d / "s.so"), str(d / "s.cpp")], check=True)
+    return ctypes.CDLL(str(d / "s.so"))
 
 
 def _early_write(stages: int, mine: list[list[int]], blocks: int) -> tuple | None:
@@ -39,26 +58,48 @@ def _early_write(stages: int, mine: list[list[int]], blocks: int) -> tuple | Non
     return None
 
 
-@pytest.mark.parametrize("stages", [2, 3])
-def test_no_half_takes_an_unread_stage(stages):
-    rule = re.search(r"const int sub = ([uhalf0-9 +*]+);", SOURCE.read_text()).group(1)
+def _split(lib, blocks):
+    per = lib.row_blocks()
+    return [[per * rs + lib.row_block(u, half) for rs in range(blocks // per) for u in range(per // 2)] for half in (0, 1)]
+
+
+@pytest.mark.parametrize("gated", [0, 1])
+def test_no_half_takes_an_unread_stage(kernel_side, gated):
     blocks = 24
-    mine = [[4 * rs + eval(rule, {"u": u, "half": half}) for rs in range(blocks // 4) for u in (0, 1)] for half in (0, 1)]
-    assert sorted(mine[0] + mine[1]) == list(range(blocks))
-    assert _early_write(stages, mine, blocks) is None
+    mine = _split(kernel_side, blocks)
+    assert sorted(mine[0] + mine[1]) == list(range(blocks)) and all(m == sorted(m) for m in mine)
+    assert _early_write(kernel_side.a_stages(gated), mine, blocks) is None
 
 
+def test_the_walk_finds_the_race_of_neighbouring_blocks():
+    assert _early_write(2, [[4 * rs + half * 2 + u for rs in range(6) for u in (0, 1)] for half in (0, 1)], 24) is not None
+
+
+def test_a_stage_is_full_when_the_half_that_owns_its_block_has_arrived(kernel_side):
+    mine = _split(kernel_side, 8)
+    assert not set(mine[0]) & set(mine[1])            # one half of the warps per k-block
+    assert kernel_side.a_full_arrivals(1) == kernel_side.warps() // 2
+    assert kernel_side.a_full_arrivals(0) == kernel_side.warps()
+
+
+# up to 16 tokens the tile is asked for: by size such products take another kernel
 @pytest.mark.gpu
+@pytest.mark.parametrize("T,bn", [(5, 16), (16, 16), (17, 0), (32, 0), (40, 0), (64, 0)])
 @pytest.mark.parametrize("K,group", [(704, 32), (2816, 32), (4096, 128)])
 @pytest.mark.parametrize("gated", [False, True])
-def test_repeated_int4_products_are_the_same(K, group, gated):
-    from litevllm_b200.ops.awq import Int4Weight, int4_linear
+def test_repeated_int4_products_are_the_same(T, bn, K, group, gated):
+    from litevllm_b200.ops.awq import Int4Weight, dequantize, int4_linear
+    from test_skinny_gemm import _close
     g = torch.Generator(device="cuda").manual_seed(1)
     N = 1408
     nib = torch.randint(0, 16, (N, K), generator=g, device="cuda", dtype=torch.uint8)
-    scales = torch.rand(N, K // group, generator=g, device="cuda").mul_(0.01).to(torch.bfloat16)
+    scales = (torch.rand(N, K // group, generator=g, device="cuda") + 0.5).mul_(0.2 * K ** -0.5).to(torch.bfloat16)
     w = Int4Weight(nib, scales, None, group, torch.bfloat16)
-    x = torch.randn(5, K, generator=g, device="cuda").to(torch.bfloat16)
-    first = int4_linear(x, w, gated_act="gelu_tanh" if gated else None)
+    x = torch.randn(T, K, generator=g, device="cuda").to(torch.bfloat16)
+    first = int4_linear(x, w, gated_act="gelu_tanh" if gated else None, bn=bn)
+    ref = x.float() @ dequantize(nib, scales, None, group).t()
+    if gated:
+        ref = torch.nn.functional.gelu(ref[:, :N // 2], approximate="tanh") * ref[:, N // 2:]
+    _close(first, ref, torch.bfloat16, 4.0)           # the bound of the same products in test_skinny_gemm.py
     for _ in range(300):
-        assert torch.equal(int4_linear(x, w, gated_act="gelu_tanh" if gated else None), first)
+        assert torch.equal(int4_linear(x, w, gated_act="gelu_tanh" if gated else None, bn=bn), first)
