@@ -61,6 +61,30 @@ def test_int4(T, N, K, group, zero, gated):
         _close(int4_linear(x, w, residual=r), y + r.float(), dtype, 4.0)
 
 
+@pytest.mark.parametrize("T,N,gated", [(8, 9616, False), (8, 4808, True), (9, 4912, False), (9, 4808, True), (12, 9616, False),
+                                       (12, 6152, True), (16, 7200, False), (16, 6152, True)])
+@pytest.mark.parametrize("group", [32, 128])
+def test_int4_tokens_in_pieces_over_several_rounds(T, N, gated, group):
+    """Tokens that do not fit shared memory in one piece and more tiles than CTAs: every round stages the pieces again, while
+    the ring of weights runs on."""
+    from litevllm_b200.ops import _lib
+    from litevllm_b200.ops.awq import Int4Weight, dequantize, int4_linear
+    g = torch.Generator(device=DEV).manual_seed(N + T)
+    dtype, K, rows = torch.float16 if group == 128 else torch.bfloat16, 12288, 2 * N if gated else N
+    assert _lib.kernels().fi_skinny_takes(1, 0, T, N, K, gated)
+    nib = torch.randint(0, 16, (rows, K), generator=g, device=DEV, dtype=torch.uint8)
+    scales = (torch.rand(rows, K // group, generator=g, device=DEV) + 0.5).mul_(0.2 * K ** -0.5).to(dtype)
+    zeros = torch.randint(5, 11, (rows, K // group), generator=g, device=DEV, dtype=torch.uint8) if group == 128 else None
+    x = torch.randn(T, K, generator=g, device=DEV).to(dtype)
+    y = x.float() @ dequantize(nib, scales, zeros, group).t()
+    w = Int4Weight(nib, scales, zeros, group, dtype)
+    if gated:
+        ref = torch.nn.functional.gelu(y[:, :N], approximate="tanh") * y[:, N:]
+        _close(int4_linear(x, w, gated_act="gelu_tanh"), ref, dtype, 4.0)
+    else:
+        _close(int4_linear(x, w), y, dtype, 4.0)
+
+
 @pytest.mark.parametrize("T,E,K,H,inter", [(1, 8, 2, 128, 64), (3, 16, 4, 2816, 704), (40, 8, 2, 256, 96 * 2), (33, 128, 8, 192, 64)])
 def test_experts_of_few_rows(T, E, K, H, inter):
     """Tables of 8- and 16-row tiles, experts with more rows than a tile and with none, K that ends inside a chunk."""
