@@ -85,7 +85,7 @@ def test_int4_tokens_in_pieces_over_several_rounds(T, N, gated, group):
         _close(int4_linear(x, w), y, dtype, 4.0)
 
 
-@pytest.mark.parametrize("T,E,K,H,inter", [(1, 8, 2, 128, 64), (3, 16, 4, 2816, 704), (40, 8, 2, 256, 96 * 2), (33, 128, 8, 192, 64)])
+@pytest.mark.parametrize("T,E,K,H,inter", [(1, 8, 2, 128, 64), (3, 16, 4, 2816, 704), (40, 8, 2, 256, 96 * 2), (33, 128, 8, 192, 64), (11, 2, 2, 4096, 4096)])
 def test_experts_of_few_rows(T, E, K, H, inter):
     """Tables of 8- and 16-row tiles, experts with more rows than a tile and with none, K that ends inside a chunk."""
     from litevllm_b200.ops import moe
