@@ -30,8 +30,8 @@
 //   16-bit with RMSNorm, one token, N x K: 2560 x 2048   6.6 -> 4.7 (1.6)    2 x 5632 x 2048   14.4 -> 9.9 (6.9)
 //   int4 group 128, three tokens:  6144 x 4096  20.6 -> 8.2 (1.9)    2 x 12288 x 4096  48.4 -> 20.5 (7.6)   4096 x 12288   29.5 -> 14.0 (3.8)
 //   int4 group 32, 16 tokens:      8192 x 2816  17.0 -> 11.8 (1.7)   2 x 2112 x 2816   13.3 -> 8.2 (0.9)
-// The int4 forms are bound by the issue of about 3.6 instructions per weight (62 % of the slots, ALU 50 %), the 16-bit forms of
-// large matrices by memory, small ones by the latencies of one CTA's life.
+// The int4 forms are bound by the issue of 3.6 (layers) to 5.4 (experts' down products) instructions per weight (56 to 62 % of the
+// slots, ALU 45 to 51 %), the 16-bit forms of large matrices by memory, small ones by the latencies of one CTA's life.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -507,8 +507,11 @@ int launch(const SkinnyParams& p, int tiles, cudaStream_t s) {
 // Which split of the warps.  Measured on one B200, us per launch in a captured chain, weights cold (512 tiles: N = 8192):
 //   plain products split every tile's K over all eight warps; fewer warps per tile lengthen the chain of a warp and were
 //   slower at every size tried (int4 N = K = 4096, one token: 5.7 against 7.5 with four warps, 11.2 with two).
-//   Two tiles per warp share the reads of the tokens but halve the CTAs: for up to 8 tokens they pay from about 320 tiles on
-//   (int4 N = 6144, K = 4096: 7.3 against 8.1; N = 4096, K = 12288: 17.8 against 11.9), for 9 to 16 always (24.9 against 34.3).
+//   Two tiles per warp share the reads of the tokens but halve the CTAs.  For up to 8 tokens one tile per warp needs a second round
+//   of CTAs past 296 tiles: two tiles pay from there on (one / two, K = 4096, one token: 0.87 of the time at 288 tiles, 1.13 at 320, 1.07 at 512;
+//   K = 2816 0.89, 1.16, 1.12), with K of 8192 and more less or not at all (0.74, 0.92, 1.00), with K up to 1024 everywhere.  For 9 to
+//   16 tokens, whose accumulators leave one CTA per SM either way, two tiles are 0 to 45 % faster at nearly every size (K = 704 to
+//   12288, 192 to 1536 tiles), up to 10 % slower at 128 tiles.
 //   Experts have short K and many tiles: two warps per tile (128 experts of 2816 x 704, 32 tokens: 153; four warps 202).
 template <typename T, bool POST>
 int int4_by_size(const SkinnyParams& p, cudaStream_t s) {

@@ -446,6 +446,8 @@ def pick_decode_splits(B: int, nkv: int, max_kv_len: int, sm_count: int = 148, c
     # Few sequences: eight splits of a few more keys cost less than a second launch per layer.  us per step, more splits and a
     # merge kernel / eight (contexts of 100 to 2040 tokens): TinyLlama 1 sequence 1161 / 932 to 1170 / 1021, 4 (19 wanted) 1126 / 1074
     # to 1183 / 1136; 8 heads of 128 at 4 sequences (10 wanted) lose 1 to 3 %.  Heads of 256: 1 sequence (37) 832 / 805, 2 (19) lose up to 4 %.
+    # Alone, 280 forms within the rule (head sizes 64 to 256, 1 to 8 KV heads, 1 to 15 sequences, 100 to 2560 keys) take 0.45 to 1.01 of the time.
+    # The length is the capacity that a graph is captured for, not the present context: engines above 2560 tokens keep their splits.
     if cluster_head > 0 and want >= (19 if cluster_head <= 128 else 37) and max_kv_len <= 8 * 320:
         want = 8
     return int(max(1, min(want, chunks, 32)))
