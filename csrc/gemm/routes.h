@@ -2,11 +2,12 @@
 // which tile, follows from the smaller one.  Plain host arithmetic.
 //
 // The forms follow the kernels (waves of tiles, a main loop that hides the epilogue of the tile in front, K split over a
-// cluster where there are few tiles); their numbers are fitted to one B200, products of 129 to 1000 tokens, K = 128 to 12288,
-// 64 to 32000 rows, weights cold.  Over 1485 of them choosing by the estimates takes 0.2 % longer than the better kernel each time;
-// against one_tile_us's kernel alone the products take 0.79 of the time on average, 12 of them more than 3 % longer (at most 11 %).
-// Persistent alone: 0.86, 305 of them longer, up to twice as long.  The int4 forms: 129 to 3000 tokens, groups of 32 and 128, gated
-// and plain, K = 256 to 16384, 64 to 12288 rows.
+// cluster where there are few tiles); their numbers are fitted to one B200, to products alone and behind a norm in captured chains,
+// weights cold: 16-bit weights at 129 to 1023 tokens, K = 128 to 12288, 64 to 32000 rows; int4 at 129 to 3000 tokens, groups of 32 and
+// 128, gated and plain, K = 256 to 16384, 64 to 12288 outputs.  Of 1485 and 2448 products alone choosing by the estimates takes 0.2 %
+// longer than the better kernel each time; 31 and 23 are more than 3 % slower than in the kernel that took all of them
+// before (at most 14 and 19 %), against 305 and 293 (up to twice as slow) with the persistent kernel always.  Behind a norm, where
+// clusters wait for room that single CTAs do not need, the 476 and 480 closest of them take 0.97 and 0.98 of the time there.
 #pragma once
 
 namespace fi {
@@ -53,31 +54,30 @@ inline float persistent_us(int T, int N, int K, bool gated, int sms) {
 // SM and the last split the persistent kernel was the faster one at every size tried.)
 inline float one_tile_us(int T, int N, int K, int sms) {
   const int tiles = ceil_div(N, 128) * ceil_div(T, 128);
-  int split = 108 / tiles;
+  int split = 150 / tiles;
   if (split > 8) split = 8;
   if (split > K / 128) split = K / 128;
-  // tiles in other numbers than powers of two were 2 to 3 us slower from five on (N = 128, K = 2816: 10.6 us with 4 tiles, 13.9 with
-  // 6, 11.5 with 8)
-  const float odd = tiles > 4 && (tiles & (tiles - 1)) != 0 ? 2.f : 0.f;
-  if (split > 1) return 6.9f + (N > 64 ? 1.6f : 0.f) + 0.175f * (tiles < 12 ? tiles : 12) + odd + 0.0052f * K / split;
+  // tiles in other numbers than powers of two are slower from five on (N = 128, K = 2816: 10.6 us with 4 tiles, 13.9 with 6, 11.5
+  // with 8)
+  const float odd = tiles > 4 && (tiles & (tiles - 1)) != 0 ? 0.8f : 0.f;
+  if (split > 1) return 6.9f + (N > 64 ? 2.2f : 0.f) + 0.2f * (tiles < 12 ? tiles : 12) + odd + 0.0076f * K / split;
   if (tiles <= sms) return 1e9f;
   const float rounds = tiles <= 4 * sms ? static_cast<float>(ceil_div(tiles, 2 * sms)) : tiles / (2.f * sms);
-  return rounds * (6.8f + 0.0068f * K);
+  return rounds * (7.35f + 0.0071f * K);
 }
 
 // awq_gemm.cu, token tiles of 128: each tile expands its weights again; gated tiles have an SM to themselves.
 inline float int4_fused_us(int T, int N, int K, bool gated, int sms) {
   const int tiles = ceil_div(N, 128) * ceil_div(T, 128);
-  if (gated) return ceil_div(tiles, sms) * (18.5f + 0.0113f * K);
-  int split = 82 / tiles;
+  if (gated) return ceil_div(tiles, sms) * (17.9f + 0.0114f * K);
+  int split = 81 / tiles;
   if (split > 8) split = 8;
   if (split > K / 128) split = K / 128;
-  if (split > 1) return 5.9f + (N > 64 ? 3.1f : 0.f) + 0.0116f * K / split;
-  const int rounds = ceil_div(tiles, 2 * sms);
-  return 7.1f * rounds + K * (0.0059f * rounds + 0.0022f * tiles / sms);
+  if (split > 1) return 6.3f + (N > 64 ? 5.f : 0.f) + 0.01f * K / split;
+  return ceil_div(tiles, 2 * sms) * (5.4f + 0.0122f * (K < 4096 ? K : 4096) + 0.007f * (K < 4096 ? 0 : K - 4096));
 }
 
 // The copy in 16 bits: half a byte and the scales of each value read, two written.
-inline float int4_expand_us(int rows, int K, int group) { return 0.5f + 3.9e-7f * rows * K * (1.f + 10.f / group); }
+inline float int4_expand_us(int rows, int K, int group) { return 0.37f + 3.8e-7f * rows * K * (1.f + 9.4f / group); }
 
 }  // namespace fi

@@ -34,7 +34,7 @@ def test_everything_off(monkeypatch):
     (129, 64, 4096, 128, False, 10.8, 15.3), (512, 64, 8192, 32, False, 15.0, 23.5), (129, 256, 8192, 128, False, 18.2, 24.1),
     (200, 512, 12288, 128, False, 24.9, 35.1), (1024, 4096, 512, 128, False, 13.7, 18.5), (512, 8192, 512, 32, False, 13.7, 18.9),
     (768, 6144, 256, 128, False, 11.0, 16.7), (300, 12288, 8192, 128, False, 101.6, 119.6), (200, 8192, 12288, 32, True, 180.4, 227.1),
-    (192, 6144, 4096, 128, False, 42.0, 28.0), (2048, 6144, 4096, 128, False, 157.0, 97.0), (2048, 4096, 12288, 128, False, 268.0, 201.0),
+    (192, 6144, 4096, 128, False, 42.0, 28.0), (351, 8192, 2816, 32, False, 43.8, 32.5), (1250, 2816, 2112, 32, False, 38.9, 27.5), (2048, 6144, 4096, 128, False, 157.0, 97.0), (2048, 4096, 12288, 128, False, 268.0, 201.0),
     (2048, 8192, 2816, 32, False, 139.0, 93.0), (1000, 256, 4096, 128, False, 23.3, 15.8), (512, 512, 2816, 32, False, 20.8, 13.6),
     (129, 64, 512, 128, True, 24.5, 12.4), (192, 12288, 4096, 128, True, 141.0, 109.0), (2048, 2112, 2816, 32, True, 109.0, 46.0)])
 def test_the_faster_kernel_by_size(T, N, K, group, gated, fused, expanded):
