@@ -30,87 +30,22 @@
 #include "../common/ptx.cuh"
 #include "../common/tensormap.h"
 #include "comm_desc.h"
+#include "persistent.cuh"
 #include "routes.h"
 
 using namespace fi;
 
 namespace {
 
-constexpr int BM = 128;   // weight rows per tile (UMMA M)
+constexpr int BM = kTileRows;
 constexpr int BK = 64;    // k-block: 64 16-bit values = one 128-byte swizzled row
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = 64 + 32 * kEpiWarps;
 
-struct PParams {
-  void* C;
-  const void* bias;
-  const void* residual;
-  int T, N, K, ldc;
-  int dual_rows, act, is_fp16, out_fp32;
-  float act_limit;     // act 4
-  int second_off;   // weight rows between the two A tiles of a CTA: dual_rows (gated) or 128 (grouped plain form, 256-row tile)
-  int rows_per_tile;   // output rows (of N) one tile covers: 128, or 256 in the grouped plain form
-  int n_tiles_n, n_tiles;
-  int n_group;         // weight tiles that are worked on together over all token tiles (grouped mode: all of them)
-  int* status;
-  // grouped mode (tile_expert != null): n_tiles is the grid's upper bound, the true number of token tiles is *tiles
-  const int* tile_expert;
-  const int* tile_row0;
-  const int* tile_rows;
-  const int* tiles;
-  int expert_rows;     // weight rows per expert
-};
-
-__device__ __forceinline__ float act_f(float g, int act) {
-  if (act == 1) return g / (1.f + __expf(-g));
-  if (act == 2) {
-    const float inner = 0.7978845608028654f * (g + 0.044715f * g * g * g);
-    return g / (1.f + __expf(-2.f * inner));
-  }
-  if (act == 3) return fmaxf(g, 0.f);
-  if (act == 5) { g = fmaxf(g, 0.f); return g * g; }
-  if (act == 6) return 1.f - 2.f / (1.f + __expf(2.f * g));
-  return g;
-}
-// Gated form of one channel: act(g) * u; 4: bounds on both halves (g from above only), g sigmoid(1.702 g) * (u + 1).
-__device__ __forceinline__ float gated_f(float g, float u, int act, float limit) {
-  if (act == 4) {
-    g = fminf(g, limit);
-    u = fminf(fmaxf(u, -limit), limit);
-    return g / (1.f + __expf(-1.702f * g)) * (u + 1.f);
-  }
-  return act_f(g, act) * u;
-}
-__device__ __forceinline__ float ld16(const void* p, size_t i, int is_fp16) {
-  if (is_fp16) return __half2float(reinterpret_cast<const __half*>(p)[i]);
-  return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]);
-}
-
-// a / b of non-negative numbers.  The estimate is within one below 2^22 (two units in its last place are half a unit there); the
-// exact division takes 0.2 us of a tile's start, twice (gated 2 x 4096 x 256 at 4096 tokens: 69.2 us, so 65.8).
-__device__ __forceinline__ int quotient(int a, int b) {
-  if (a >= (1 << 22)) return a / b;
-  const int q = static_cast<int>(__fdividef(static_cast<float>(a), static_cast<float>(b)));
-  const int r = a - q * b;
-  return r < 0 ? q - 1 : r >= b ? q + 1 : q;
-}
-
-// Weight tile and token tile of a place in the order of work.  The tiles in flight at a time form a block of n_group weight tiles
-// by as many token tiles as there are CTAs for, so that what they share stays in L2 and matrices larger than L2 leave HBM once.
-// us with 2, 8, 16, 32 and all weight tiles in a group (one B200): gated 2 x 12288 x 4096 (201 MB) at 2048 tokens 321, 298, 312, 330, 407;
-// 2 x 8192 x 2816 (92 MB) 133, 135, 135, 145, 168; plain 12288 x 4096 (101 MB) 160, 161, 160, 166, 204; below about 50 MB all the same.
-__device__ __forceinline__ void tile_at(const PParams& p, int tile, int n_token_tiles, int* n, int* tt) {
-  const int per = p.n_group * n_token_tiles;
-  const int g = quotient(tile, per), at = tile - g * per;
-  const int width = min(p.n_group, p.n_tiles_n - g * p.n_group);      // the last group may be narrower
-  *tt = quotient(at, width);
-  *n = g * p.n_group + (at - *tt * width);
-}
-
 template <int STAGES, bool DUAL, int BN>      // BN: tokens per tile (UMMA N)
 __global__ void __launch_bounds__(kThreads)
 dense_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
-                             const PParams p) {
+                             const PersistentParams p) {
   constexpr int A_BYTES = BM * 128;
   constexpr int B_BYTES = BN * 128;
   constexpr int STAGE_BYTES = A_BYTES * (DUAL ? 2 : 1) + B_BYTES;
@@ -126,7 +61,7 @@ dense_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
   uint64_t* acc_empty = acc_full + 2;         // [2] epilogue -> MMA
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* aborted = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* stage = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(tmem_slot) + 16);   // [epilogue warps][16 tokens][32 rows]
+  float* stage = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(tmem_slot) + 16);   // a patch per epilogue warp (drain_tile)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   pdl_launch_dependents();
@@ -227,7 +162,6 @@ dense_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
     // ------------------------------------------------------------ epilogue warps
     const int c_begin = ((warp - 2) >> 2) * (BN / 2), c_end = c_begin + BN / 2;   // this warp's half of the tokens
     const int q = warp & 3;                     // TMEM lane quarter this warp may read
-    const int n_local = q * 32 + lane;          // weight row inside the tile
     int local = 0;
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++local) {
       const int b = local & 1;
@@ -242,96 +176,8 @@ dense_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
       const int n0 = nt * p.rows_per_tile;
       const int t0 = grouped ? p.tile_row0[tt] : tt * BN;
       const int t_end = grouped ? t0 + p.tile_rows[tt] : p.T;
-      const bool gated = p.dual_rows > 0;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(b * ACC_COLS);
-      // Each thread owns one weight row of the accumulator (a TMEM lane) but the output is
-      // token-major: a batch of 16 tokens x 32 rows goes through this warp's shared-memory patch as
-      // fp32 and comes back as 8-row vectors, so bias / residual / store are 16-byte accesses.
-      float* patch = stage + (warp - 2) * (16 * 32);
-      const int vc = lane & 3;                // which 8-row chunk of the warp's 32 rows this lane finishes
-      const int vj = lane >> 2;               // tokens vj and vj + 8 of the batch
-      // gated: one output row per thread (gate and up combined); plain wide tile: two rows, 128 apart
-      const int halves = (DUAL && !gated) ? 2 : 1;
-      float bias_g = 0.f, bias_u = 0.f;       // gated: bias of this thread's weight row in either half
-      if (DUAL && gated && p.bias != nullptr && n0 + n_local < p.N) {
-        bias_g = ld16(p.bias, n0 + n_local, p.is_fp16);
-        bias_u = ld16(p.bias, p.dual_rows + n0 + n_local, p.is_fp16);
-      }
-      for (int hh = 0; hh < halves; ++hh) {
-        const int nv = n0 + hh * BM + q * 32 + vc * 8;      // first of the 8 rows this lane stores
-        const bool nv_ok = nv < p.N;
-        float bias8[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) bias8[e] = (p.bias != nullptr && nv_ok && !gated) ? ld16(p.bias, nv + e, p.is_fp16) : 0.f;
-        // the residual values of a batch are requested one batch ahead, so their latency hides behind
-        // the TMEM read and the transposition of the batch in front
-        auto load_res = [&](int c0, uint4 (&dst)[2]) {
-#pragma unroll
-          for (int rep = 0; rep < 2; ++rep) {
-            const int t = t0 + c0 + vj + rep * 8;
-            dst[rep] = make_uint4(0, 0, 0, 0);
-            if (p.residual != nullptr && nv_ok && c0 < c_end && t < t_end)
-              dst[rep] = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.residual) +
-                                                         static_cast<size_t>(t) * p.ldc + nv);
-          }
-        };
-        uint4 res_cur[2], res_next[2];
-        load_res(c_begin, res_cur);
-#pragma unroll 1
-        for (int c0 = c_begin; c0 < c_end; c0 += 16) {
-          uint32_t r[16], u[16];
-          tmem_ld_x16(taddr + hh * BN + c0, r);
-          if (DUAL && gated) tmem_ld_x16(taddr + BN + c0, u);
-          load_res(c0 + 16, res_next);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            float v = __uint_as_float(r[j]);
-            if (DUAL && gated) v = gated_f(v + bias_g, __uint_as_float(u[j]) + bias_u, p.act, p.act_limit);
-            else v = act_f(v, p.act);
-            patch[j * 32 + lane] = v;
-          }
-          __syncwarp();
-#pragma unroll
-          for (int rep = 0; rep < 2; ++rep) {
-            const int j = vj + rep * 8;
-            const int t = t0 + c0 + j;
-            if (nv_ok && t < t_end) {
-              const float4 a0 = *reinterpret_cast<const float4*>(patch + j * 32 + vc * 8);
-              const float4 a1 = *reinterpret_cast<const float4*>(patch + j * 32 + vc * 8 + 4);
-              float v[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-              const size_t off = static_cast<size_t>(t) * p.ldc + nv;
-              if (p.out_fp32) {               // 32-bit output (no residual in this form)
-                float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.C) + off);
-                dst[0] = make_float4(v[0] + bias8[0], v[1] + bias8[1], v[2] + bias8[2], v[3] + bias8[3]);
-                dst[1] = make_float4(v[4] + bias8[4], v[5] + bias8[5], v[6] + bias8[6], v[7] + bias8[7]);
-                continue;
-              }
-              const uint4 raw = res_cur[rep];
-              const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w};
-              uint32_t ow[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                float lo = v[2 * e] + bias8[2 * e], hi = v[2 * e + 1] + bias8[2 * e + 1];
-                if (p.is_fp16) {
-                  const __half2 rr = *reinterpret_cast<const __half2*>(&rw[e]);
-                  lo += __low2float(rr); hi += __high2float(rr);
-                  const __half2 o = __floats2half2_rn(lo, hi);
-                  ow[e] = *reinterpret_cast<const uint32_t*>(&o);
-                } else {
-                  lo += __uint_as_float(rw[e] << 16); hi += __uint_as_float(rw[e] & 0xffff0000u);
-                  const __nv_bfloat162 o = __floats2bfloat162_rn(lo, hi);
-                  ow[e] = *reinterpret_cast<const uint32_t*>(&o);
-                }
-              }
-              *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.C) + off) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
-            }
-          }
-          __syncwarp();
-          res_cur[0] = res_next[0];
-          res_cur[1] = res_next[1];
-        }
-      }
+      drain_tile<BN, DUAL>(p, taddr, stage + (warp - 2) * kPatchFloats, n0, t0, t_end, c_begin, c_end, q, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[b]);   // this warp's quarter of the accumulator is free again
@@ -356,9 +202,9 @@ inline int sm_count() {
 }
 
 template <int STAGES, bool DUAL, int BN>
-int launch(const CUtensorMap& tw, const CUtensorMap& tx, const PParams& p, cudaStream_t stream) {
+int launch(const CUtensorMap& tw, const CUtensorMap& tx, const PersistentParams& p, cudaStream_t stream) {
   auto kern = dense_gemm_persistent_kernel<STAGES, DUAL, BN>;
-  constexpr int smem = STAGES * (BM * 128 * (DUAL ? 2 : 1) + BN * 128) + (2 * STAGES + 4) * 8 + 16 + kEpiWarps * 16 * 32 * 4 + 1024;
+  constexpr int smem = STAGES * (BM * 128 * (DUAL ? 2 : 1) + BN * 128) + (2 * STAGES + 4) * 8 + 16 + kEpiWarps * kPatchFloats * 4 + 1024;
   static_assert(smem <= 227 * 1024, "shared memory of one SM");
   {
     cudaError_t e = fi::ensure_dynamic_smem(kern, smem);
@@ -391,7 +237,7 @@ extern "C" int fi_dense_gemm_persistent(const void* X, const void* W, void* C, c
   if (r != 0) return r * 100 - 1;
   r = make_tmap_2d_16bit_sw128(&tx, X, T, K, ldx, tokens);
   if (r != 0) return r * 100 - 2;
-  PParams p = {};
+  PersistentParams p = {};
   p.C = C; p.bias = bias; p.residual = residual;
   p.T = T; p.N = N; p.K = K; p.ldc = ldc;
   p.dual_rows = dual_rows; p.act = act; p.act_limit = act_limit; p.is_fp16 = dtype == 1; p.out_fp32 = out_fp32;
@@ -438,7 +284,7 @@ extern "C" int fi_dense_gemm_persistent_grouped(const void* X, const void* W, vo
   if (r != 0) return r * 100 - 1;
   r = make_tmap_2d_16bit_sw128(&tx, X, n_rows, K, ldx, 128);
   if (r != 0) return r * 100 - 2;
-  PParams p = {};
+  PersistentParams p = {};
   p.C = C; p.T = n_rows; p.N = N; p.K = K; p.ldc = ldc; p.dual_rows = dual_rows; p.act = act; p.act_limit = act_limit; p.is_fp16 = dtype == 1;
   const bool wide = dual_rows == 0 && N > BM;
   p.second_off = dual_rows > 0 ? dual_rows : BM;
