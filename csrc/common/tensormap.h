@@ -63,4 +63,38 @@ inline int make_tmap_3d_16bit_sw128(CUtensorMap* out, const void* base, uint64_t
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 
+// Packed weights as a 2-D int32 tensor [rows, K/8]; box = 8 * subs words x 128 rows with the swizzle of its width.
+inline int make_tmap_packed(CUtensorMap* out, const void* base, uint64_t rows, uint64_t k_words, int subs) {
+  EncodeTiledFn enc = get_encode_tiled();
+  if (enc == nullptr) return -1;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || ((k_words * 4) & 15) != 0) return -2;
+  cuuint64_t dims[2] = {k_words, rows};
+  cuuint64_t strides[1] = {k_words * 4};
+  cuuint32_t box[2] = {static_cast<cuuint32_t>(8 * subs), 128};
+  cuuint32_t estr[2] = {1, 1};
+  const CUtensorMapSwizzle swz = subs == 4 ? CU_TENSOR_MAP_SWIZZLE_128B
+                                           : (subs == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE);
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<void*>(base), dims, strides, box,
+                   estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -3;
+}
+
+// Rows of plain 8- or 16-bit elements [rows, cols], pitch = cols: box = box_cols x box_rows, no swizzle (group scales and zero points,
+// whose neighbouring columns are neighbouring weight rows).
+inline int make_tmap_plain(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, int elem_bytes, uint32_t box_cols,
+                           uint32_t box_rows) {
+  EncodeTiledFn enc = get_encode_tiled();
+  if (enc == nullptr) return -1;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || ((cols * elem_bytes) & 15) != 0) return -2;
+  cuuint64_t dims[2] = {cols, rows};
+  cuuint64_t strides[1] = {cols * elem_bytes};
+  cuuint32_t box[2] = {box_cols, box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = enc(out, elem_bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(base), dims,
+                   strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -3;
+}
+
 }  // namespace fi

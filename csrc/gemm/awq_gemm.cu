@@ -540,23 +540,6 @@ int dispatch(int bn, const CUtensorMap& tw, const TokenMaps& tx, const GemmParam
   }
 }
 
-// Packed weights as a 2-D int32 tensor [rows, K/8]; box = 8 words x 128 rows, no swizzle.
-inline int make_tmap_packed(CUtensorMap* out, const void* base, uint64_t rows, uint64_t k_words, int subs) {
-  EncodeTiledFn enc = get_encode_tiled();
-  if (enc == nullptr) return -1;
-  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || ((k_words * 4) & 15) != 0) return -2;
-  cuuint64_t dims[2] = {k_words, rows};
-  cuuint64_t strides[1] = {k_words * 4};
-  cuuint32_t box[2] = {static_cast<cuuint32_t>(8 * subs), 128};
-  cuuint32_t estr[2] = {1, 1};
-  const CUtensorMapSwizzle swz = subs == 4 ? CU_TENSOR_MAP_SWIZZLE_128B
-                                           : (subs == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE);
-  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<void*>(base), dims, strides, box,
-                   estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : -3;
-}
-
 // The weights in 16 bits, [rows, K]: the values that the dequantisers above hand to the tensor core.  A warp takes 128
 // words (1024 values) of one row; lanes read neighbouring words, so both streams are whole lines.
 template <typename T>

@@ -1,0 +1,402 @@
+// Int4 products whose weights are expanded into tensor memory, sm_100a: routed experts of many rows.
+//
+//   C[t, n] = act(X[t, :] W[n, :]^T)                                   (dual_rows == 0)
+//   C[t, i] = act(X[t, :] Wg[i, :]^T) * (X[t, :] Wu[i, :]^T)           (dual_rows == rows of the gate half)
+//
+// An expert's weights meet a few dozen rows, so the expansion of the weights, not the products, is the work: about 15
+// instructions per eight weights (shift, mask, subtract, multiply), half of them on the half-rate integer pipe.  awq_gemm.cu writes
+// the expanded tile to shared memory, which costs a proxy fence per 64 values and leaves room for two tiles; its eight
+// converting warps then wait on one another most of the time.  Here an expanded tile is operand A of tcgen05.mma in tensor memory:
+//
+//   * a thread owns one weight row, 64 values of which are the 32 registers of one tcgen05.st: no bank conflicts, no proxy fence
+//   * tensor memory holds four units of 2 x 128 rows x 64 values beside two accumulators of 2 x 128 rows (gate | up, or 256 rows)
+//   * sixteen converting warps, four to a scheduler, in four groups of four (the quarters of tensor memory); a group takes every
+//     fourth k-block.  Group scales and zero points arrive by TMA beside the packed weights, so that a converting warp reads nothing
+//     but shared memory
+//   * CTAs are persistent: a tile's epilogue runs under the next tile's products
+//
+// Measured (one B200, us of both products, gather and sum; awq_gemm.cu or skinny_gemm.cu before; the stream of the weights alone at 6.46
+// TB/s): 128 experts of 2816 x 704, groups of 32, 8 per token: 768 tokens 470 -> 207 (66), 256 419 -> 172, 32 154 -> 136 (57); 64 of
+// 2048 x 1408, groups of 128, 6 per token: 256 tokens 298 -> 130 (45).  Of the gate and up product at 768 tokens (117 us) conversion
+// takes 25, products 10, the loads alone 84: packed weights and tokens together come near what L2 delivers to an SM.
+//
+// Roles: warp 0 weights (TMA), warp 1 MMA issuer and owner of tensor memory, warp 2 tokens (TMA), warps 3..6 epilogue,
+// warps 7..22 conversion.  Every wait is bounded; a timeout records a status code and the kernel winds down normally.
+#include "../common/launch.cuh"
+#include "../common/tensormap.h"
+#include "comm_desc.h"
+#include "persistent.cuh"
+
+using namespace fi;
+
+namespace {
+
+constexpr int kBlock = 64;             // k-block: 64 values, 128 bytes of a token row
+constexpr int kRawBlocks = 4;          // k-blocks per stage of packed weights: 128 bytes of each row
+constexpr int kGroups = 4;             // groups of four converting warps
+constexpr int kEpilogueWarps = 4;
+constexpr int kConvert = 3 + kEpilogueWarps;          // first converting warp
+constexpr int kThreads = 32 * (kConvert + 4 * kGroups);
+
+template <typename T> struct Expand;
+template <> struct Expand<__nv_bfloat16> {
+  using v2 = __nv_bfloat162;
+  static constexpr uint32_t kMagic2 = 0x43004300u;   // bf16 128 in both halves: (q | magic) = 128 + q
+};
+template <> struct Expand<__half> {
+  using v2 = __half2;
+  static constexpr uint32_t kMagic2 = 0x64006400u;   // fp16 1024
+};
+
+// The eight values of a packed word as 16-bit numbers (q - z) * s: the same operations, so the same bits, as in awq_gemm.cu.
+template <typename T>
+__device__ __forceinline__ void expand_word(uint32_t w, uint32_t z2, uint32_t s2, uint32_t* out) {
+  using v2 = typename Expand<T>::v2;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    uint32_t m;
+    asm("lop3.b32 %0, %1, 0x000F000F, %2, 0xEA;" : "=r"(m) : "r"(w >> (4 * i)), "r"(Expand<T>::kMagic2));
+    const v2 y = __hmul2(__hsub2(*reinterpret_cast<const v2*>(&m), *reinterpret_cast<const v2*>(&z2)), *reinterpret_cast<const v2*>(&s2));
+    out[i] = *reinterpret_cast<const uint32_t*>(&y);
+  }
+}
+
+__device__ __forceinline__ uint4 lds128(uint32_t at) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds16(uint32_t at) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(at));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds8(uint32_t at) {
+  uint32_t v;
+  asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(at));
+  return v;
+}
+
+template <int BN, int RST, int TST>
+struct Layout {
+  static constexpr int kPacked = kTileRows * 32 * kRawBlocks;      // one tile of a raw stage
+  static constexpr int kScales = kTileRows * 8 * 2;                // up to eight groups of 32 in 256 values
+  static constexpr int kZeros = kTileRows * 8;
+  static constexpr int kRaw = 2 * (kPacked + kScales + kZeros);    // [packed a, b][scales a, b][zeros a, b]
+  static constexpr int kTokens = BN * 128;
+  static constexpr int kBars = 512;
+  static constexpr int kBytes = RST * kRaw + TST * kTokens + kBars + kEpilogueWarps * kPatchFloats * 4 + 1024;
+  static_assert(kRaw % 1024 == 0 && kTokens % 1024 == 0, "swizzled tiles start on 1024 bytes");
+};
+
+template <typename T, int BN, int RST, int TST, bool ZEROS>
+__global__ void __launch_bounds__(kThreads, 1)
+int4_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
+                 const __grid_constant__ CUtensorMap tmap_s, const __grid_constant__ CUtensorMap tmap_z, const PersistentParams p,
+                 const int group_shift) {
+  using L = Layout<BN, RST, TST>;
+  constexpr int ACC_COLS = 2 * BN;
+  constexpr uint32_t A_COL = 2 * ACC_COLS;               // the A units lie behind the accumulators
+  static_assert(2 * ACC_COLS + kGroups * 64 <= 512 && BN % 16 == 0, "tensor memory");
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* raw_ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t* tok_ring = raw_ring + RST * L::kRaw;
+  uint64_t* raw_full = reinterpret_cast<uint64_t*>(tok_ring + TST * L::kTokens);
+  uint64_t* raw_empty = raw_full + RST;
+  uint64_t* tok_full = raw_empty + RST;
+  uint64_t* tok_empty = tok_full + TST;
+  uint64_t* a_full = tok_empty + TST;
+  uint64_t* a_empty = a_full + kGroups;
+  uint64_t* acc_full = a_empty + kGroups;          // [2]
+  uint64_t* acc_empty = acc_full + 2;          // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  volatile int* aborted = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  static_assert((2 * RST + 2 * TST + 2 * kGroups + 4) * 8 + 8 <= L::kBars, "barrier block");
+  float* patches = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(raw_full) + L::kBars);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < RST; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 4 * kGroups); }
+    for (int s = 0; s < TST; ++s) { mbar_init(&tok_full[s], 1); mbar_init(&tok_empty[s], 1); }
+    for (int s = 0; s < kGroups; ++s) { mbar_init(&a_full[s], 4); mbar_init(&a_empty[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], kEpilogueWarps); }
+    *aborted = 0;
+    mbar_fence_init();
+  }
+  // All 512 columns: the kernel in front must not find them taken by a CTA that waits for it, so the wait comes first and the
+  // kernels behind may start only when the columns are held here.
+  pdl_wait();
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();
+
+  const int kb_total = p.K / kBlock;
+  const int raw_total = (kb_total + kRawBlocks - 1) / kRawBlocks;
+  const int n_tiles = *p.tiles * p.n_tiles_n;
+  const int n_token_tiles = n_tiles / p.n_tiles_n;
+  // tile of this CTA's turn w: back and forth over the CTAs, so that who starts a round early ends the next one late
+  auto place = [&](int w) { return w * static_cast<int>(gridDim.x) + static_cast<int>((w & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x); };
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ packed weights, scales, zero points
+    if (elect_one()) {
+      tma_prefetch_desc(&tmap_w);
+      tma_prefetch_desc(&tmap_s);
+      const uint32_t meta_rows = static_cast<uint32_t>((kRawBlocks * kBlock) >> group_shift);
+      const uint32_t bytes = 2 * (L::kPacked + kTileRows * meta_rows * (ZEROS ? 3 : 2));
+      int s = 0;
+      uint32_t ph = 1;
+      for (int tile = blockIdx.x, w = 0; tile < n_tiles && !*aborted; tile = place(++w)) {
+        int nt, tt;
+        tile_at(p, tile, n_token_tiles, &nt, &tt);
+        const int n0 = nt * p.rows_per_tile + p.tile_expert[tt] * p.expert_rows;
+        for (int rs = 0; rs < raw_total; ++rs) {
+          if (!mbar_wait(&raw_empty[s], ph)) {
+            set_status(p.status, kStatusTimeoutEmpty);
+            *aborted = 1;
+            break;
+          }
+          uint8_t* r = raw_ring + s * L::kRaw;
+          mbar_expect_tx(&raw_full[s], bytes);
+          const int g0 = (rs * kRawBlocks * kBlock) >> group_shift;
+#pragma unroll
+          for (int a = 0; a < 2; ++a) {
+            const int row = n0 + a * p.second_off;
+            tma_load_2d(r + a * L::kPacked, &tmap_w, &raw_full[s], rs * 8 * kRawBlocks, row);
+            tma_load_2d(r + 2 * L::kPacked + a * L::kScales, &tmap_s, &raw_full[s], row, g0);
+            if (ZEROS) tma_load_2d(r + 2 * (L::kPacked + L::kScales) + a * L::kZeros, &tmap_z, &raw_full[s], row, g0);
+          }
+          if (++s == RST) { s = 0; ph ^= 1; }
+        }
+      }
+    }
+  } else if (warp == 2) {
+    // ------------------------------------------------------------ token tiles
+    if (elect_one()) {
+      tma_prefetch_desc(&tmap_x);
+      int s = 0;
+      uint32_t ph = 1;
+      for (int tile = blockIdx.x, w = 0; tile < n_tiles && !*aborted; tile = place(++w)) {
+        int nt, tt;
+        tile_at(p, tile, n_token_tiles, &nt, &tt);
+        const int t0 = p.tile_row0[tt];
+        for (int kb = 0; kb < kb_total; ++kb) {
+          if (!mbar_wait(&tok_empty[s], ph)) {
+            set_status(p.status, kStatusTimeoutEmpty);
+            *aborted = 1;
+            break;
+          }
+          mbar_expect_tx(&tok_full[s], L::kTokens);
+          tma_load_2d(tok_ring + s * L::kTokens, &tmap_x, &tok_full[s], kb * kBlock, t0);
+          if (++s == TST) { s = 0; ph ^= 1; }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMA issuer
+    if (elect_one()) {
+      const uint32_t idesc = umma_idesc_f16(p.is_fp16 ? 0 : 1, kTileRows, BN);
+      int ts = 0, local = 0;
+      uint32_t tph = 0, kbg = 0;            // kbg: k-blocks so far
+      for (int tile = blockIdx.x; tile < n_tiles && !*aborted; tile = place(++local)) {
+        const int b = local & 1;
+        bool ok = mbar_wait(&acc_empty[b], ((static_cast<uint32_t>(local) >> 1) & 1u) ^ 1u);
+        if (!ok) set_status(p.status, kStatusTimeoutAccum);
+        tc_fence_after();
+        const uint32_t acc = tmem_base + static_cast<uint32_t>(b * ACC_COLS);
+        for (int kb = 0; kb < kb_total && ok; ++kb) {
+          ok = mbar_wait(&tok_full[ts], tph);
+          const uint64_t db = umma_desc_sw128_kmajor(smem_u32(tok_ring + ts * L::kTokens));
+          const uint32_t u = kbg & (kGroups - 1), at = tmem_base + A_COL + u * 64;
+          ok = ok && mbar_wait(&a_full[u], (kbg / kGroups) & 1u);
+          if (ok) {
+            tc_fence_after();
+            // the two accumulators in turn: a product that follows one into the same accumulator waits some 40 cycles for it
+#pragma unroll
+            for (int k = 0; k < kBlock / 16; ++k)
+#pragma unroll
+              for (int a = 0; a < 2; ++a)
+                umma_f16_a_tmem(acc + a * BN, at + a * 32 + k * 8, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+            umma_commit(&a_empty[u]);
+            ++kbg;
+          }
+          if (!ok) { set_status(p.status, kStatusTimeoutFull); break; }
+          umma_commit(&tok_empty[ts]);
+          if (++ts == TST) { ts = 0; tph ^= 1; }
+        }
+        if (!ok) { *aborted = 1; break; }
+        umma_commit(&acc_full[b]);
+      }
+    }
+  } else if (warp >= kConvert) {
+    // ------------------------------------------------------------ conversion
+    // A group takes every fourth k-block, both halves of it (gate and up, or first and second 128 rows), and has a unit of 64
+    // columns for itself.  Its first half is expanded while the products of its last k-block still run.
+    const int group = (warp - kConvert) >> 2, q = warp & 3, row = q * 32 + lane;
+    const uint32_t unit = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + A_COL + group * 64;
+    const uint32_t raw0 = smem_u32(raw_ring);
+    const uint32_t at_packed = row * 128, sw = static_cast<uint32_t>(row & 7) << 4;
+    const uint32_t at_scale = 2 * L::kPacked + row * 2, at_zero = 2 * (L::kPacked + L::kScales) + row;
+    const int half_group = group_shift == 5 ? 1 : 0;      // groups of 32: the second half of a k-block has its own
+    int s = 0;
+    uint32_t ph = 0, kb_base = 0, turn_ph = 1;             // kb_base: k-blocks of all raw stages so far
+    bool ok = true;
+    for (int tile = blockIdx.x, w = 0; tile < n_tiles && ok; tile = place(++w)) {
+      int nt, tt;
+      tile_at(p, tile, n_token_tiles, &nt, &tt);
+      // rows past the end are not converted (their accumulators are never stored): the last tile of 704 rows is half empty
+      const int n_warp = nt * p.rows_per_tile + q * 32;
+      const bool on0 = n_warp < p.N, on1 = n_warp + (p.dual_rows > 0 ? 0 : kTileRows) < p.N;
+      for (int rs = 0; rs < raw_total && ok; ++rs) {
+        const int here = min(kRawBlocks, kb_total - rs * kRawBlocks);
+        const int sub = static_cast<int>((group - kb_base) & (kGroups - 1));
+        if (!mbar_wait(&raw_full[s], ph)) { ok = false; break; }
+        if (sub < here) {
+          const uint32_t r = raw0 + s * L::kRaw;
+          const int g0 = (sub * kBlock) >> group_shift;
+          auto expand = [&](int a, uint32_t* v) {
+            const uint32_t at = r + at_packed + a * L::kPacked, s_at = r + at_scale + a * L::kScales + g0 * (kTileRows * 2);
+            const uint4 lo = lds128(at + ((sub * 32) ^ sw)), hi = lds128(at + ((sub * 32 + 16) ^ sw));
+            const uint32_t s0 = lds16(s_at) * 0x00010001u, s1 = lds16(s_at + half_group * (kTileRows * 2)) * 0x00010001u;
+            uint32_t z0 = Expand<T>::kMagic2 + 0x00080008u, z1 = z0;
+            if constexpr (ZEROS) {
+              const uint32_t z_at = r + at_zero + a * L::kZeros + g0 * kTileRows;
+              z0 = Expand<T>::kMagic2 + lds8(z_at) * 0x00010001u;
+              z1 = Expand<T>::kMagic2 + lds8(z_at + half_group * kTileRows) * 0x00010001u;
+            }
+            expand_word<T>(lo.x, z0, s0, v);
+            expand_word<T>(lo.y, z0, s0, v + 4);
+            expand_word<T>(lo.z, z0, s0, v + 8);
+            expand_word<T>(lo.w, z0, s0, v + 12);
+            expand_word<T>(hi.x, z1, s1, v + 16);
+            expand_word<T>(hi.y, z1, s1, v + 20);
+            expand_word<T>(hi.z, z1, s1, v + 24);
+            expand_word<T>(hi.w, z1, s1, v + 28);
+          };
+          uint32_t v[32];
+          if (on0) expand(0, v);
+          if (!mbar_wait(&a_empty[group], turn_ph)) { ok = false; break; }
+          turn_ph ^= 1;
+          tc_fence_after();
+          if (on0) tmem_st_x32(unit, v);
+          if (on1) {
+            uint32_t v1[32];
+            expand(1, v1);
+            tmem_st_x32(unit + 32, v1);
+          }
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&a_full[group]);
+        }
+        kb_base += here;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&raw_empty[s]);
+        if (++s == RST) { s = 0; ph ^= 1; }
+      }
+    }
+    if (!ok) {
+      set_status(p.status, kStatusTimeoutFull);
+      *aborted = 1;
+    }
+  } else {
+    // ------------------------------------------------------------ epilogue
+    const int q = warp & 3;
+    int local = 0;
+    for (int tile = blockIdx.x; tile < n_tiles; tile = place(++local)) {
+      const int b = local & 1;
+      if (*aborted || !mbar_wait(&acc_full[b], (static_cast<uint32_t>(local) >> 1) & 1u)) {
+        if (!*aborted) { set_status(p.status, kStatusTimeoutAccum); *aborted = 1; }
+        break;
+      }
+      tc_fence_after();
+      int nt, tt;
+      tile_at(p, tile, n_token_tiles, &nt, &tt);
+      const int t0 = p.tile_row0[tt];
+      drain_tile<BN, true>(p, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(b * ACC_COLS),
+                           patches + q * kPatchFloats, nt * p.rows_per_tile, t0, t0 + p.tile_rows[tt], 0, BN, q, lane);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[b]);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+template <typename T, int BN, int RST, int TST>
+int launch(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& ts, const CUtensorMap& tz, const PersistentParams& p,
+           int group_shift, bool with_zeros, int sms, cudaStream_t stream) {
+  auto kern = with_zeros ? int4_tmem_kernel<T, BN, RST, TST, true> : int4_tmem_kernel<T, BN, RST, TST, false>;
+  constexpr int smem = Layout<BN, RST, TST>::kBytes;
+  static_assert(smem <= 227 * 1024, "shared memory of one SM");
+  const cudaError_t e = fi::ensure_dynamic_smem(kern, smem);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  const int grid = p.n_tiles < sms ? p.n_tiles : sms;
+  return static_cast<int>(launch_kernel(kern, dim3(grid), dim3(kThreads), smem, stream, 0, tw, tx, ts, tz, p, group_shift));
+}
+
+inline int sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v > 0 ? v : 148;
+  }();
+  return n;
+}
+
+}  // namespace
+
+// Routed int4 experts of many rows: X [n_rows, K] (pitch ldx) sorted by expert, weights of all experts stacked in the layout of
+// awq_gemm.cu; C [n_rows, ldc].  Gated mode (dual_rows > 0): an expert's rows are [gate; up] and N == dual_rows.  bn: rows of the tile
+// table, 16, 32 or 64.  Returns -12 where the operands are outside what this kernel takes (the caller then uses awq_gemm.cu).
+extern "C" int fi_int4_tmem_grouped(const void* X, const void* qw, const void* scales, const void* zeros, void* C, int n_rows, int N,
+                                    int K, int group, int ldx, int ldc, int act, int dual_rows, int dtype, int bn, const FiGrouped* g,
+                                    int* status, void* stream) {
+  if (n_rows <= 0 || N <= 0 || K <= 0 || g->max_tiles <= 0) return 0;
+  if (dual_rows > 0 && N != dual_rows) return -11;
+  // the scales' boxes start at weight rows: whole 16-byte groups of 16-bit scales and 8-bit zero points
+  const int unit = zeros != nullptr ? 16 : 8;
+  if ((group != 32 && group != 64 && group != 128) || (K % 64) != 0 || (N % 8) != 0 || (ldx % 8) != 0 || (ldc % 8) != 0 ||
+      g->expert_rows % unit != 0 || dual_rows % unit != 0 || (reinterpret_cast<uintptr_t>(C) & 15) != 0 || (bn != 16 && bn != 32 && bn != 64))
+    return -12;
+  const uint64_t rows = static_cast<uint64_t>(g->num_experts) * g->expert_rows, groups = (K + group - 1) / group;
+  const uint32_t meta_rows = kRawBlocks * kBlock / group;
+  CUtensorMap tw, tx, ts, tz;
+  if (make_tmap_packed(&tw, qw, rows, K / 8, kRawBlocks) != 0 || make_tmap_2d_16bit_sw128(&tx, X, n_rows, K, ldx, bn) != 0 ||
+      make_tmap_plain(&ts, scales, groups, rows, 2, kTileRows, meta_rows) != 0)
+    return -12;
+  tz = ts;
+  if (zeros != nullptr && make_tmap_plain(&tz, zeros, groups, rows, 1, kTileRows, meta_rows) != 0) return -12;
+  PersistentParams p = {};
+  p.C = C; p.T = n_rows; p.N = N; p.K = K; p.ldc = ldc; p.dual_rows = dual_rows; p.act = act; p.is_fp16 = dtype == 1;
+  p.second_off = dual_rows > 0 ? dual_rows : kTileRows;
+  p.rows_per_tile = dual_rows > 0 ? kTileRows : 2 * kTileRows;
+  p.n_tiles_n = (N + p.rows_per_tile - 1) / p.rows_per_tile;
+  p.n_tiles = p.n_tiles_n * g->max_tiles;
+  p.n_group = 1;          // all experts' first tiles, their second ones, ...: a last tile with few rows comes last
+  p.tile_expert = g->tile_expert; p.tile_row0 = g->tile_row0; p.tile_rows = g->tile_rows; p.tiles = g->n_tiles;
+  p.expert_rows = g->expert_rows; p.status = status;
+  const int shift = group == 32 ? 5 : group == 64 ? 6 : 7;
+  const bool wz = zeros != nullptr;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (bn == 16)
+    return dtype == 1 ? launch<__half, 16, 4, 16>(tw, tx, ts, tz, p, shift, wz, sm_count(), s)
+                      : launch<__nv_bfloat16, 16, 4, 16>(tw, tx, ts, tz, p, shift, wz, sm_count(), s);
+  if (bn == 32)
+    return dtype == 1 ? launch<__half, 32, 4, 12>(tw, tx, ts, tz, p, shift, wz, sm_count(), s)
+                      : launch<__nv_bfloat16, 32, 4, 12>(tw, tx, ts, tz, p, shift, wz, sm_count(), s);
+  return dtype == 1 ? launch<__half, 64, 4, 8>(tw, tx, ts, tz, p, shift, wz, sm_count(), s)
+                    : launch<__nv_bfloat16, 64, 4, 8>(tw, tx, ts, tz, p, shift, wz, sm_count(), s);
+}

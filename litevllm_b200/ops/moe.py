@@ -259,6 +259,34 @@ def _reference_experts(x, w_gate_up: Int4Weight, w_down: Int4Weight, ids, weight
     return out.to(x.dtype)
 
 
+def _few_rows(mean: int, H: int, inter: int) -> bool:
+    """An expert sees a few rows, its product streams weights (skinny_gemm.cu).  us before / now over 9 layers' sizes (8 to 256
+    experts, widths 704 to 4096, 1 to 15 rows each): 1.1 to 2.8 times as fast, level with 12 and more rows of wide experts
+    (8 experts of 4096 x 1408 76 / 78); 16 experts of 4096 x 4096 281 / 269 with 8 rows, 281 / 298 with 12."""
+    return mean < (10 if min(H, inter) >= 4096 else 16)
+
+
+def _tmem_takes(w_gate_up: Int4Weight, w_down: Int4Weight, H: int, inter: int) -> bool:
+    """Whether int4_tmem.cu takes both products: its boxes of scales and zero points start on whole 16-byte groups."""
+    return H % 16 == 0 and inter % 16 == 0 and all(
+        w.group in (32, 64, 128) and all(t is None or t.data_ptr() % 16 == 0 for t in (w.qw, w.scales_t, w.zeros_t))
+        for w in (w_gate_up, w_down))
+
+
+# From this many routes on experts take int4_tmem.cu, below it skinny_gemm.cu, which spreads the rows of few experts over all SMs.  us of
+# the layer there / in int4_tmem.cu: 128 experts of 2816 x 704 with 8 of them per token 30 / 35 at 8 routes, 52 / 43 at 24, 79 / 70 at 48,
+# 154 / 136 at 256; 8 of 4096 x 1408 27 / 44 at 2, 47 / 50 at 24, 60 / 50 at 32; 16 of 4096 x 4096 111 / 134 at 16, 143 / 154 at 24,
+# 146 / 133 at 32; 256 of 2048 x 1024 54 / 55 at 24, 69 / 57 at 32; 32 of 1024 x 512 18 / 24 at 24, 26 / 25 at 32.
+_TMEM_MIN_ROUTES = 32
+
+
+def _tmem_tile(mean: int) -> int:
+    """Rows per tile of int4_tmem.cu by the mean number of rows per expert: an expert that needs a second tile has its weights expanded twice.
+    us with tiles of 16, 32 and 64 rows (128 experts of 2816 x 704): 164, 167, 170 at 8 rows each, 170, 169, 173 at 12, 279, 179, 181 at
+    24, 331, 227, 190 at 32, 446, 302, 207 at 48; 64 experts of 2048 x 1408: 116, 118, 121 at 9, 130, 121, 126 at 12, 200, 138, 130 at 24."""
+    return 16 if mean < 11 else 32 if mean < 22 else 64
+
+
 def fused_expert_rows(x: torch.Tensor, w_gate_up: Int4Weight, w_down: Int4Weight, ids: torch.Tensor, weights: torch.Tensor,
                       num_experts_local: int, e_lo: int, act: str = "gelu_tanh") -> RoutedRows:
     """:func:`fused_experts` before its sum (CUDA): the rows live in scratch until the next call on the stream."""
@@ -270,11 +298,12 @@ def fused_expert_rows(x: torch.Tensor, w_gate_up: Int4Weight, w_down: Int4Weight
         raise RuntimeError("expert weights are not in the device runtime layout (were they loaded on the CPU?)")
     n = T * K
     mean = n // max(num_experts_local, 1)
-    # decode steps: an expert sees a few rows, its product streams weights (skinny_gemm.cu).  us before / now over 9 layers' sizes (8 to 256
-    # experts, widths 704 to 4096, 1 to 15 rows each): 1.1 to 2.8 times as fast, level with 12 and more rows of wide experts
-    # (8 experts of 4096 x 1408 76 / 78); 16 experts of 4096 x 4096 281 / 269 with 8 rows, 281 / 298 with 12
-    few = mean < (10 if min(H, inter) >= 4096 else 16) and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
-    bn = 8 if few and mean < 4 else 16 if mean < 16 else 32 if mean < 48 else 64
+    few = _few_rows(mean, H, inter)
+    tmem = _tmem_tile(mean) if (n >= _TMEM_MIN_ROUTES or not few) and _tmem_takes(w_gate_up, w_down, H, inter) else 0
+    few = few and not tmem and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
+    if not few and (not x.is_contiguous() or x.data_ptr() % 16):        # the gather reads whole rows in 16-byte groups
+        x = x.clone(memory_format=torch.contiguous_format)
+    bn = tmem or (8 if few and mean < 4 else 16 if mean < 16 else 32 if mean < 48 else 64)
     max_tiles = min(n, num_experts_local + (n + bn - 1) // bn)
     dev = x.device
     ints = scratch("moe_ints", (2 * n + num_experts_local + 1 + 3 * max_tiles + 8) * 4, dev).view(torch.int32)
@@ -312,14 +341,22 @@ def fused_expert_rows(x: torch.Tensor, w_gate_up: Int4Weight, w_down: Int4Weight
     else:
         rc = lib.fi_moe_gather(_p(x), _p(sorted_route), _p(offsets), num_experts_local, n, K, H, _p(x_sorted), dt, st)
         _lib.check(rc, "fi_moe_gather")
-        rc = lib.fi_awq_gemm_grouped(_p(x_sorted), _p(w_gate_up.qw), _p(w_gate_up.scales_t), _p(w_gate_up.zeros_t),
-                                     _p(a_sorted), None, None, n, inter, H, w_gate_up.group, H, inter, _ACT[act], inter,
-                                     0, dt, 1, bn, sw, st, ctypes.byref(g))
-        _lib.check(rc, "fi_awq_gemm_grouped(gate_up)")
-        rc = lib.fi_awq_gemm_grouped(_p(a_sorted), _p(w_down.qw), _p(w_down.scales_t), _p(w_down.zeros_t), _p(y_sorted),
-                                     None, None, n, H, inter, w_down.group, inter, H, 0, 0, 0, dt, 1, bn, sw,
-                                     st, ctypes.byref(g2))
-        _lib.check(rc, "fi_awq_gemm_grouped(down)")
+        if tmem:
+            rc = lib.fi_int4_tmem_grouped(_p(x_sorted), _p(w_gate_up.qw), _p(w_gate_up.scales_t), _p(w_gate_up.zeros_t), _p(a_sorted),
+                                          n, inter, H, w_gate_up.group, H, inter, _ACT[act], inter, dt, bn, ctypes.byref(g), sw, st)
+            _lib.check(rc, "fi_int4_tmem_grouped(gate_up)")
+            rc = lib.fi_int4_tmem_grouped(_p(a_sorted), _p(w_down.qw), _p(w_down.scales_t), _p(w_down.zeros_t), _p(y_sorted),
+                                          n, H, inter, w_down.group, inter, H, 0, 0, dt, bn, ctypes.byref(g2), sw, st)
+            _lib.check(rc, "fi_int4_tmem_grouped(down)")
+        else:
+            rc = lib.fi_awq_gemm_grouped(_p(x_sorted), _p(w_gate_up.qw), _p(w_gate_up.scales_t), _p(w_gate_up.zeros_t),
+                                         _p(a_sorted), None, None, n, inter, H, w_gate_up.group, H, inter, _ACT[act], inter,
+                                         0, dt, 1, bn, sw, st, ctypes.byref(g))
+            _lib.check(rc, "fi_awq_gemm_grouped(gate_up)")
+            rc = lib.fi_awq_gemm_grouped(_p(a_sorted), _p(w_down.qw), _p(w_down.scales_t), _p(w_down.zeros_t), _p(y_sorted),
+                                         None, None, n, H, inter, w_down.group, inter, H, 0, 0, 0, dt, 1, bn, sw,
+                                         st, ctypes.byref(g2))
+            _lib.check(rc, "fi_awq_gemm_grouped(down)")
     _count(3 if few else 4)
     return RoutedRows(y_sorted, weights, slot_of.view(T, K))
 
