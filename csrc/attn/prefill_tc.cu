@@ -32,6 +32,8 @@
 // (vllm/attention/ops/triton_prefix_prefill.py in the reference tree).
 #include <math_constants.h>
 
+#include <algorithm>
+
 #include "../common/launch.cuh"
 #include "../common/ptx.cuh"
 #include "../common/tensormap.h"
@@ -553,6 +555,432 @@ int launch_tc(const CUtensorMap& qm, const CUtensorMap& km, const CUtensorMap& v
   return static_cast<int>(ce != cudaSuccess ? ce : cudaGetLastError());
 }
 
+// ---------------------------------------------------------------------------------------------------------------------------
+// Softmax attention, two query tiles per CTA.  The exponentials bound it: 128 x 128 of them are 1024 cycles of an SM's special-function
+// units, the two products of a tile 760 (head size 64) or 1430 cycles of its tensor pipe.  With one tile per CTA the chain
+// scores - maximum - exponentials - product left both units idle half of the time (2200 cycles per tile at head size 64), and the 16-token boxes of
+// K and V kept the TMA unit busy as long as the exponentials (32 bytes per cycle).  So a CTA works on two tiles that share K and V:
+// two heads of a group with the same 128 tokens, or, where a group holds an odd number of heads, 256 tokens of one head.
+//
+//   warp 0 TMA, warp 1 UMMA, warps 2-5 softmax of the first tile, warps 6-9 of the second: on each SM sub-partition one warp of either tile,
+//   which take turns at the special-function unit (the second tile starts half a period later)
+//   * one thread per query row, all 128 scores in registers: no exchange of maxima (with two threads per row and 16 warps the
+//     hand-overs took as long as the exponentials: 4000 cycles for both tiles)
+//   * O stays in tensor memory, where PV adds up; a warp one of whose rows has a new maximum rescales it before it hands over P.  (Waiting with
+//     that until the maximum has grown by 2^8 is 12 % faster, but then the largest weight of a row is no power of two and is
+//     rounded like the others: 3 % more error.)
+//   * head size 64: scores, P and O have columns of their own (128 + 64 + 64 per tile), the scores of the next tile are under way while
+//     this one's exponentials run.  Head size 128: P lies over the scores, the next scores follow the product that reads it; the other
+//     tile's exponentials fill the time
+// us of single tiles and here (one B200; pages of 16 tokens): 2048 tokens after 2000, 32 heads on 4, head size 64: 145 -> 102; two prompts of
+// 1024: 45 -> 29; 2048 tokens, 32 heads on 8, head size 128: 93 -> 53; eight of them 603 -> 380.  What is left is the chain of one warp: the
+// special-function unit is busy 60 % of the time.
+template <int HD> struct PairSmem {
+  static constexpr int kStages = HD == 64 ? 5 : 2;
+  static constexpr int kQ = HD * 256;            // one query tile
+  static constexpr int kKV = HD * 256;           // one K or V tile
+  static constexpr int kHead = 1024;             // barriers
+  static constexpr int kBytes = kHead + 2 * kQ + 2 * kStages * kKV;
+};
+constexpr int kPairThreads = 32 * 10;
+
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n.reg .b64 x, y, z, w;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %5};\nmov.b64 z, {%6, %7};\nfma.rn.f32x2 w, x, y, z;\nmov.b64 {%0, %1}, w;\n}\n"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n.reg .b64 x, y, w;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %5};\nadd.rn.f32x2 w, x, y;\nmov.b64 {%0, %1}, w;\n}\n"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+
+template <int HD>
+__global__ void __launch_bounds__(kPairThreads, 1)
+prefill_pair_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
+                    const __grid_constant__ CUtensorMap v_map, const TcParams p, const int by_head) {
+  using L = PairSmem<HD>;
+  constexpr int STAGES = L::kStages, kAtoms = HD / 64;
+  constexpr uint32_t kTile0Cols = 256;                          // tensor memory of one query tile: scores 0..127
+  constexpr uint32_t kPCol = HD == 64 ? 128 : 0, kOCol = HD == 64 ? 192 : 128;
+  const int box_rows = min(p.block_size, kTile);
+  const int n_boxes = (kTile / box_rows) * kAtoms;
+
+  pdl_wait();          // before all 512 TMEM columns are taken, see above
+  if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) return;
+  const int b = blockIdx.z;
+  const int q_begin = p.cu_q[b], q_len = p.cu_q[b + 1] - q_begin;
+  const int tokens_here = by_head ? kTile : 2 * kTile;
+  // the tiles with the longest KV range are scheduled first
+  const int qt0 = (static_cast<int>(gridDim.y) - 1 - static_cast<int>(blockIdx.y)) * tokens_here;
+  if (qt0 >= q_len) return;
+  const int head0 = by_head ? blockIdx.x * 2 : blockIdx.x;
+  const int seq_len = p.seq_lens[b], pos0 = seq_len - q_len;
+  const bool two = by_head || qt0 + kTile < q_len;              // whether the second tile has rows
+  const int last_pos = pos0 + min(qt0 + tokens_here, q_len) - 1;
+  const int kv_lo = p.window > 0 ? max(0, pos0 + qt0 - p.window + 1) : 0;
+  const int tile_begin = kv_lo / kTile;
+  const int n_tiles = last_pos / kTile + 1 - tile_begin;
+  const int kvh = head0 / (p.nh / p.nkv);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  if ((smem_u32(smem_raw) & 1023u) != 0) {
+    if (threadIdx.x == 0) set_status(p.status, kStatusBadArg);
+    return;
+  }
+  uint8_t* sQ = smem_raw + L::kHead;
+  uint8_t* sK = sQ + 2 * L::kQ;
+  uint8_t* sV = sK + STAGES * L::kKV;
+  uint64_t* q_full = reinterpret_cast<uint64_t*>(smem_raw);
+  uint64_t* k_full = q_full + 1;
+  uint64_t* v_full = k_full + STAGES;
+  uint64_t* k_empty = v_full + STAGES;
+  uint64_t* v_empty = k_empty + STAGES;
+  // Per query tile.  Every one of these barriers completes once per KV tile, and nobody can complete it for the next one
+  // before all who wait for this one have passed, so one parity bit is enough.
+  uint64_t* s_full = v_empty + STAGES;       // [2] scores in tensor memory
+  uint64_t* s_free = s_full + 2;             // [2] scores in registers (head size 64)
+  uint64_t* p_full = s_free + 2;             // [2] probabilities in tensor memory, O rescaled
+  uint64_t* pv_done = p_full + 2;            // [2] product added to O
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
+  volatile int* aborted = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  static_assert((1 + 4 * STAGES + 8) * 8 + 8 <= L::kHead, "barrier block");
+
+  if (threadIdx.x == 0) {
+    mbar_init(q_full, 1);
+    for (int i = 0; i < STAGES; ++i) {
+      mbar_init(&k_full[i], n_boxes);         // every producer lane announces its own box
+      mbar_init(&v_full[i], n_boxes);
+      mbar_init(&k_empty[i], 1);
+      mbar_init(&v_empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&s_full[i], 1);
+      mbar_init(&s_free[i], 4);
+      mbar_init(&p_full[i], 4);
+      mbar_init(&pv_done[i], 1);
+    }
+    *aborted = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer, one lane per box as above
+    if (lane == 0) {
+      tma_prefetch_desc(&q_map);
+      mbar_expect_tx(q_full, two ? 2 * L::kQ : L::kQ);
+      for (int h = 0; h < (two ? 2 : 1); ++h)
+#pragma unroll
+        for (int a = 0; a < kAtoms; ++a)
+          tma_load_2d(sQ + h * L::kQ + a * kAtomBytes, &q_map, q_full, (head0 + (by_head ? h : 0)) * HD + a * 64,
+                      q_begin + qt0 + (by_head ? 0 : h * kTile));
+    }
+    if (lane < 2 * n_boxes) {
+      const bool is_v = lane >= n_boxes;
+      const int pg = ((lane % n_boxes) / kAtoms), a = lane % kAtoms;
+      const uint32_t box_bytes = static_cast<uint32_t>(box_rows) * 128u;
+      const CUtensorMap* map = is_v ? &v_map : &k_map;
+      uint8_t* tile0 = (is_v ? sV : sK) + a * kAtomBytes + pg * box_bytes;
+      uint64_t* full = is_v ? v_full : k_full;
+      uint64_t* empty = is_v ? v_empty : k_empty;
+      tma_prefetch_desc(map);
+      const int* bt = p.block_tables + static_cast<long>(b) * p.max_blocks;
+      auto row_of = [&](int j) -> int {
+        const int tok = (tile_begin + j) * kTile + pg * box_rows;
+        const int blk = tok < seq_len ? bt[tok / p.block_size] : 0;     // past the end: the null block
+        return (blk * p.nkv + kvh) * p.block_size + tok % p.block_size;
+      };
+      int row_next = row_of(0);
+      int issued = 0;
+      for (int j = 0; j < n_tiles; ++j) {
+        const int st = j % STAGES;
+        const int row = row_next;
+        if (j + 1 < n_tiles) row_next = row_of(j + 1);   // the page id of the next tile is in flight during the wait
+        if (!mbar_wait(&empty[st], ((j / STAGES) & 1) ^ 1)) {
+          set_status(p.status, kStatusTimeoutEmpty);
+          *aborted = 1;
+          break;
+        }
+        mbar_expect_tx(&full[st], box_bytes);
+        tma_load_2d(tile0 + st * L::kKV, map, &full[st], a * 64, row);
+        issued = j + 1;
+      }
+      // own copies in flight: the last tiles issued must have landed before the CTA may leave
+      for (int j = max(0, issued - STAGES); j < issued; ++j) {
+        if (!mbar_wait(&full[j % STAGES], (j / STAGES) & 1)) {
+          set_status(p.status, kStatusTimeoutFull);
+          break;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ UMMA issuer
+    // The tensor pipe runs the products in the order they are issued: scores of tile j+1 (over P of tile j at head size 128) come
+    // after P V of tile j there.
+    if (elect_one()) {
+      const uint32_t fmt = p.is_fp16 ? 0 : 1;
+      const uint32_t idesc_qk = umma_idesc_f16(fmt, kTile, kTile);
+      const uint32_t idesc_pv = umma_idesc_f16(fmt, kTile, HD) | kUmmaBMnMajor;
+      const int heads = two ? 2 : 1;
+      bool ok = mbar_wait(q_full, 0);
+      auto issue_qk = [&](int h, int j) {
+        const int st = j % STAGES;
+#pragma unroll
+        for (int a = 0; a < kAtoms; ++a) {
+          const uint64_t dq = umma_desc_sw128_kmajor(smem_u32(sQ + h * L::kQ + a * kAtomBytes));
+          const uint64_t dk = umma_desc_sw128_kmajor(smem_u32(sK + st * L::kKV + a * kAtomBytes));
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            umma_f16(tmem_base + h * kTile0Cols, dq + 2 * k, dk + 2 * k, idesc_qk, (a | k) != 0 ? 1u : 0u);
+        }
+        umma_commit(&s_full[h]);
+        if (h == heads - 1) umma_commit(&k_empty[st]);
+      };
+      auto issue_pv = [&](int h, int j) {
+        const int st = j % STAGES;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          // P: rows in lanes, keys [16k, 16k + 16) in 8 columns; V: 16 keys = 16 rows of 128 bytes, the second 64 channels one
+          // block of 128 rows later
+          const uint64_t dv = umma_desc_sw128_mnmajor(smem_u32(sV + st * L::kKV + k * 2048), kAtomBytes);
+          umma_f16_a_tmem(tmem_base + h * kTile0Cols + kOCol, tmem_base + h * kTile0Cols + kPCol + k * 8, dv, idesc_pv, (k | j) != 0 ? 1u : 0u);
+        }
+        umma_commit(&pv_done[h]);
+        if (h == heads - 1) umma_commit(&v_empty[st]);
+      };
+      ok = ok && mbar_wait(&k_full[0], 0);
+      tc_fence_after();
+      if (ok)
+        for (int h = 0; h < heads; ++h) issue_qk(h, 0);
+      for (int j = 0; j < n_tiles && ok; ++j) {
+        const bool more = j + 1 < n_tiles;
+        const uint32_t ph = j & 1, next_ph = ((j + 1) / STAGES) & 1;
+        if constexpr (HD == 64) {
+          if (more) {
+            ok = mbar_wait(&k_full[(j + 1) % STAGES], next_ph);
+            for (int h = 0; h < heads && ok; ++h) {
+              ok = mbar_wait(&s_free[h], ph);
+              tc_fence_after();
+              if (ok) issue_qk(h, j + 1);
+            }
+          }
+          ok = ok && mbar_wait(&v_full[j % STAGES], (j / STAGES) & 1);
+          for (int h = 0; h < heads && ok; ++h) {
+            ok = mbar_wait(&p_full[h], ph);
+            tc_fence_after();
+            if (ok) issue_pv(h, j);
+          }
+        } else {
+          ok = mbar_wait(&v_full[j % STAGES], (j / STAGES) & 1);
+          for (int h = 0; h < heads && ok; ++h) {
+            ok = mbar_wait(&p_full[h], ph);
+            tc_fence_after();
+            if (ok) issue_pv(h, j);
+            if (ok && more) {
+              if (h == 0) ok = mbar_wait(&k_full[(j + 1) % STAGES], next_ph);
+              if (ok) issue_qk(h, j + 1);
+            }
+          }
+        }
+      }
+      if (!ok) {
+        set_status(p.status, kStatusTimeoutFull);
+        *aborted = 1;
+      }
+    }
+  } else if (warp < 6 || two) {
+    // ------------------------------------------------------------------ softmax + output rows
+    const int h = warp >= 6 ? 1 : 0;
+    const int quad = warp & 3;                       // TMEM lanes this warp may read: [32 quad, 32 quad + 32)
+    const int row = quad * 32 + lane;
+    const int head = head0 + (by_head ? h : 0);
+    const int qt = qt0 + (by_head ? 0 : h * kTile);                     // first token of this tile in the sequence's new ones
+    const int rows = min(kTile, q_len - qt);
+    const int first_pos = pos0 + qt, qpos = first_pos + row, tile_last = first_pos + rows - 1;
+    const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + h * kTile0Cols;
+    const bool capped = p.softcap > 0.f;
+    const float cap_in = capped ? p.sm_scale / p.softcap : 0.f;
+    const float to_log2 = capped ? p.softcap * kLog2e : p.sm_scale * kLog2e;    // raw (or tanh'ed) score -> exponent of 2
+    float m = -CUDART_INF_F, l = 0.f;                // maximum (log2), denominator
+    bool ok = true;
+    for (int j = 0; j < n_tiles; ++j) {
+      ok = mbar_wait(&s_full[h], j & 1);
+      if (j == 0 && h == 1 && n_tiles >= 4) {        // half a period behind the first tile
+        const long long t0 = clock64();
+        while (clock64() - t0 < 1000) {}
+      }
+      if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+      tc_fence_after();
+      // this thread's 128 scores: read once, kept in registers
+      uint32_t sr[128];
+#pragma unroll
+      for (int c = 0; c < 128; c += 32) tmem_ld_x32(t_lane + c, sr + c);
+      tmem_ld_wait();
+      if constexpr (HD == 64) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_free[h]);
+      }
+      // keys of this tile the row may see: [vis_lo, vis_hi); only tiles on an edge look at them
+      const int k0 = (tile_begin + j) * kTile;
+      if (capped) {
+#pragma unroll
+        for (int e = 0; e < 128; ++e) sr[e] = __float_as_uint(fast_tanh(__uint_as_float(sr[e]) * cap_in));
+      }
+      if ((k0 + 127 > first_pos) || (p.window > 0 && k0 <= tile_last - p.window)) {
+        const int vis_hi = qpos - k0 + 1;
+        const int vis_lo = p.window > 0 ? qpos - p.window + 1 - k0 : 0;
+#pragma unroll
+        for (int e = 0; e < 128; ++e)
+          if (e < vis_lo || e >= vis_hi) sr[e] = 0xff800000u;   // -inf: probability 0
+      }
+      float mt4[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+#pragma unroll
+      for (int e = 0; e < 128; e += 8)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mt4[i] = fmaxf(fmaxf(mt4[i], __uint_as_float(sr[e + 2 * i])), __uint_as_float(sr[e + 2 * i + 1]));
+      const float mt = fmaxf(fmaxf(mt4[0], mt4[1]), fmaxf(mt4[2], mt4[3])) * to_log2;   // the factor is positive
+      bool waited = j == 0;
+      if (j == 0) {
+        m = mt;
+      } else if (__any_sync(0xffffffffu, mt > m)) {
+        const float m_new = fmaxf(m, mt);
+        const float alpha = m_new == -CUDART_INF_F ? 1.f : fast_exp2(m - m_new);
+        l *= alpha;
+        m = m_new;
+        ok = mbar_wait(&pv_done[h], (j - 1) & 1);
+        if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+        waited = true;
+        tc_fence_after();
+#pragma unroll 1
+        for (int c = 0; c < HD; c += 16) {
+          uint32_t r[16];
+          tmem_ld_x16(t_lane + kOCol + c, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * alpha);
+          tmem_st_x16(t_lane + kOCol + c, r);
+        }
+      }
+      // probabilities, packed in place (two per register): the A operand of P V, read from tensor memory
+      const float m_use = m == -CUDART_INF_F ? 0.f : m;
+      const float2 scale2 = make_float2(to_log2, to_log2), shift2 = make_float2(-m_use, -m_use);
+      float2 rs[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+      for (int e = 0; e < 128; e += 2) {
+        const float2 x = fma2(make_float2(__uint_as_float(sr[e]), __uint_as_float(sr[e + 1])), scale2, shift2);
+        const float2 y = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+        rs[(e >> 1) & 1] = add2(rs[(e >> 1) & 1], y);
+        sr[e >> 1] = pack2(y.x, y.y, p.is_fp16);
+      }
+      l += (rs[0].x + rs[1].x) + (rs[0].y + rs[1].y);
+      if (HD == 64 && !waited) {          // P of the tile in front has been read (head size 128: before these scores were made)
+        ok = mbar_wait(&pv_done[h], (j - 1) & 1);
+        if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+        tc_fence_after();
+      }
+      tmem_st_x32(t_lane + kPCol, sr);
+      tmem_st_x32(t_lane + kPCol + 32, sr + 32);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_full[h]);
+    }
+    ok = ok && mbar_wait(&pv_done[h], (n_tiles - 1) & 1);
+    if (ok) {
+      tc_fence_after();
+      if (p.x.sinks != nullptr) l += fast_exp2(fmaf(p.x.sinks[head], kLog2e, -m));     // every row sees at least its own key
+    }
+    if (__all_sync(0xffffffffu, ok)) {
+      float inv = l > 0.f ? 1.f / l : 0.f;
+      const long token = q_begin + qt + row;
+      if (p.x.gate != nullptr && p.x.gate_per_head && row < rows) {
+        const uint16_t raw = reinterpret_cast<const uint16_t*>(p.x.gate)[token * p.x.gate_stride + head];
+        const float g = p.is_fp16 ? __half2float(__ushort_as_half(raw)) : __uint_as_float(static_cast<uint32_t>(raw) << 16);
+        inv /= 1.f + __expf(-g);
+      }
+      uint16_t* dst = reinterpret_cast<uint16_t*>(p.out) + (token * p.nh + head) * p.x.out_dim;
+#pragma unroll 1
+      for (int c = 0; c < HD; c += 16) {
+        uint32_t o[16];
+        tmem_ld_x16(t_lane + kOCol + c, o);
+        tmem_ld_wait();
+        if (row >= rows) continue;
+#pragma unroll
+        for (int i = 0; i < 16; i += 8) {
+          if (c + i >= p.x.out_dim) break;
+          float y[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) y[e] = __uint_as_float(o[i + e]) * inv;
+          if (p.x.gate != nullptr && !p.x.gate_per_head) {
+            const uint4 raw = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.x.gate) + token * p.x.gate_stride +
+                                                              head * p.x.out_dim + c + i);
+            const uint32_t gw[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              float g0 = __uint_as_float(gw[e] << 16), g1 = __uint_as_float(gw[e] & 0xffff0000u);
+              if (p.is_fp16) {
+                const float2 hh = __half22float2(*reinterpret_cast<const __half2*>(&gw[e]));
+                g0 = hh.x; g1 = hh.y;
+              }
+              y[2 * e] /= 1.f + __expf(-g0);
+              y[2 * e + 1] /= 1.f + __expf(-g1);
+            }
+          }
+          *reinterpret_cast<uint4*>(dst + c + i) = make_uint4(pack2(y[0], y[1], p.is_fp16), pack2(y[2], y[3], p.is_fp16),
+                                                              pack2(y[4], y[5], p.is_fp16), pack2(y[6], y[7], p.is_fp16));
+        }
+      }
+    }
+    if (!ok) {
+      set_status(p.status, kStatusTimeoutAccum);
+      *aborted = 1;
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+template <int HD>
+int launch_pair(const CUtensorMap& qm, const CUtensorMap& km, const CUtensorMap& vm, const TcParams& p, int B, int max_q_len, cudaStream_t s) {
+  auto kern = prefill_pair_kernel<HD>;
+  constexpr int smem = PairSmem<HD>::kBytes;
+  static_assert(smem <= 227 * 1024, "shared memory of one SM");
+  cudaError_t ce = fi::ensure_dynamic_smem(kern, smem);
+  if (ce != cudaSuccess) return static_cast<int>(ce);
+  const int by_head = (p.nh / p.nkv) % 2 == 0 ? 1 : 0, tokens = by_head ? kTile : 2 * kTile;
+  ce = fi::launch_kernel(kern, dim3(by_head ? p.nh / 2 : p.nh, (max_q_len + tokens - 1) / tokens, B), dim3(kPairThreads), smem, s, 0, qm, km,
+                         vm, p, by_head);
+  return static_cast<int>(ce != cudaSuccess ? ce : cudaGetLastError());
+}
+
+inline int sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v > 0 ? v : 148;
+  }();
+  return n;
+}
+
 unsigned long long* g_tc_trace = nullptr;
 
 }  // namespace
@@ -604,7 +1032,10 @@ extern "C" int fi_paged_prefill_tc(const void* q, long q_stride, const void* k_c
   if (p.x.turn != nullptr && (reinterpret_cast<uintptr_t>(p.x.turn) & 15) != 0) return -12;
   if (p.x.bias != nullptr)
     return hd == 64 ? launch_tc<64, 6, 1, true>(qm, km, vm, p, B, max_q_len, s) : launch_tc<128, 3, 1, true>(qm, km, vm, p, B, max_q_len, s);
-  if (hd == 64)
-    return pairs ? launch_tc<64, 6, 2>(qm, km, vm, p, B, max_q_len, s) : launch_tc<64, 6, 1>(qm, km, vm, p, B, max_q_len, s);
-  return pairs ? launch_tc<128, 3, 2>(qm, km, vm, p, B, max_q_len, s) : launch_tc<128, 3, 1>(qm, km, vm, p, B, max_q_len, s);
+  // Two tiles per CTA where one per CTA would not fit the SMs at a time (us single / two: one prompt of 100 tokens, 32 heads of size 64, 6.6 / 9.4;
+  // 700 tokens, 8 heads, 12.9 / 18.7; eight prompts of 100, 32 heads of 128, 15.5 / 10.7; five of 150, 32 heads of 64, 20.1 / 16.3).
+  const long tiles = static_cast<long>(nh) * std::min<long>(static_cast<long>(B) * ((max_q_len + kTile - 1) / kTile), T_total / kTile + B);
+  if (!pairs && tiles > sm_count()) return hd == 64 ? launch_pair<64>(qm, km, vm, p, B, max_q_len, s) : launch_pair<128>(qm, km, vm, p, B, max_q_len, s);
+  if (!pairs) return hd == 64 ? launch_tc<64, 6, 1>(qm, km, vm, p, B, max_q_len, s) : launch_tc<128, 3, 1>(qm, km, vm, p, B, max_q_len, s);
+  return hd == 64 ? launch_tc<64, 6, 2>(qm, km, vm, p, B, max_q_len, s) : launch_tc<128, 3, 2>(qm, km, vm, p, B, max_q_len, s);
 }

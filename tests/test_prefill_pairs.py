@@ -1,0 +1,68 @@
+"""Prefill attention with two query tiles per CTA (csrc/attn/prefill_tc.cu) against a 64-bit oracle."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# Even groups pair two heads, odd ones two tiles of one head; every case has more tiles than SMs, so that the pairs are taken.
+# new tokens and cached ones per sequence: tiles that end inside, a second tile of one row and without rows, one key tile and many
+LENS = [(130, 0), (129, 500), (1, 700), (128, 0), (300, 333), (256, 1)]
+
+
+@pytest.mark.parametrize("nh,nkv,hd,window,softcap,dtype,extra", [
+    (64, 8, 64, 0, 0.0, torch.bfloat16, ""), (32, 16, 128, 0, 0.0, torch.float16, ""), (48, 16, 64, 200, 0.0, torch.float16, ""),
+    (48, 16, 128, 70, 0.0, torch.bfloat16, "sinks"), (32, 32, 64, 0, 20.0, torch.bfloat16, "gate"), (32, 8, 128, 150, 30.0, torch.float16, "head gate"),
+    (32, 4, 64, 0, 0.0, torch.float16, "rising"), (36, 12, 128, 0, 0.0, torch.bfloat16, "falling")])
+def test_pairs_of_tiles(nh, nkv, hd, window, softcap, dtype, extra):
+    from litevllm_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(nh + hd)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    bs, B = 16, len(LENS)
+    totals = [n + past for n, past in LENS]
+    per = (max(totals) + bs - 1) // bs
+    kc, vc = rnd(B * per + 1, nkv, bs, hd).to(dtype), rnd(B * per + 1, nkv, bs, hd).to(dtype)
+    bt = (torch.randperm(B * per, generator=g, device=DEV) + 1).view(B, per).int()
+    cu = torch.tensor([0] + [n for n, _ in LENS], device=DEV).cumsum(0).int()
+    sl = torch.tensor(totals, device=DEV, dtype=torch.int32)
+    T, scale = int(cu[-1]), hd ** -0.5
+    assert nh * ((T + 127) // 128) > 148
+    q = rnd(T, (nh + 2 * nkv) * hd).to(dtype)
+    if extra in ("rising", "falling"):      # one query direction, keys along it that grow or shrink with the position
+        d = rnd(hd)
+        q[:, :nh * hd] = (d * 3 / d.norm() * hd ** 0.25).repeat(nh).to(dtype)
+        for b in range(B):
+            step = torch.arange(per * bs, device=DEV, dtype=torch.float32) * (0.02 if extra == "rising" else -0.02)
+            kc[bt[b].long()] = (kc[bt[b].long()].float() * 0.1 + (d / d.norm() * hd ** 0.25) * step.view(per, 1, bs, 1)).to(dtype)
+    sinks = rnd(nh) if extra == "sinks" else None
+    gate = rnd(T, nh * hd).to(dtype) if extra == "gate" else rnd(T, nh).to(dtype) if extra == "head gate" else None
+    got = ops.paged_attention_prefill(q, kc, vc, bt, sl, cu, max(n for n, _ in LENS), nh, nkv, hd, scale, window, softcap,
+                                      sinks=sinks, gate=gate).double().view(T, nh, hd)
+    ops.check_status(torch.device(DEV, 0))
+    worst = 0.0
+    for b, (n, past) in enumerate(LENS):
+        lo = int(cu[b])
+        k, v = (c[bt[b].long()].permute(1, 0, 2, 3).reshape(nkv, per * bs, hd)[:, :n + past].double() for c in (kc, vc))
+        qb = q[lo:lo + n, :nh * hd].view(n, nkv, nh // nkv, hd).double()
+        s = torch.einsum("tkgd,ksd->kgts", qb, k) * scale
+        if softcap:
+            s = torch.tanh(s / softcap) * softcap
+        pos, keys = torch.arange(past, past + n, device=DEV)[:, None], torch.arange(n + past, device=DEV)
+        hidden = keys > pos
+        if window:
+            hidden |= keys <= pos - window
+        s = s.masked_fill(hidden, float("-inf"))
+        if sinks is not None:
+            s = torch.cat([s, sinks.double().view(nkv, -1, 1, 1).expand(-1, -1, n, 1)], -1)
+        w = s.softmax(-1)[..., :n + past]
+        ref = torch.einsum("kgts,ksd->tkgd", w, v).reshape(n, nh, hd)
+        size = torch.einsum("kgts,ksd->tkgd", w, v.abs()).reshape(n, nh, hd)     # what the roundings of the weights act on
+        if gate is not None:
+            f = torch.sigmoid(gate[lo:lo + n].double()).view(n, nh, -1)
+            ref, size = ref * f, size * f
+        # a weight is rounded to 16 bits (half an ulp of it), the result once more; fast tanh of the soft cap: 2^-11 of a capped score
+        eps = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+        bound = eps * (size + ref.abs()) + 1e-5 + (2.0 ** -10 * softcap * size if softcap else 0.0)
+        worst = max(worst, float(((got[lo:lo + n] - ref).abs() / bound).max()))
+    assert worst <= 1.0, worst
