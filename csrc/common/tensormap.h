@@ -63,6 +63,22 @@ inline int make_tmap_3d_16bit_sw128(CUtensorMap* out, const void* base, uint64_t
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 
+// Gated weights [2 * half, cols] (gate rows, then up rows) as tiles of eight gate rows, their eight up rows, the next eight gate rows and so
+// on: box = 128 rows of 64 columns.  half is a multiple of 8.
+inline int make_tmap_gate_up_16bit_sw128(CUtensorMap* out, const void* base, uint64_t half, uint64_t cols, uint64_t ld) {
+  EncodeTiledFn enc = get_encode_tiled();
+  if (enc == nullptr) return -1;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || ((ld * 2) & 15) != 0 || half % 8 != 0) return -2;
+  cuuint64_t dims[4] = {cols, 8, 2, half / 8};
+  cuuint64_t strides[3] = {ld * 2, half * ld * 2, 8 * ld * 2};
+  cuuint32_t box[4] = {64, 8, 2, 8};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -3;
+}
+
 // Packed weights as a 2-D int32 tensor [rows, K/8]; box = 8 * subs words x 128 rows with the swizzle of its width.
 inline int make_tmap_packed(CUtensorMap* out, const void* base, uint64_t rows, uint64_t k_words, int subs) {
   EncodeTiledFn enc = get_encode_tiled();

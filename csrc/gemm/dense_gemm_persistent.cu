@@ -216,7 +216,7 @@ int launch(const CUtensorMap& tw, const CUtensorMap& tx, const PersistentParams&
 
 }  // namespace
 
-// Prefill-sized dense GEMM (see the top of the file).  dtype: 0 bf16, 1 fp16 for X, W, bias, residual and
+// Prefill-sized dense GEMM (see the top of the file), with CTA pairs where routes.h says so.  dtype: 0 bf16, 1 fp16 for X, W, bias, residual and
 // C (C is 32-bit with out_fp32, which takes no residual).  dual_rows > 0: gated mode, W holds [gate rows; up
 // rows], bias (if any) [gate bias; up bias] and N must equal dual_rows.  Nothing is
 // allocated; returns 0, a negative argument error or a positive CUDA error code.
@@ -230,6 +230,13 @@ extern "C" int fi_dense_gemm_persistent(const void* X, const void* W, void* C, c
   if (dual_rows > 0 && N != dual_rows) return -11;
   if (act == 4 && (dual_rows <= 0 || !(act_limit > 0.f))) return -12;
   if (out_fp32 && residual != nullptr) return -13;
+  PersistentParams p = {};
+  p.C = C; p.bias = bias; p.residual = residual;
+  p.T = T; p.N = N; p.K = K; p.ldc = ldc;
+  p.dual_rows = dual_rows; p.act = act; p.act_limit = act_limit; p.is_fp16 = dtype == 1; p.out_fp32 = out_fp32;
+  p.status = status;
+  if (const int pair = pair_tokens(T, N, K, dual_rows > 0, sm_count()))
+    return dense_gemm_pair(X, W, p, ldx, ldw, pair, reinterpret_cast<cudaStream_t>(stream));
   const int w_rows = dual_rows > 0 ? 2 * dual_rows : N;
   const int tokens = persistent_tile(T, N, dual_rows > 0, sm_count()).tokens;
   CUtensorMap tw, tx;
@@ -237,10 +244,6 @@ extern "C" int fi_dense_gemm_persistent(const void* X, const void* W, void* C, c
   if (r != 0) return r * 100 - 1;
   r = make_tmap_2d_16bit_sw128(&tx, X, T, K, ldx, tokens);
   if (r != 0) return r * 100 - 2;
-  PersistentParams p = {};
-  p.C = C; p.bias = bias; p.residual = residual;
-  p.T = T; p.N = N; p.K = K; p.ldc = ldc;
-  p.dual_rows = dual_rows; p.act = act; p.act_limit = act_limit; p.is_fp16 = dtype == 1; p.out_fp32 = out_fp32;
   p.second_off = dual_rows;
   p.rows_per_tile = BM;
   p.n_tiles_n = (N + BM - 1) / BM;
@@ -248,7 +251,6 @@ extern "C" int fi_dense_gemm_persistent(const void* X, const void* W, void* C, c
   // about as many weight rows as tokens in the block of tiles in flight (tile_at)
   p.n_group = dual_rows > 0 ? 8 : 16;
   if (p.n_group > p.n_tiles_n) p.n_group = p.n_tiles_n;
-  p.status = status;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (dual_rows > 0) return tokens == 96 ? launch<4, true, 96>(tw, tx, p, s) : launch<4, true, 128>(tw, tx, p, s);
   switch (tokens) {

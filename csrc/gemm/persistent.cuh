@@ -101,6 +101,38 @@ __device__ __forceinline__ void tile_at(const PersistentParams& p, int tile, int
 
 constexpr int kPatchPitch = 36;                        // floats between the tokens of a patch: 16-byte reads of eight lanes meet no bank twice
 constexpr int kPatchFloats = 16 * kPatchPitch;
+constexpr int kPairPitch = 20;                         // the same for 32 tokens x 16 rows (drain_gate_up), the second sixteen 16 floats on
+constexpr int kPairPatchFloats = 32 * kPairPitch + 16;
+static_assert(kPairPatchFloats >= kPatchFloats, "a patch of CTA pairs serves both forms");
+
+// Eight outputs of one token: bias is in, residual (raw: eight 16-bit values) is added, the result rounded once and stored.
+__device__ __forceinline__ void store8(const PersistentParams& p, size_t off, const float4& a0, const float4& a1, const uint4& raw) {
+  if (p.out_fp32) {               // 32-bit output (no residual in this form)
+    float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.C) + off);
+    dst[0] = a0;
+    dst[1] = a1;
+    return;
+  }
+  const float v[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+  const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w};
+  uint32_t ow[4];
+  if (p.is_fp16) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 rr = __half22float2(*reinterpret_cast<const __half2*>(&rw[e]));
+      const __half2 o = __floats2half2_rn(v[2 * e] + rr.x, v[2 * e + 1] + rr.y);
+      ow[e] = *reinterpret_cast<const uint32_t*>(&o);
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const __nv_bfloat162 o = __floats2bfloat162_rn(v[2 * e] + __uint_as_float(rw[e] << 16),
+                                                     v[2 * e + 1] + __uint_as_float(rw[e] & 0xffff0000u));
+      ow[e] = *reinterpret_cast<const uint32_t*>(&o);
+    }
+  }
+  *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.C) + off) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+}
 
 // One warp's part of a finished tile: the 32 weight rows of TMEM quarter q, tokens [c_begin, c_end) of the tile whose first token is
 // t0 (rows from t_end on are not stored).  taddr: the accumulator (gated: gate rows, BN columns later the up rows; otherwise with
@@ -160,32 +192,7 @@ __device__ __forceinline__ void drain_tile(const PersistentParams& p, uint32_t t
         if (nv_ok && c0 + j < c_end) {
           const float4 a0 = *reinterpret_cast<const float4*>(patch + j * kPatchPitch + vc * 8);
           const float4 a1 = *reinterpret_cast<const float4*>(patch + j * kPatchPitch + vc * 8 + 4);
-          float v[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-          const size_t off = static_cast<size_t>(t0 + c0 + j) * p.ldc + nv;
-          if (p.out_fp32) {               // 32-bit output (no residual in this form)
-            float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.C) + off);
-            dst[0] = a0;
-            dst[1] = a1;
-            continue;
-          }
-          const uint32_t rw[4] = {res[rep].x, res[rep].y, res[rep].z, res[rep].w};
-          uint32_t ow[4];
-          if (p.is_fp16) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 rr = __half22float2(*reinterpret_cast<const __half2*>(&rw[e]));
-              const __half2 o = __floats2half2_rn(v[2 * e] + rr.x, v[2 * e + 1] + rr.y);
-              ow[e] = *reinterpret_cast<const uint32_t*>(&o);
-            }
-          } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const __nv_bfloat162 o = __floats2bfloat162_rn(v[2 * e] + __uint_as_float(rw[e] << 16),
-                                                             v[2 * e + 1] + __uint_as_float(rw[e] & 0xffff0000u));
-              ow[e] = *reinterpret_cast<const uint32_t*>(&o);
-            }
-          }
-          *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.C) + off) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+          store8(p, static_cast<size_t>(t0 + c0 + j) * p.ldc + nv, a0, a1, res[rep]);
         }
       }
       __syncwarp();
@@ -194,5 +201,53 @@ __device__ __forceinline__ void drain_tile(const PersistentParams& p, uint32_t t
     }
   }
 }
+
+// The same for a gated tile whose weight rows lie as eight gate rows, their eight up rows, and so on (make_tmap_gate_up_16bit_sw128): the
+// warp finishes 16 outputs from n on.  32 tokens at a time; lanes of gate rows take the first sixteen of them and lanes of up rows the
+// others, so that either sends its partner (lane ^ 8) what that one lacks and no lane computes in vain.
+__device__ __forceinline__ void drain_gate_up(const PersistentParams& p, uint32_t taddr, float* patch, int n, int t0, int t_end, int c_begin,
+                                              int c_end, int lane) {
+  if (n >= p.N) return;
+  c_end = min(c_end, t_end - t0);
+  const bool up = (lane & 8) != 0;
+  const int o = (lane >> 4) * 8 + (lane & 7);             // this lane's output of the 16
+  float bias_g = 0.f, bias_u = 0.f;
+  if (p.bias != nullptr && n + o < p.N) {
+    bias_g = ld16(p.bias, n + o, p.is_fp16);
+    bias_u = ld16(p.bias, p.dual_rows + n + o, p.is_fp16);
+  }
+  float* const mine = patch + (up ? 16 * kPairPitch + 16 : 0) + o;
+  const float* const token = patch + lane * kPairPitch + (lane >= 16 ? 16 : 0);
+#pragma unroll 1
+  for (int c0 = c_begin; c0 < c_end; c0 += 32) {
+    uint32_t r[32], g[16], u[16];
+    tmem_ld_x32(taddr + c0, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? r[j] : r[16 + j], 8);
+      g[j] = up ? got : r[j];
+      u[j] = up ? r[16 + j] : got;
+    }
+    act16(g, u, true, bias_g, bias_u, p.act, p.act_limit);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) mine[j * kPairPitch] = __uint_as_float(g[j]);
+    __syncwarp();
+    if (c0 + lane < c_end) {
+      const size_t off = static_cast<size_t>(t0 + c0 + lane) * p.ldc + n;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (n + h * 8 >= p.N) break;
+        uint4 raw = make_uint4(0, 0, 0, 0);
+        if (p.residual != nullptr) raw = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.residual) + off + h * 8);
+        store8(p, off + h * 8, *reinterpret_cast<const float4*>(token + h * 8), *reinterpret_cast<const float4*>(token + h * 8 + 4), raw);
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// dense_gemm_pair.cu: the product with CTA pairs, `tokens` of 128, 192 or 256 per tile.  0, or an error as in fi_dense_gemm_persistent.
+int dense_gemm_pair(const void* X, const void* W, PersistentParams p, int ldx, int ldw, int tokens, cudaStream_t stream);
 
 }  // namespace fi

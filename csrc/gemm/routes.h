@@ -50,6 +50,34 @@ inline float persistent_us(int T, int N, int K, bool gated, int sms) {
   return 3.9f + larger(loop, 0.0021f * K) + (t.waves - 1) * larger(loop, epilogue) + epilogue;
 }
 
+// Tokens per tile of dense_gemm_pair.cu, or 0 where the tiles of single CTAs stay.  Both estimates are fitted to 3520 products of 129 to 4096
+// tokens, K = 512 to 12288, 256 to 14336 outputs, plain and gated, weights cold.  A pair's tile of 256 tokens takes 0.31 us per k-block (two
+// tiles of 128 x 256 side by side 0.36), but half as many tiles fit the chip, and a pair starts 1.5 us later: 256 rows by cluster
+// launch and TMEM of both CTAs.  Taken where it promises 6 % and that: 0.947 of the time over all of these products, 0.938 with the
+// better one each time, 20 of them more than 3 % longer (the worst 21 %: 4352 rows, K = 768, 885 tokens 11.3 / 13.2).  us single /
+// pair: gated 2 x 12288 x 4096 at 2048 tokens 284 / 261, 2 x 5632 x 2048 70.1 / 65.3; plain 4096 x 12288 163 / 140, 2048 x 5632
+// 36.4 / 34.6, 2048 x 2048 (stays) 16.7 / 17.5.
+inline int pair_tokens(int T, int N, int K, bool gated, int sms) {
+  const PersistentTile one = persistent_tile(T, N, gated, sms);
+  const float loop1 = larger(2.6e-5f * one.tokens * one.cost * K * (gated ? 2 : 1), 0.00177f * K), end1 = (gated ? 0.0237f : 0.0189f) * one.tokens;
+  const float single = 2.65f + loop1 + (one.waves - 1) * larger(loop1, end1) + end1;
+  constexpr int kTokens[] = {256, 192, 128};
+  constexpr float kBlock[] = {0.31f, 0.248f, 0.208f};       // us per k-block of 64
+  int best = 0;
+  float best_us = 0.f;
+  for (int i = 0; i < 3; ++i) {
+    const long tiles = static_cast<long>(ceil_div(N, gated ? 128 : 256)) * ceil_div(T, kTokens[i]);
+    const long waves = (tiles + sms / 2 - 1) / (sms / 2);
+    const float loop = larger(ceil_div(K, 64) * kBlock[i], 0.00077f * K), end = (gated ? 0.0255f : 0.0219f) * kTokens[i];
+    const float us = 2.3f + loop + (waves - 1) * larger(loop, end) + end;
+    if (best == 0 || us < best_us) {
+      best = kTokens[i];
+      best_us = us;
+    }
+  }
+  return best_us * 1.06f + 1.5f < single ? best : 0;
+}
+
 // dense_gemm.cu, token tiles of 128: up to two CTAs per SM, few tiles split K over clusters of up to eight.  (Between one tile per
 // SM and the last split the persistent kernel was the faster one at every size tried.)
 inline float one_tile_us(int T, int N, int K, int sms) {

@@ -69,17 +69,17 @@ def _compile_one(src: Path, cmd_prefix: list[str], flags: list[str], verbose: bo
 # these into a library of their own instead of everything.
 KERNEL_SETS = {
     "fimodra": ["attn/latent_rows.cu", "attn/mla_decode.cu", "attn/paged_attention.cu", "attn/prefill_tc.cu",
-                "gemm/dense_gemm.cu", "gemm/dense_gemm_persistent.cu", "gemm/skinny_gemm.cu", "linear_attn/hgrn2.cu",
+                "gemm/dense_gemm.cu", "gemm/dense_gemm_pair.cu", "gemm/dense_gemm_persistent.cu", "gemm/skinny_gemm.cu", "linear_attn/hgrn2.cu",
                 "misc/norm_rope_misc.cu", "misc/residual_stream.cu", "misc/sampling.cu"],
     "pofadra": ["attn/latent_rows.cu", "attn/paged_attention.cu", "attn/prefill_tc.cu", "attn/qk_prepare.cu",
-                "gemm/dense_gemm.cu", "gemm/dense_gemm_persistent.cu", "gemm/skinny_gemm.cu", "linear_attn/channel_delta.cu",
+                "gemm/dense_gemm.cu", "gemm/dense_gemm_pair.cu", "gemm/dense_gemm_persistent.cu", "gemm/skinny_gemm.cu", "linear_attn/channel_delta.cu",
                 "linear_attn/hgrn2.cu", "misc/norm_rope_misc.cu", "misc/residual_stream.cu", "misc/sampling.cu",
                 "moe/moe_kernels.cu"],
     "luzerax": ["attn/head_prepare.cu", "attn/latent_rows.cu", "attn/paged_attention.cu", "attn/prefill_tc.cu",
-                "gemm/dense_gemm.cu", "gemm/dense_gemm_persistent.cu", "gemm/skinny_gemm.cu", "misc/norm_rope_misc.cu", "misc/residual_stream.cu",
+                "gemm/dense_gemm.cu", "gemm/dense_gemm_pair.cu", "gemm/dense_gemm_persistent.cu", "gemm/skinny_gemm.cu", "misc/norm_rope_misc.cu", "misc/residual_stream.cu",
                 "misc/sampling.cu", "moe/moe_kernels.cu"],
     "divadra": ["attn/latent_rows.cu", "attn/paged_attention.cu", "attn/prefill_tc.cu", "attn/qk_prepare.cu",
-                "gemm/dense_gemm.cu", "gemm/dense_gemm_persistent.cu", "gemm/skinny_gemm.cu", "linear_attn/decay_scan.cu", "misc/norm_rope_misc.cu",
+                "gemm/dense_gemm.cu", "gemm/dense_gemm_pair.cu", "gemm/dense_gemm_persistent.cu", "gemm/skinny_gemm.cu", "linear_attn/decay_scan.cu", "misc/norm_rope_misc.cu",
                 "misc/sampling.cu", "misc/shift_stream.cu", "moe/moe_kernels.cu"],
 }
 
