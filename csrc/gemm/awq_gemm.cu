@@ -23,6 +23,7 @@
 #include "comm_desc.h"
 #include "epilogue.cuh"
 #include "int4_stages.h"
+#include "int4_tmem.h"
 #include "routes.h"
 #include "skinny_gemm.h"
 
@@ -610,6 +611,21 @@ extern "C" int fi_int4_expand_pays(int T, int N, int K, int group, int gated) {
   return persistent_us(T, N, K, gated != 0, sms) + int4_expand_us(gated ? 2 * N : N, K, group) <= int4_fused_us(T, N, K, gated != 0, sms) ? 1 : 0;
 }
 
+// Layers of 9 to 128 tokens whose weights are expanded into tensor memory.  That kernel starts 3 to 4 us later than the others (an
+// SM to each CTA, a meeting of the CTAs that share K), and then expands 1.5 to 2.5 times as fast.  Gated products from 17 tokens on always (of
+// 2590 8 were more than 3 % slower: 0.35 of the time from 65 tokens on, 0.78 below), the others where the estimates say so (of 4700
+// 0.94 to 0.98 of the time, 114 more than 3 % slower).  us there / here: gated 2 x 12288 x 4096 29 / 25 at 16 tokens, 50 / 29 at 32, 75 / 45 at
+// 128; 4096 x 12288 25 / 19, 25 / 21, 44 / 30; 6144 x 4096 13.0 / 13.0, 18 / 15, 29 / 23; 4096 x 4096 (stays up to 64) 9.9 / 12.0, 12.9 / 14.4, 22 / 19.
+static bool int4_tmem_pays(int T, int N, int K, bool gated) {
+  if (T < 9 || T > 128) return false;
+  if (gated && T > 16) return true;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+    sms = 148;
+  const float other = T <= 16 ? int4_few_us(T, N, K, gated) : int4_split_us(T, N, K, sms);
+  return int4_tmem_us(T, N, K, gated, sms) * 1.05f + 0.3f < other;
+}
+
 // C = X dequant(Wq)^T with optional epilogue.  qw/scales/zeros in the runtime layout described at
 // the top of this file.  dtype: 0 bf16, 1 fp16 (X, scales, bias, C unless out_fp32).
 // dual_rows > 0: gated mode, the weight holds [gate rows; up rows] and N == dual_rows.
@@ -622,6 +638,11 @@ static int fi_awq_gemm_impl(const void* X, const void* qw, const void* scales, c
   if ((K % 64) != 0 || (ldc % 8) != 0 || (reinterpret_cast<uintptr_t>(C) & 15) != 0) return -10;
   if (group != 32 && group != 64 && group != 128 && !(group > 128 && group % 64 == 0)) return -13;
   if (dual_rows > 0 && N != dual_rows) return -11;
+  if (bn == 0 && splits == 0 && comm == nullptr && grp == nullptr && int4_tmem_pays(T, N, K, dual_rows > 0)) {
+    const int r = fi_int4_tmem(X, qw, scales, zeros, C, bias, residual, T, N, K, group, ldx, ldc, act, dual_rows, out_fp32, dtype, 0,
+                               T <= 16 ? 16 : T <= 32 ? 32 : 64, status, stream);
+    if (r != -12) return r;       // -12: operands that kernel does not take
+  }
   if (bn == 0 && splits == 0 && comm == nullptr && grp == nullptr && (ldx % 8) == 0 &&
       (reinterpret_cast<uintptr_t>(X) & 15) == 0 && (reinterpret_cast<uintptr_t>(qw) & 15) == 0 &&
       skinny_takes(true, false, T, N, K, dual_rows > 0)) {

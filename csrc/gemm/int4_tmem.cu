@@ -1,4 +1,4 @@
-// Int4 products whose weights are expanded into tensor memory, sm_100a: routed experts of many rows.
+// Int4 products whose weights are expanded into tensor memory, sm_100a: routed experts, and layers of 9 to 128 tokens.
 //
 //   C[t, n] = act(X[t, :] W[n, :]^T)                                   (dual_rows == 0)
 //   C[t, i] = act(X[t, :] Wg[i, :]^T) * (X[t, :] Wu[i, :]^T)           (dual_rows == rows of the gate half)
@@ -20,12 +20,18 @@
 // 2048 x 1408, groups of 128, 6 per token: 256 tokens 298 -> 130 (45).  Of the gate and up product at 768 tokens (117 us) conversion
 // takes 25, products 10, the loads alone 84: packed weights and tokens together come near what L2 delivers to an SM.
 //
+// Layers have fewer tiles than the chip has SMs: clusters of up to eight CTAs share a tile's K, stage their sums (32 bits) in shared memory and
+// each finishes a share of the tile from all of them, always in the same order.  Weights are fetched and expanded before the
+// kernel in front has ended.  (Measured: int4_tmem_pays in awq_gemm.cu.)
+//
 // Roles: warp 0 weights (TMA), warp 1 MMA issuer and owner of tensor memory, warp 2 tokens (TMA), warps 3..6 epilogue,
 // warps 7..22 conversion.  Every wait is bounded; a timeout records a status code and the kernel winds down normally.
 #include "../common/launch.cuh"
 #include "../common/tensormap.h"
 #include "comm_desc.h"
+#include "int4_tmem.h"
 #include "persistent.cuh"
+#include "routes.h"
 
 using namespace fi;
 
@@ -77,7 +83,7 @@ __device__ __forceinline__ uint32_t lds8(uint32_t at) {
   return v;
 }
 
-template <int BN, int RST, int TST>
+template <int BN, int RST, int TST, bool GROUPED>
 struct Layout {
   static constexpr int kPacked = kTileRows * 32 * kRawBlocks;      // one tile of a raw stage
   static constexpr int kScales = kTileRows * 8 * 2;                // up to eight groups of 32 in 256 values
@@ -85,16 +91,18 @@ struct Layout {
   static constexpr int kRaw = 2 * (kPacked + kScales + kZeros);    // [packed a, b][scales a, b][zeros a, b]
   static constexpr int kTokens = BN * 128;
   static constexpr int kBars = 512;
-  static constexpr int kBytes = RST * kRaw + TST * kTokens + kBars + kEpilogueWarps * kPatchFloats * 4 + 1024;
+  // sums of a split tile for the other CTAs of the cluster, [2 halves][BN tokens][128 rows]; the patches of whole tiles otherwise
+  static constexpr int kStaged = GROUPED ? 0 : 2 * BN * kTileRows * 4, kPatches = kEpilogueWarps * kPatchFloats * 4;
+  static constexpr int kBytes = RST * kRaw + TST * kTokens + kBars + (kStaged > kPatches ? kStaged : kPatches) + 1024;
   static_assert(kRaw % 1024 == 0 && kTokens % 1024 == 0, "swizzled tiles start on 1024 bytes");
 };
 
-template <typename T, int BN, int RST, int TST, bool ZEROS>
+template <typename T, int BN, int RST, int TST, bool ZEROS, bool GROUPED>
 __global__ void __launch_bounds__(kThreads, 1)
 int4_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                  const __grid_constant__ CUtensorMap tmap_s, const __grid_constant__ CUtensorMap tmap_z, const PersistentParams p,
-                 const int group_shift) {
-  using L = Layout<BN, RST, TST>;
+                 const int group_shift, const int splits) {
+  using L = Layout<BN, RST, TST, GROUPED>;
   constexpr int ACC_COLS = 2 * BN;
   constexpr uint32_t A_COL = 2 * ACC_COLS;               // the A units lie behind the accumulators
   static_assert(2 * ACC_COLS + kGroups * 64 <= 512 && BN % 16 == 0, "tensor memory");
@@ -109,9 +117,11 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   uint64_t* a_empty = a_full + kGroups;
   uint64_t* acc_full = a_empty + kGroups;          // [2]
   uint64_t* acc_empty = acc_full + 2;          // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint64_t* sums_full = acc_empty + 2;         // every CTA of the cluster has staged its sums of a tile
+  uint64_t* sums_empty = sums_full + 1;        // and has read those staged here
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sums_empty + 1);
   volatile int* aborted = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  static_assert((2 * RST + 2 * TST + 2 * kGroups + 4) * 8 + 8 <= L::kBars, "barrier block");
+  static_assert((2 * RST + 2 * TST + 2 * kGroups + 6) * 8 + 8 <= L::kBars, "barrier block");
   float* patches = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(raw_full) + L::kBars);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -120,28 +130,35 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     for (int s = 0; s < TST; ++s) { mbar_init(&tok_full[s], 1); mbar_init(&tok_empty[s], 1); }
     for (int s = 0; s < kGroups; ++s) { mbar_init(&a_full[s], 4); mbar_init(&a_empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], kEpilogueWarps); }
+    mbar_init(sums_full, kEpilogueWarps * splits);
+    mbar_init(sums_empty, kEpilogueWarps * splits);
     *aborted = 0;
     mbar_fence_init();
   }
-  // All 512 columns: the kernel in front must not find them taken by a CTA that waits for it, so the wait comes first and the
-  // kernels behind may start only when the columns are held here.
-  pdl_wait();
+  // Grouped: the table of tiles comes from the kernel in front.  Layers: only the tokens and the output wait for it, the expansion of
+  // the weights does not.  (All 512 TMEM columns are taken: kernels that use them let this one start only when they hold theirs.)
+  if constexpr (GROUPED) pdl_wait();
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
+  if (!GROUPED && splits > 1) cluster_sync();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_launch_dependents();
 
-  const int kb_total = p.K / kBlock;
-  const int raw_total = (kb_total + kRawBlocks - 1) / kRawBlocks;
-  const int n_tiles = *p.tiles * p.n_tiles_n;
+  // this CTA's part of K, in whole raw stages
+  const int rank = GROUPED ? 0 : static_cast<int>(blockIdx.x) % splits;
+  const int kb_all = p.K / kBlock, raw_all = (kb_all + kRawBlocks - 1) / kRawBlocks;
+  const int raw_first = raw_all * rank / splits, raw_total = raw_all * (rank + 1) / splits - raw_first;
+  const int kb_first = raw_first * kRawBlocks, kb_total = min(kb_all, kb_first + raw_total * kRawBlocks) - kb_first;
+  const int n_tiles = GROUPED ? *p.tiles * p.n_tiles_n : p.n_tiles;
   const int n_token_tiles = n_tiles / p.n_tiles_n;
-  // tile of this CTA's turn w: back and forth over the CTAs, so that who starts a round early ends the next one late
-  auto place = [&](int w) { return w * static_cast<int>(gridDim.x) + static_cast<int>((w & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x); };
+  // tile of this cluster's turn w: back and forth over the clusters, so that who starts a round early ends the next one late
+  const int clusters = static_cast<int>(gridDim.x) / splits, me = static_cast<int>(blockIdx.x) / splits;
+  auto place = [&](int w) { return w * clusters + ((w & 1) ? clusters - 1 - me : me); };
 
   if (warp == 0) {
     // ------------------------------------------------------------ packed weights, scales, zero points
@@ -152,10 +169,10 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       const uint32_t bytes = 2 * (L::kPacked + kTileRows * meta_rows * (ZEROS ? 3 : 2));
       int s = 0;
       uint32_t ph = 1;
-      for (int tile = blockIdx.x, w = 0; tile < n_tiles && !*aborted; tile = place(++w)) {
+      for (int tile = me, w = 0; tile < n_tiles && !*aborted; tile = place(++w)) {
         int nt, tt;
         tile_at(p, tile, n_token_tiles, &nt, &tt);
-        const int n0 = nt * p.rows_per_tile + p.tile_expert[tt] * p.expert_rows;
+        const int n0 = nt * p.rows_per_tile + (GROUPED ? p.tile_expert[tt] * p.expert_rows : 0);
         for (int rs = 0; rs < raw_total; ++rs) {
           if (!mbar_wait(&raw_empty[s], ph)) {
             set_status(p.status, kStatusTimeoutEmpty);
@@ -164,11 +181,11 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           }
           uint8_t* r = raw_ring + s * L::kRaw;
           mbar_expect_tx(&raw_full[s], bytes);
-          const int g0 = (rs * kRawBlocks * kBlock) >> group_shift;
+          const int g0 = ((raw_first + rs) * kRawBlocks * kBlock) >> group_shift;
 #pragma unroll
           for (int a = 0; a < 2; ++a) {
             const int row = n0 + a * p.second_off;
-            tma_load_2d(r + a * L::kPacked, &tmap_w, &raw_full[s], rs * 8 * kRawBlocks, row);
+            tma_load_2d(r + a * L::kPacked, &tmap_w, &raw_full[s], (raw_first + rs) * 8 * kRawBlocks, row);
             tma_load_2d(r + 2 * L::kPacked + a * L::kScales, &tmap_s, &raw_full[s], row, g0);
             if (ZEROS) tma_load_2d(r + 2 * (L::kPacked + L::kScales) + a * L::kZeros, &tmap_z, &raw_full[s], row, g0);
           }
@@ -180,12 +197,13 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     // ------------------------------------------------------------ token tiles
     if (elect_one()) {
       tma_prefetch_desc(&tmap_x);
+      if constexpr (!GROUPED) pdl_wait();
       int s = 0;
       uint32_t ph = 1;
-      for (int tile = blockIdx.x, w = 0; tile < n_tiles && !*aborted; tile = place(++w)) {
+      for (int tile = me, w = 0; tile < n_tiles && !*aborted; tile = place(++w)) {
         int nt, tt;
         tile_at(p, tile, n_token_tiles, &nt, &tt);
-        const int t0 = p.tile_row0[tt];
+        const int t0 = GROUPED ? p.tile_row0[tt] : tt * BN;
         for (int kb = 0; kb < kb_total; ++kb) {
           if (!mbar_wait(&tok_empty[s], ph)) {
             set_status(p.status, kStatusTimeoutEmpty);
@@ -193,7 +211,7 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             break;
           }
           mbar_expect_tx(&tok_full[s], L::kTokens);
-          tma_load_2d(tok_ring + s * L::kTokens, &tmap_x, &tok_full[s], kb * kBlock, t0);
+          tma_load_2d(tok_ring + s * L::kTokens, &tmap_x, &tok_full[s], (kb_first + kb) * kBlock, t0);
           if (++s == TST) { s = 0; ph ^= 1; }
         }
       }
@@ -204,7 +222,7 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       const uint32_t idesc = umma_idesc_f16(p.is_fp16 ? 0 : 1, kTileRows, BN);
       int ts = 0, local = 0;
       uint32_t tph = 0, kbg = 0;            // kbg: k-blocks so far
-      for (int tile = blockIdx.x; tile < n_tiles && !*aborted; tile = place(++local)) {
+      for (int tile = me; tile < n_tiles && !*aborted; tile = place(++local)) {
         const int b = local & 1;
         bool ok = mbar_wait(&acc_empty[b], ((static_cast<uint32_t>(local) >> 1) & 1u) ^ 1u);
         if (!ok) set_status(p.status, kStatusTimeoutAccum);
@@ -247,7 +265,7 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     int s = 0;
     uint32_t ph = 0, kb_base = 0, turn_ph = 1;             // kb_base: k-blocks of all raw stages so far
     bool ok = true;
-    for (int tile = blockIdx.x, w = 0; tile < n_tiles && ok; tile = place(++w)) {
+    for (int tile = me, w = 0; tile < n_tiles && ok; tile = place(++w)) {
       int nt, tt;
       tile_at(p, tile, n_token_tiles, &nt, &tt);
       // rows past the end are not converted (their accumulators are never stored): the last tile of 704 rows is half empty
@@ -308,8 +326,9 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   } else {
     // ------------------------------------------------------------ epilogue
     const int q = warp & 3;
+    if constexpr (!GROUPED) pdl_wait();
     int local = 0;
-    for (int tile = blockIdx.x; tile < n_tiles; tile = place(++local)) {
+    for (int tile = me; tile < n_tiles; tile = place(++local)) {
       const int b = local & 1;
       if (*aborted || !mbar_wait(&acc_full[b], (static_cast<uint32_t>(local) >> 1) & 1u)) {
         if (!*aborted) { set_status(p.status, kStatusTimeoutAccum); *aborted = 1; }
@@ -318,32 +337,99 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       tc_fence_after();
       int nt, tt;
       tile_at(p, tile, n_token_tiles, &nt, &tt);
-      const int t0 = p.tile_row0[tt];
-      drain_tile<BN, true>(p, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(b * ACC_COLS),
-                           patches + q * kPatchFloats, nt * p.rows_per_tile, t0, t0 + p.tile_rows[tt], 0, BN, q, lane);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[b]);
+      const int t0 = GROUPED ? p.tile_row0[tt] : tt * BN, t_end = GROUPED ? t0 + p.tile_rows[tt] : p.T;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(b * ACC_COLS);
+      if (GROUPED || splits == 1) {
+        drain_tile<BN, true>(p, taddr, patches + q * kPatchFloats, nt * p.rows_per_tile, t0, t_end, 0, BN, q, lane);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[b]);
+        continue;
+      }
+      if constexpr (!GROUPED) {
+        // the others have read what the last tile left here
+        bool ok = mbar_wait_cluster(sums_empty, (static_cast<uint32_t>(local) & 1u) ^ 1u);
+        float* const staged = patches + q * 32 + lane;
+        const int here = min(BN, p.T - t0);
+#pragma unroll 1
+        for (int c = 0; c < here; c += 16) {
+          uint32_t g[16], u[16];
+          tmem_ld_x16(taddr + c, g);
+          tmem_ld_x16(taddr + BN + c, u);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            staged[(c + j) * kTileRows] = __uint_as_float(g[j]);
+            staged[(BN + c + j) * kTileRows] = __uint_as_float(u[j]);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[b]);
+        if (lane < splits) mbar_arrive_cluster(cluster_addr(sums_full, lane));
+        ok = ok && mbar_wait_cluster(sums_full, static_cast<uint32_t>(local) & 1u);
+        if (!__all_sync(0xffffffffu, ok)) {
+          set_status(p.status, kStatusTimeoutPeer);
+          *aborted = 1;
+          break;
+        }
+        // this CTA's share of the tile: groups of eight rows of a token, summed over the cluster in its order
+        const bool gated = p.dual_rows > 0;
+        const int per_token = gated ? kTileRows / 8 : kTileRows / 4, items = per_token * here;
+        const int item0 = items * rank / splits, item1 = items * (rank + 1) / splits;
+        for (int item = item0 + (warp - 3) * 32 + lane; item < item1; item += 32 * kEpilogueWarps) {
+          const int tk = item / per_token, c = item % per_token;
+          const int n = nt * p.rows_per_tile + c * 8;
+          if (n >= p.N) continue;
+          float acc[2][8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[0][j] = acc[1][j] = 0.f;
+          const uint32_t at = smem_u32(patches) + (((c >> 4) * BN + tk) * kTileRows + (c & 15) * 8) * 4;
+#pragma unroll 2
+          for (int r = 0; r < splits; ++r) {
+            uint32_t remote;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(r));
+            const float4 x0 = ld_cluster_v4(remote), x1 = ld_cluster_v4(remote + 16);
+            acc[0][0] += x0.x; acc[0][1] += x0.y; acc[0][2] += x0.z; acc[0][3] += x0.w;
+            acc[0][4] += x1.x; acc[0][5] += x1.y; acc[0][6] += x1.z; acc[0][7] += x1.w;
+            if (gated) {
+              const float4 y0 = ld_cluster_v4(remote + BN * kTileRows * 4), y1 = ld_cluster_v4(remote + BN * kTileRows * 4 + 16);
+              acc[1][0] += y0.x; acc[1][1] += y0.y; acc[1][2] += y0.z; acc[1][3] += y0.w;
+              acc[1][4] += y1.x; acc[1][5] += y1.y; acc[1][6] += y1.z; acc[1][7] += y1.w;
+            }
+          }
+          uint32_t v[8], u[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            v[j] = __float_as_uint(acc[0][j]);
+            u[j] = __float_as_uint(acc[1][j]);
+            if (p.bias != nullptr && gated) {
+              v[j] = __float_as_uint(acc[0][j] + ld16(p.bias, n + j, p.is_fp16));
+              u[j] = __float_as_uint(acc[1][j] + ld16(p.bias, p.dual_rows + n + j, p.is_fp16));
+            }
+          }
+          act_all(v, u, gated, 0.f, 0.f, p.act, p.act_limit);
+          if (p.bias != nullptr && !gated)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + ld16(p.bias, n + j, p.is_fp16));
+          const size_t off = static_cast<size_t>(t0 + tk) * p.ldc + n;
+          uint4 raw = make_uint4(0, 0, 0, 0);
+          if (p.residual != nullptr) raw = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.residual) + off);
+          store8(p, off, make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), __uint_as_float(v[3])),
+                 make_float4(__uint_as_float(v[4]), __uint_as_float(v[5]), __uint_as_float(v[6]), __uint_as_float(v[7])), raw);
+        }
+        __syncwarp();
+        if (lane < splits) mbar_arrive_cluster(cluster_addr(sums_empty, lane));
+      }
     }
   }
   tc_fence_before();
   __syncthreads();
+  if (!GROUPED && splits > 1) cluster_sync();      // nobody reads sums of this CTA any more
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
-}
-
-template <typename T, int BN, int RST, int TST>
-int launch(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& ts, const CUtensorMap& tz, const PersistentParams& p,
-           int group_shift, bool with_zeros, int sms, cudaStream_t stream) {
-  auto kern = with_zeros ? int4_tmem_kernel<T, BN, RST, TST, true> : int4_tmem_kernel<T, BN, RST, TST, false>;
-  constexpr int smem = Layout<BN, RST, TST>::kBytes;
-  static_assert(smem <= 227 * 1024, "shared memory of one SM");
-  const cudaError_t e = fi::ensure_dynamic_smem(kern, smem);
-  if (e != cudaSuccess) return static_cast<int>(e);
-  const int grid = p.n_tiles < sms ? p.n_tiles : sms;
-  return static_cast<int>(launch_kernel(kern, dim3(grid), dim3(kThreads), smem, stream, 0, tw, tx, ts, tz, p, group_shift));
 }
 
 inline int sm_count() {
@@ -354,6 +440,78 @@ inline int sm_count() {
     return v > 0 ? v : 148;
   }();
   return n;
+}
+
+template <typename T, int BN, int RST, int TST>
+int launch_grouped(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& ts, const CUtensorMap& tz, const PersistentParams& p,
+                   int group_shift, bool with_zeros, cudaStream_t stream) {
+  auto kern = with_zeros ? int4_tmem_kernel<T, BN, RST, TST, true, true> : int4_tmem_kernel<T, BN, RST, TST, false, true>;
+  constexpr int smem = Layout<BN, RST, TST, true>::kBytes;
+  static_assert(smem <= 227 * 1024, "shared memory of one SM");
+  const cudaError_t e = fi::ensure_dynamic_smem(kern, smem);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  const int grid = p.n_tiles < sm_count() ? p.n_tiles : sm_count();
+  return static_cast<int>(launch_kernel(kern, dim3(grid), dim3(kThreads), smem, stream, 0, tw, tx, ts, tz, p, group_shift, 1));
+}
+
+// Clusters of S CTAs with an SM each that the chip holds at a time.
+template <typename K>
+int most_clusters(K kern, int smem, int S) {
+  if (S == 1) return sm_count();
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(sm_count() / S * S);
+  c.blockDim = dim3(kThreads);
+  c.dynamicSmemBytes = smem;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  c.attrs = at; c.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &c) != cudaSuccess || n <= 0) {
+    cudaGetLastError();
+    n = sm_count() / S * 3 / 4;
+  }
+  return n;
+}
+
+template <typename T, int BN, int RST, int TST, bool ZEROS>
+int launch_layer(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& ts, const CUtensorMap& tz, const PersistentParams& p,
+                 int group_shift, int splits, cudaStream_t stream) {
+  auto kern = int4_tmem_kernel<T, BN, RST, TST, ZEROS, false>;
+  constexpr int smem = Layout<BN, RST, TST, false>::kBytes;
+  static_assert(smem <= 227 * 1024, "shared memory of one SM");
+  const cudaError_t e = fi::ensure_dynamic_smem(kern, smem);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  static int most[9] = {0};
+  const int raw = (p.K / kBlock + kRawBlocks - 1) / kRawBlocks;
+  if (splits <= 0) {
+    float best = 0.f;
+    for (int S = 1; S <= 8 && S <= raw; ++S) {
+      if (most[S] == 0) most[S] = most_clusters(kern, smem, S);
+      // 0.39 us for two tiles of a k-block; a split tile ends with the meeting of its CTAs
+      const float us = ceil_div(p.n_tiles, most[S]) * (ceil_div(raw, S) * kRawBlocks * 0.39f + (S > 1 ? 0.4f : 0.2f)) + (S > 1 ? 1.2f : 0.6f);
+      if (splits <= 0 || us < best) { splits = S; best = us; }
+    }
+  }
+  if (most[splits] == 0) most[splits] = most_clusters(kern, smem, splits);
+  const int clusters = p.n_tiles < most[splits] ? p.n_tiles : most[splits];
+  if (splits == 1)
+    return static_cast<int>(launch_kernel(kern, dim3(clusters), dim3(kThreads), smem, stream, 0, tw, tx, ts, tz, p, group_shift, 1));
+  return static_cast<int>(launch_kernel_cluster(kern, dim3(clusters * splits), dim3(kThreads), smem, stream, dim3(splits, 1, 1), tw, tx, ts,
+                                                tz, p, group_shift, splits));
+}
+
+template <typename T>
+int layer_by_tile(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& ts, const CUtensorMap& tz, const PersistentParams& p,
+                  int group_shift, bool zeros, int bn, int splits, cudaStream_t s) {
+  if (bn == 16)
+    return zeros ? launch_layer<T, 16, 5, 8, true>(tw, tx, ts, tz, p, group_shift, splits, s)
+                 : launch_layer<T, 16, 5, 8, false>(tw, tx, ts, tz, p, group_shift, splits, s);
+  if (bn == 32)
+    return zeros ? launch_layer<T, 32, 4, 8, true>(tw, tx, ts, tz, p, group_shift, splits, s)
+                 : launch_layer<T, 32, 4, 8, false>(tw, tx, ts, tz, p, group_shift, splits, s);
+  return zeros ? launch_layer<T, 64, 3, 4, true>(tw, tx, ts, tz, p, group_shift, splits, s)
+               : launch_layer<T, 64, 3, 4, false>(tw, tx, ts, tz, p, group_shift, splits, s);
 }
 
 }  // namespace
@@ -392,11 +550,46 @@ extern "C" int fi_int4_tmem_grouped(const void* X, const void* qw, const void* s
   const bool wz = zeros != nullptr;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (bn == 16)
-    return dtype == 1 ? launch<__half, 16, 4, 16>(tw, tx, ts, tz, p, shift, wz, sm_count(), s)
-                      : launch<__nv_bfloat16, 16, 4, 16>(tw, tx, ts, tz, p, shift, wz, sm_count(), s);
+    return dtype == 1 ? launch_grouped<__half, 16, 4, 16>(tw, tx, ts, tz, p, shift, wz, s)
+                      : launch_grouped<__nv_bfloat16, 16, 4, 16>(tw, tx, ts, tz, p, shift, wz, s);
   if (bn == 32)
-    return dtype == 1 ? launch<__half, 32, 4, 12>(tw, tx, ts, tz, p, shift, wz, sm_count(), s)
-                      : launch<__nv_bfloat16, 32, 4, 12>(tw, tx, ts, tz, p, shift, wz, sm_count(), s);
-  return dtype == 1 ? launch<__half, 64, 4, 8>(tw, tx, ts, tz, p, shift, wz, sm_count(), s)
-                    : launch<__nv_bfloat16, 64, 4, 8>(tw, tx, ts, tz, p, shift, wz, sm_count(), s);
+    return dtype == 1 ? launch_grouped<__half, 32, 4, 12>(tw, tx, ts, tz, p, shift, wz, s)
+                      : launch_grouped<__nv_bfloat16, 32, 4, 12>(tw, tx, ts, tz, p, shift, wz, s);
+  return dtype == 1 ? launch_grouped<__half, 64, 4, 8>(tw, tx, ts, tz, p, shift, wz, s)
+                    : launch_grouped<__nv_bfloat16, 64, 4, 8>(tw, tx, ts, tz, p, shift, wz, s);
+}
+
+// Layers of few tokens: C [T, N] as in fi_awq_gemm (weights in its layout).  bn: tokens per tile, 16, 32 or 64; splits: CTAs that share
+// a tile's K as a cluster, 0: by size.  Returns -12 where the operands are outside what this kernel takes.
+extern "C" int fi_int4_tmem(const void* X, const void* qw, const void* scales, const void* zeros, void* C, const void* bias,
+                            const void* residual, int T, int N, int K, int group, int ldx, int ldc, int act, int dual_rows, int out_fp32,
+                            int dtype, int splits, int bn, int* status, void* stream) {
+  if (T <= 0 || N <= 0 || K <= 0) return 0;
+  if (dual_rows > 0 && N != dual_rows) return -11;
+  const int rows = dual_rows > 0 ? 2 * dual_rows : N, unit = zeros != nullptr ? 16 : 8;
+  if ((group != 32 && group != 64 && group != 128) || (K % 64) != 0 || (N % 8) != 0 || (ldx % 8) != 0 || (ldc % 8) != 0 || rows % unit != 0 ||
+      dual_rows % unit != 0 || (reinterpret_cast<uintptr_t>(C) & 15) != 0 ||
+      (residual != nullptr && (out_fp32 || (reinterpret_cast<uintptr_t>(residual) & 15) != 0)) || (bn != 16 && bn != 32 && bn != 64) ||
+      splits < 0 || splits > 8 || splits > (K / 64 + kRawBlocks - 1) / kRawBlocks)
+    return -12;
+  const uint64_t groups = (K + group - 1) / group;
+  const uint32_t meta_rows = kRawBlocks * kBlock / group;
+  CUtensorMap tw, tx, ts, tz;
+  if (make_tmap_packed(&tw, qw, rows, K / 8, kRawBlocks) != 0 || make_tmap_2d_16bit_sw128(&tx, X, T, K, ldx, bn) != 0 ||
+      make_tmap_plain(&ts, scales, groups, rows, 2, kTileRows, meta_rows) != 0)
+    return -12;
+  tz = ts;
+  if (zeros != nullptr && make_tmap_plain(&tz, zeros, groups, rows, 1, kTileRows, meta_rows) != 0) return -12;
+  PersistentParams p = {};
+  p.C = C; p.bias = bias; p.residual = residual; p.T = T; p.N = N; p.K = K; p.ldc = ldc; p.dual_rows = dual_rows; p.act = act;
+  p.is_fp16 = dtype == 1; p.out_fp32 = out_fp32; p.status = status;
+  p.second_off = dual_rows > 0 ? dual_rows : kTileRows;
+  p.rows_per_tile = dual_rows > 0 ? kTileRows : 2 * kTileRows;
+  p.n_tiles_n = (N + p.rows_per_tile - 1) / p.rows_per_tile;
+  p.n_tiles = p.n_tiles_n * ((T + bn - 1) / bn);
+  p.n_group = p.n_tiles_n;
+  const int shift = group == 32 ? 5 : group == 64 ? 6 : 7;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  return dtype == 1 ? layer_by_tile<__half>(tw, tx, ts, tz, p, shift, zeros != nullptr, bn, splits, s)
+                    : layer_by_tile<__nv_bfloat16>(tw, tx, ts, tz, p, shift, zeros != nullptr, bn, splits, s);
 }

@@ -1,0 +1,6 @@
+// Int4 layers whose weights are expanded into tensor memory (int4_tmem.cu), for the kernels that hand products over to it.
+#pragma once
+
+extern "C" int fi_int4_tmem(const void* X, const void* qw, const void* scales, const void* zeros, void* C, const void* bias,
+                            const void* residual, int T, int N, int K, int group, int ldx, int ldc, int act, int dual_rows, int out_fp32,
+                            int dtype, int splits, int bn, int* status, void* stream);

@@ -53,24 +53,25 @@ __device__ __forceinline__ float gated_f(float g, float u, float limit) {
   }
   return act_f<ACT>(g) * u;
 }
-// Sixteen channels at a time: the activation is chosen once and not for each of them.
-template <int ACT>
-__device__ __forceinline__ void act16_as(uint32_t (&r)[16], const uint32_t (&u)[16], bool gated, float bias_g, float bias_u, float limit) {
+// Several channels at a time: the activation is chosen once and not for each of them.
+template <int ACT, int M>
+__device__ __forceinline__ void act_as(uint32_t (&r)[M], const uint32_t (&u)[M], bool gated, float bias_g, float bias_u, float limit) {
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
+  for (int j = 0; j < M; ++j) {
     const float v = __uint_as_float(r[j]);
     r[j] = __float_as_uint(gated ? gated_f<ACT>(v + bias_g, __uint_as_float(u[j]) + bias_u, limit) : act_f<ACT>(v) + bias_g);
   }
 }
-__device__ __forceinline__ void act16(uint32_t (&r)[16], const uint32_t (&u)[16], bool gated, float bias_g, float bias_u, int act, float limit) {
+template <int M>
+__device__ __forceinline__ void act_all(uint32_t (&r)[M], const uint32_t (&u)[M], bool gated, float bias_g, float bias_u, int act, float limit) {
   switch (act) {
-    case 1: return act16_as<1>(r, u, gated, bias_g, bias_u, limit);
-    case 2: return act16_as<2>(r, u, gated, bias_g, bias_u, limit);
-    case 3: return act16_as<3>(r, u, gated, bias_g, bias_u, limit);
-    case 4: return act16_as<4>(r, u, gated, bias_g, bias_u, limit);
-    case 5: return act16_as<5>(r, u, gated, bias_g, bias_u, limit);
-    case 6: return act16_as<6>(r, u, gated, bias_g, bias_u, limit);
-    default: return act16_as<0>(r, u, gated, bias_g, bias_u, limit);
+    case 1: return act_as<1>(r, u, gated, bias_g, bias_u, limit);
+    case 2: return act_as<2>(r, u, gated, bias_g, bias_u, limit);
+    case 3: return act_as<3>(r, u, gated, bias_g, bias_u, limit);
+    case 4: return act_as<4>(r, u, gated, bias_g, bias_u, limit);
+    case 5: return act_as<5>(r, u, gated, bias_g, bias_u, limit);
+    case 6: return act_as<6>(r, u, gated, bias_g, bias_u, limit);
+    default: return act_as<0>(r, u, gated, bias_g, bias_u, limit);
   }
 }
 __device__ __forceinline__ float ld16(const void* p, size_t i, int is_fp16) {
@@ -182,7 +183,7 @@ __device__ __forceinline__ void drain_tile(const PersistentParams& p, uint32_t t
       if (gated) tmem_ld_x16(taddr + BN + c0, u);
       if (with_res) load_res(c0 + 16, res_next);
       tmem_ld_wait();
-      act16(r, u, gated, bias_g, bias_u, p.act, p.act_limit);
+      act_all(r, u, gated, bias_g, bias_u, p.act, p.act_limit);
 #pragma unroll
       for (int j = 0; j < 16; ++j) patch[j * kPatchPitch + lane] = __uint_as_float(r[j]);
       __syncwarp();
@@ -229,7 +230,7 @@ __device__ __forceinline__ void drain_gate_up(const PersistentParams& p, uint32_
       g[j] = up ? got : r[j];
       u[j] = up ? r[16 + j] : got;
     }
-    act16(g, u, true, bias_g, bias_u, p.act, p.act_limit);
+    act_all(g, u, true, bias_g, bias_u, p.act, p.act_limit);
 #pragma unroll
     for (int j = 0; j < 16; ++j) mine[j * kPairPitch] = __uint_as_float(g[j]);
     __syncwarp();

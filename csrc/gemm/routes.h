@@ -94,6 +94,43 @@ inline float one_tile_us(int T, int N, int K, int sms) {
   return rounds * (7.35f + 0.0071f * K);
 }
 
+// int4_tmem.cu for layers of 9 to 128 tokens (token tiles of 16, 32 and 64): clusters of `split` CTAs share a tile's K, with an SM to each
+// CTA.  Fitted, like int4_split_us, to 8000 products, K = 256 to 14336, 128 to 14336 outputs, groups of 32 and 128, weights cold.
+struct Int4Tile { float start, block, whole, part, meet; };     // us: launch and ramp, k-block of two tiles, tile whole / split, meeting
+
+inline int tmem_clusters(int split, int sms) {      // groups of SMs are no multiples of all splits
+  constexpr float kOf148[] = {148, 74, 48, 36, 28, 23, 20, 18};
+  return static_cast<int>(kOf148[split - 1] * sms / 148.f);
+}
+
+inline float int4_tmem_us(int T, int N, int K, bool gated, int sms) {
+  constexpr Int4Tile kPlain[] = {{1.05f, 0.415f, 2.0f, 1.27f, 3.4f}, {1.9f, 0.462f, 2.1f, 0.74f, 4.2f}, {4.2f, 0.466f, 1.7f, 1.f, 3.9f},
+                                 {5.7f, 0.427f, 1.4f, 0.47f, 4.2f}};
+  constexpr Int4Tile kGated = {1.3f, 0.426f, 1.76f, 1.37f, 3.1f};
+  const Int4Tile& c = gated ? kGated : kPlain[T <= 16 ? 0 : T <= 32 ? 1 : T <= 64 ? 2 : 3];
+  const int tiles = ceil_div(N, gated ? 128 : 256) * ceil_div(T, T <= 16 ? 16 : T <= 32 ? 32 : 64), raw = ceil_div(K, 256);
+  float best = 0.f;
+  for (int split = 1; split <= 8 && split <= raw; ++split) {
+    const float us = ceil_div(tiles, tmem_clusters(split, sms)) * (ceil_div(raw, split) * 4 * c.block + (split > 1 ? c.part : c.whole)) +
+                     (split > 1 ? c.meet : 0.f);
+    if (split == 1 || us < best) best = us;
+  }
+  return c.start + best;
+}
+
+// awq_gemm.cu, plain layers of 17 to 128 tokens: K split over clusters of up to eight.
+inline float int4_split_us(int T, int N, int K, int sms) {
+  struct Form { float start, k, row_k, row; };
+  constexpr Form kForms[] = {{6.1f, 0.00445f, 2.85e-5f, -0.0069f}, {6.8f, 0.00513f, 2.55e-5f, -0.0073f}, {8.8f, 0.00667f, 4.74e-5f, -0.0134f}};
+  const int rows = ceil_div(N, 128);
+  int split = ceil_div(107, rows);
+  if (split > 8) split = 8;
+  if (split > K / 128) split = K / 128 > 0 ? K / 128 : 1;
+  while (split > 1 && rows * split > 2 * sms * 19 / 20) --split;
+  const Form& f = kForms[T <= 32 ? 0 : T <= 64 ? 1 : 2];
+  return f.start + f.k * K / split + rows * (f.row_k * K + f.row);
+}
+
 // awq_gemm.cu, token tiles of 128: each tile expands its weights again; gated tiles have an SM to themselves.
 inline float int4_fused_us(int T, int N, int K, bool gated, int sms) {
   const int tiles = ceil_div(N, 128) * ceil_div(T, 128);

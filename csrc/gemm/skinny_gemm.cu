@@ -529,11 +529,11 @@ int int4_by_size(const SkinnyParams& p, cudaStream_t s) {
 // than the better kernel each time and 0.67 of awq_gemm.cu's time; 33 are more than 3 % longer than there (at most 17 %), with
 // this kernel always 259 (up to 1.7 times).  us there / here: 1024 x 12288 15 / 18 at 9 tokens, 15 / 22 at 16; 4096 x 12288 29 / 25
 // at 16; gated 2 x 8192 x 12288 71 / 91 at 16.
-bool int4_pays(int T, int N, int K, bool gated) {
+struct Int4Estimate { float here, there; bool settled; };      // settled: this kernel, whatever the estimates say
+Int4Estimate int4_estimate(int T, int N, int K, bool gated) {
   const int tiles = gated ? (N + 7) / 8 : (N + 15) / 16;
   const Shape f = T > 8 ? shape_of<true, 8, 2, 2, 2>(T, K, tiles) : tiles >= 320 ? shape_of<true, 8, 2, 1, 2>(T, K, tiles)
                                                                              : shape_of<true, 8, 1, 1, 4>(T, K, tiles);
-  if (T <= 8 && f.segs == 1) return true;
   const int rounds = (f.blocks + f.per_sm * sm_count() - 1) / (f.per_sm * sm_count());
   const float tk = static_cast<float>(T) * K;
   const float piece = f.segs == 1 ? 0.f : T > 8 ? 5.8e-5f : 2.4e-5f;        // of a token's value, staged again in each round
@@ -545,7 +545,11 @@ bool int4_pays(int T, int N, int K, bool gated) {
   while (split > 1 && rows * split > most) --split;
   const float k = static_cast<float>(K) / split;
   const float there = gated ? 8.3f + 0.0084f * k + rows * (1.67e-5f * K + 0.0011f) : 4.36f + 0.0061f * k + rows * (2.7e-5f * K + 0.0011f);
-  return here <= there;
+  return {here, there, T <= 8 && f.segs == 1};
+}
+bool int4_pays(int T, int N, int K, bool gated) {
+  const Int4Estimate e = int4_estimate(T, N, K, gated);
+  return e.settled || e.here <= e.there;
 }
 
 // 16-bit products with a fused norm: against dense_gemm.cu, whose rings stream long rows better (us there / here, one token: 6144 x
@@ -568,6 +572,11 @@ int by_kind(const SkinnyParams& p, cudaStream_t s) {
 }
 
 }  // namespace
+
+float int4_few_us(int T, int N, int K, bool gated) {
+  const Int4Estimate e = int4_estimate(T, N, K, gated);
+  return e.here < e.there ? e.here : e.there;
+}
 
 bool skinny_takes(bool int4, bool norm, int T, int N, int K, bool gated) {
   if (static_cast<double>(N) * K * (gated ? 2 : 1) >= 3.e10) return false;      // rows are counted in 32 bits (skinny_gemm)

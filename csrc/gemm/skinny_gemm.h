@@ -12,6 +12,8 @@ namespace fi {
 // with q|k|v alone).  The others are faster alone too, but not in a step, where their predecessors' rings hide the start of
 // dense_gemm.cu's stream (o 1.264 ms, down 1.246, logits of 151936 rows at three tokens 160 us slower).
 bool skinny_takes(bool int4, bool norm, int T, int N, int K, bool gated);
+// us of an int4 product of 9 to 16 tokens in the faster one of this kernel and awq_gemm.cu.
+float int4_few_us(int T, int N, int K, bool gated);
 
 struct SkinnyParams {
   const void* x;            // [T, K] rows of pitch ldx, 16-bit

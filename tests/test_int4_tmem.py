@@ -44,3 +44,57 @@ def test_experts_in_tensor_memory(T, E, K, H, inter, group, zeros, dtype):
     eps = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
     assert (got - ref).norm() <= 2 * eps * ref.norm()
     assert (got - ref).abs().max() <= 8 * eps * ref.abs().max()
+
+
+def _layer(rows, K, group, zeros, dtype, g):
+    nib = torch.randint(0, 16, (rows, K), generator=g, device=DEV, dtype=torch.uint8)
+    s = (torch.rand(rows, K // group, generator=g, device=DEV) + 0.5).mul_(0.2 * K ** -0.5).to(dtype)
+    z = torch.randint(4, 12, (rows, K // group), generator=g, device=DEV, dtype=torch.uint8) if zeros else None
+    w = Int4Weight(nib, s, z, group, dtype)
+    return w, w.dense().to(dtype).double()               # the kernels round the weights once
+
+
+# every number of CTAs that share a tile's K (the last with less of it), every token tile, tokens that end inside one, rows that end in
+# either half of a tile, one k-block and k-blocks that end inside a stage
+@pytest.mark.gpu
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("T,N,K,group,zeros,dtype", [
+    (1, 16, 64, 64, True, torch.bfloat16), (9, 272, 320, 32, False, torch.float16), (16, 128, 2112, 64, True, torch.bfloat16),
+    (17, 1408, 2048, 128, False, torch.bfloat16), (33, 400, 2176, 128, True, torch.float16), (70, 4112, 704, 32, False, torch.bfloat16)])
+def test_layers_in_tensor_memory(T, N, K, group, zeros, dtype, gated):
+    g = torch.Generator(device=DEV).manual_seed(T + N + K)
+    w, dense = _layer(2 * N if gated else N, K, group, zeros, dtype, g)
+    x = torch.randn(T, K + 8, generator=g, device=DEV).to(dtype)[:, :K]
+    b, r = torch.randn(w.N, generator=g, device=DEV).to(dtype), torch.randn(T, N, generator=g, device=DEV).to(dtype)
+    y = x.double() @ dense.t() + b.double()
+    if gated:
+        y = torch.nn.functional.gelu(y[:, :N], approximate="tanh") * y[:, N:]
+    eps = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    raw = (K // 64 + 3) // 4
+    for splits in range(0, min(8, raw) + 1):
+        for bn in (16, 32, 64):
+            out = torch.full((T, N), float("nan"), dtype=dtype, device=DEV)
+            rc = ops._lib.kernels().fi_int4_tmem(
+                ops._p(x), ops._p(w.qw), ops._p(w.scales_t), ops._p(w.zeros_t), ops._p(out), ops._p(b), ops._p(r), T, N, K, group, x.stride(0),
+                N, ops._ACT["gelu_tanh" if gated else None], N if gated else 0, 0, ops._DT[dtype], splits, bn,
+                ops._p(ops.status_word(x.device)), ops._stream())
+            assert rc == 0
+            ops.check_status(x.device)
+            # one rounding of the result; 32-bit sums and the fast exponential are far below it
+            assert ((out.double() - (y + r.double())).abs() <= eps * (y + r.double()).abs() + 1e-4 * y.abs().mean()).all(), (splits, bn)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,N,K,gated", [(24, 1536, 512, True), (128, 1536, 512, True), (16, 12288, 4096, True), (30, 4096, 12288, False)])
+def test_layers_take_it(T, N, K, gated):
+    """Sizes whose route leads here: whole layers through the public call, 32-bit output included."""
+    from litevllm_b200.ops.awq import int4_linear
+    g = torch.Generator(device=DEV).manual_seed(T)
+    w, dense = _layer(2 * N if gated else N, K, 128, True, torch.bfloat16, g)
+    x = torch.randn(T, K, generator=g, device=DEV).to(torch.bfloat16)
+    y = x.double() @ dense.t()
+    if gated:
+        y = torch.nn.functional.silu(y[:, :N]) * y[:, N:]
+    got = int4_linear(x, w, gated_act="silu" if gated else None, out_dtype=torch.float32)
+    ops.check_status(x.device)
+    assert (got.double() - y).norm() <= 1e-5 * y.norm()
