@@ -273,11 +273,13 @@ def _tmem_takes(w_gate_up: Int4Weight, w_down: Int4Weight, H: int, inter: int) -
         for w in (w_gate_up, w_down))
 
 
-# From this many routes on experts take int4_tmem.cu, below it skinny_gemm.cu, which spreads the rows of few experts over all SMs.  us of
-# the layer there / in int4_tmem.cu: 128 experts of 2816 x 704 with 8 of them per token 30 / 35 at 8 routes, 52 / 43 at 24, 79 / 70 at 48,
-# 154 / 136 at 256; 8 of 4096 x 1408 27 / 44 at 2, 47 / 50 at 24, 60 / 50 at 32; 16 of 4096 x 4096 111 / 134 at 16, 143 / 154 at 24,
-# 146 / 133 at 32; 256 of 2048 x 1024 54 / 55 at 24, 69 / 57 at 32; 32 of 1024 x 512 18 / 24 at 24, 26 / 25 at 32.
-_TMEM_MIN_ROUTES = 32
+def _tmem_pays(routes: int, experts: int) -> bool:
+    """Whether the routed rows take int4_tmem.cu rather than skinny_gemm.cu, which spreads the rows of few experts over all SMs.  us of the
+    layer there / in int4_tmem.cu: 128 experts of 2816 x 704 with 8 of them per token 30 / 35 at 8 routes, 52 / 43 at 24, 63 / 63 at 32
+    (and 1 % of a decode step more there: its start does not hide behind the kernel in front), 79 / 70 at 48, 154 / 136 at 256; 8 of 4096
+    x 1408 27 / 44 at 2, 47 / 50 at 24, 60 / 50 at 32; 16 of 4096 x 4096 111 / 134 at 16, 143 / 154 at 24, 146 / 133 at 32; 256 of 2048
+    x 1024 54 / 55 at 24, 69 / 57 at 32; 32 of 1024 x 512 18 / 24 at 24, 26 / 25 at 32."""
+    return routes >= 32 + experts // 32
 
 
 def _tmem_tile(mean: int) -> int:
@@ -299,7 +301,7 @@ def fused_expert_rows(x: torch.Tensor, w_gate_up: Int4Weight, w_down: Int4Weight
     n = T * K
     mean = n // max(num_experts_local, 1)
     few = _few_rows(mean, H, inter)
-    tmem = _tmem_tile(mean) if (n >= _TMEM_MIN_ROUTES or not few) and _tmem_takes(w_gate_up, w_down, H, inter) else 0
+    tmem = _tmem_tile(mean) if (_tmem_pays(n, num_experts_local) or not few) and _tmem_takes(w_gate_up, w_down, H, inter) else 0
     few = few and not tmem and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
     if not few and (not x.is_contiguous() or x.data_ptr() % 16):        # the gather reads whole rows in 16-byte groups
         x = x.clone(memory_format=torch.contiguous_format)

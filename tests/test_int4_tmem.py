@@ -18,7 +18,7 @@ def test_tile_follows_the_mean_number_of_rows():
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("T,E,K,H,inter,group,zeros", [
-    (16, 4, 2, 64, 64, 32, False), (33, 8, 2, 320, 192, 64, True), (64, 16, 4, 2816, 704, 32, False), (60, 8, 2, 256, 1408, 128, True),
+    (17, 4, 2, 64, 64, 32, False), (33, 8, 2, 320, 192, 64, True), (64, 16, 4, 2816, 704, 32, False), (60, 8, 2, 256, 1408, 128, True),
     (200, 8, 2, 192, 320, 32, True), (300, 4, 2, 1024, 384, 128, False), (130, 128, 8, 128, 128, 64, False)])
 def test_experts_in_tensor_memory(T, E, K, H, inter, group, zeros, dtype):
     g = torch.Generator(device=DEV).manual_seed(T + E)
@@ -35,7 +35,7 @@ def test_experts_in_tensor_memory(T, E, K, H, inter, group, zeros, dtype):
     score[:, 1] -= 2.0                                   # and an empty one
     ids = score.topk(K).indices.int()
     wts = torch.rand(T, K, generator=g, device=DEV)
-    assert T * K >= moe._TMEM_MIN_ROUTES and moe._tmem_takes(gu, dn, H, inter)
+    assert moe._tmem_pays(T * K, E) and moe._tmem_takes(gu, dn, H, inter)
     got = moe.fused_experts(x, gu, dn, ids, wts, E, 0, "gelu_tanh").float()
     ops.check_status(x.device)
     ref = moe._reference_experts(x, gu, dn, ids, wts, E, 0, E, "gelu_tanh").float()
