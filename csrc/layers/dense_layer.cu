@@ -1,0 +1,106 @@
+// One decoder layer of a prefill step, enqueued by one native call: norm, q|k|v, rotary embedding and cache write, attention, output
+// projection, norm, gate|up, down.  Steps of few tokens were bound by the host: six launches per layer from Python take 95 us, here
+// 30 (five each for the launch and its tensor maps), the kernels of 37 tokens about 55.  No kernel of its own: the routes
+// of the products are those of litevllm_b200/ops (linear, gated_linear, int4_linear below 129 tokens, rope_and_cache,
+// paged_attention_prefill), whose arguments litevllm_b200/layers/dense_layer.py packs.
+#include <stdint.h>
+
+#include "entries.h"
+
+namespace {
+
+struct Product {
+  const void* w;          // 16-bit [rows, k] of pitch ldw, or int4 (group > 0) in the layout of awq_gemm.cu
+  const void* scales;
+  const void* zeros;
+  const void* bias;
+  int rows, k, ldw, group;
+};
+
+struct Layer {
+  Product qkv, o, gate_up, down;
+  const void* norm_in;
+  const void* norm_mid;
+  const void* q_norm;
+  const void* k_norm;
+  void* k_cache;
+  void* v_cache;
+  float eps_in, eps_mid, eps_qk, sm_scale;
+  int mode_in, mode_mid, qk_norm_mode, fused_norms, act, nh, nkv, hd, rot_dim, window, tensor_attention, reserved;
+};
+
+struct Step {
+  void* h;                // [T, H], updated in place
+  void* x;                // [T, H] normed input (where the norms are not fused)
+  void* qkv;
+  void* attn;
+  void* mid;
+  const int* positions;
+  const int* slots;
+  const float* cos_sin;
+  const int* block_tables;
+  const int* seq_lens;
+  const int* cu_q;
+  int* status;
+  void* stream;
+  long num_blocks;
+  int T, H, B, max_q_len, max_blocks, block_size, kv_fp8, dtype;
+  int plain_persistent, plain_min_t, plain_by_size, gated_persistent, gated_min_t, reserved;
+  float k_scale, v_scale;
+};
+
+static_assert(sizeof(Product) == 48 && sizeof(Layer) == 4 * 48 + 6 * 8 + 4 * 4 + 12 * 4 && sizeof(Step) == 14 * 8 + 14 * 4 + 2 * 4, "packed by Python");
+
+// C [T, rows (gated: rows / 2)] = X W^T (+ residual), with the norm of X's rows inside where norm_eps > 0.
+int product(const Step& s, const Product& w, const void* x, int ldx, void* c, const void* residual, bool gated, int act, float norm_eps) {
+  const int n = gated ? w.rows / 2 : w.rows;
+  if (w.group > 0)
+    return fi_awq_gemm(x, w.w, w.scales, w.zeros, c, w.bias, residual, s.T, n, w.k, w.group, ldx, n, act, gated ? n : 0, 0, s.dtype, 0, 0,
+                       s.status, s.stream);
+  if (norm_eps > 0.f)
+    return fi_dense_gemm_rmsnorm(x, w.w, c, w.bias, residual, s.T, n, w.k, ldx, w.ldw, n, act, gated ? n : 0, 0, s.dtype, 0, 0, norm_eps,
+                                 s.status, s.stream);
+  const bool persistent = gated ? s.gated_persistent && s.T >= s.gated_min_t
+                                : s.plain_persistent && s.T >= s.plain_min_t &&
+                                      (s.T >= 1024 || !s.plain_by_size || fi_dense_gemm_persistent_pays(s.T, n, w.k));
+  if (persistent)
+    return fi_dense_gemm_persistent(x, w.w, c, w.bias, residual, s.T, n, w.k, ldx, w.ldw, n, act, 0.f, gated ? n : 0, 0, s.dtype, s.status,
+                                    s.stream);
+  return fi_dense_gemm(x, w.w, c, w.bias, residual, s.T, n, w.k, ldx, w.ldw, n, act, 0.f, gated ? n : 0, 0, s.dtype, 0, 0, s.status, s.stream);
+}
+
+}  // namespace
+
+// Returns 0 or the first error of a launch (which one: where, counted from 1).
+extern "C" int fi_dense_layer(const void* layer, const void* step, int* where) {
+  const Layer& l = *static_cast<const Layer*>(layer);
+  const Step& s = *static_cast<const Step*>(step);
+  int at = 0, rc = 0;
+  auto done = [&](int r) {
+    ++at;
+    if (r != 0) { rc = r; *where = at; }
+    return r != 0;
+  };
+  const int q_cols = l.nh * l.hd, width = (l.nh + 2 * l.nkv) * l.hd;
+  const float eps_in = l.fused_norms ? l.eps_in : 0.f, eps_mid = l.fused_norms ? l.eps_mid : 0.f;
+  const void* x = l.fused_norms ? s.h : s.x;
+  if (!l.fused_norms && done(fi_rmsnorm(s.h, nullptr, l.norm_in, s.x, s.T, s.H, s.H, s.H, l.eps_in, l.mode_in, 1.f, s.dtype, s.stream, nullptr))) return rc;
+  if (done(product(s, l.qkv, x, s.H, s.qkv, nullptr, false, 0, eps_in))) return rc;
+  if (done(fi_rope_cache(s.qkv, s.positions, s.cos_sin, nullptr, s.slots, l.k_cache, l.v_cache, l.q_norm, l.k_norm, s.T, l.nh, l.nkv, l.hd,
+                         l.rot_dim, s.block_size, s.kv_fp8, s.k_scale, s.v_scale, l.eps_qk, l.qk_norm_mode, 0, s.dtype, s.stream)))
+    return rc;
+  int r = -12;
+  if (l.tensor_attention)
+    r = fi_paged_prefill_tc(s.qkv, width, l.k_cache, l.v_cache, s.attn, s.block_tables, s.seq_lens, s.cu_q, s.B, s.T, s.max_q_len, l.nh,
+                            l.nkv, l.hd, s.num_blocks, s.max_blocks, s.block_size, l.window, l.sm_scale, 0.f, nullptr, s.dtype, s.status,
+                            s.stream);
+  if (r == -12)       // outside what the tensor-core kernel covers
+    r = fi_paged_prefill(s.qkv, width, l.k_cache, l.v_cache, s.attn, s.block_tables, s.seq_lens, s.cu_q, s.B, s.max_q_len, l.nh, l.nkv, l.hd,
+                         s.max_blocks, s.block_size, l.window, l.sm_scale, 0.f, s.kv_fp8, s.k_scale, s.v_scale, nullptr, s.dtype, s.stream);
+  if (done(r)) return rc;
+  if (done(product(s, l.o, s.attn, q_cols, s.h, s.h, false, 0, 0.f))) return rc;
+  if (!l.fused_norms && done(fi_rmsnorm(s.h, nullptr, l.norm_mid, s.x, s.T, s.H, s.H, s.H, l.eps_mid, l.mode_mid, 1.f, s.dtype, s.stream, nullptr))) return rc;
+  if (done(product(s, l.gate_up, x, s.H, s.mid, nullptr, true, l.act, eps_mid))) return rc;
+  done(product(s, l.down, s.mid, l.gate_up.rows / 2, s.h, s.h, false, 0, 0.f));
+  return rc;
+}

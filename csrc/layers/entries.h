@@ -1,0 +1,30 @@
+// Entry points that the native layers call, as their own sources define them.
+#pragma once
+#include "../attn/attn_extra.h"
+
+extern "C" {
+int fi_rmsnorm(const void* x, void* residual, const void* w, void* out, int rows, int H, long ldx, long ldo, float eps, int w_mode,
+               float out_scale, int dtype, void* stream, const void* addend);
+int fi_rope_cache(void* qkv, const int* positions, const float* cos_sin, const int* freq_stream, const int* slot_mapping, void* k_cache,
+                  void* v_cache, const void* qw, const void* kw, int T, int nh, int nkv, int hd, int rot_dim, int block_size, int kv_fp8,
+                  float k_scale, float v_scale, float eps, int qk_norm_mode, int v_norm, int dtype, void* stream);
+int fi_paged_prefill(const void* q, long q_stride, const void* k_cache, const void* v_cache, void* out, const int* block_tables,
+                     const int* seq_lens, const int* cu_q, int B, int max_q_len, int nh, int nkv, int hd, int max_blocks, int block_size,
+                     int window, float sm_scale, float softcap, int kv_fp8, float k_scale, float v_scale, const FiAttnExtra* extra,
+                     int dtype, void* stream);
+int fi_paged_prefill_tc(const void* q, long q_stride, const void* k_cache, const void* v_cache, void* out, const int* block_tables,
+                        const int* seq_lens, const int* cu_q, int B, int T_total, int max_q_len, int nh, int nkv, int hd, long num_blocks,
+                        int max_blocks, int block_size, int window, float sm_scale, float softcap, const FiAttnExtra* extra, int dtype,
+                        int* status, void* stream);
+int fi_dense_gemm(const void* X, const void* W, void* C, const void* bias, const void* residual, int T, int N, int K, int ldx, int ldw,
+                  int ldc, int act, float act_limit, int dual_rows, int out_fp32, int dtype, int splits, int bn, int* status, void* stream);
+int fi_dense_gemm_rmsnorm(const void* X, const void* W, void* C, const void* bias, const void* residual, int T, int N, int K, int ldx,
+                          int ldw, int ldc, int act, int dual_rows, int out_fp32, int dtype, int splits, int bn, float eps, int* status,
+                          void* stream);
+int fi_dense_gemm_persistent(const void* X, const void* W, void* C, const void* bias, const void* residual, int T, int N, int K, int ldx,
+                             int ldw, int ldc, int act, float act_limit, int dual_rows, int out_fp32, int dtype, int* status, void* stream);
+int fi_dense_gemm_persistent_pays(int T, int N, int K);
+int fi_awq_gemm(const void* X, const void* qw, const void* scales, const void* zeros, void* C, const void* bias, const void* residual,
+                int T, int N, int K, int group, int ldx, int ldc, int act, int dual_rows, int out_fp32, int dtype, int splits, int bn,
+                int* status, void* stream);
+}

@@ -1,0 +1,119 @@
+"""Prefill through a dense decoder layer in one native call (csrc/layers/dense_layer.cu).
+
+The launches of a layer are the same as those of the modules' own ``forward``, in the same order, on the same operands; only the
+Python between them is left out.  A step of few tokens is otherwise bound by it (TinyLlama, 37 tokens: 95 us of host time per layer
+against about 55 of device time).  Whoever hooks a module, replaces its ``forward``, profiles stages, adapts with LoRA or
+shards over ranks gets the modules.
+"""
+from __future__ import annotations
+
+import ctypes
+import struct
+
+import torch
+
+from .. import ops
+from ..ops import awq as awq_ops, reference
+from ..parallel import state as pstate
+from ..utils.hooks import watched
+from ..utils.profiling import PROFILER
+from .linear import LiteLinear
+
+_PRODUCT = struct.Struct("4Q4i")
+_REST = struct.Struct("6Q4f12i")
+_STEP = struct.Struct("13Qq14i2f")
+
+
+class PrefillWork:
+    """What the layers of one forward pass share: scratch for their intermediate rows and the packed step."""
+
+    def __init__(self, h, batch, cos_sin, width: int, heads: int, inter: int, k_cache):
+        T, H = h.shape
+        sizes = [T * n for n in (H, width, heads, inter)]
+        self.buf = torch.empty(sum((s + 63) // 64 * 64 for s in sizes), dtype=h.dtype, device=h.device)
+        at, ptrs = self.buf.data_ptr(), []
+        for s in sizes:
+            ptrs.append(at)
+            at += (s + 63) // 64 * 64 * 2
+        cfg, bt = batch.config, batch.block_tables
+        self.h, self.cos_sin, self.T, self.shape = h, cos_sin, T, (H, width, heads, inter)
+        self.fp8 = k_cache.dtype == torch.float8_e4m3fn
+        self.tensor_attention = ops._PREFILL_TC != "off" and (ops._PREFILL_TC == "on" or int(batch.max_q_len) >= ops._PREFILL_TC_MIN_Q)
+        self.num_blocks, self.block_size = k_cache.shape[0], k_cache.shape[2]
+        self.packed = _STEP.pack(
+            h.data_ptr(), *ptrs, batch.positions.data_ptr(), batch.slot_mapping.data_ptr(), cos_sin.data_ptr(), bt.data_ptr(),
+            batch.seq_lens.data_ptr(), batch.cu_q.data_ptr(), ops.status_word(h.device).data_ptr(), ops._stream(), self.num_blocks, T, H,
+            batch.seq_lens.shape[0], int(batch.max_q_len), bt.shape[1], self.block_size, int(self.fp8), ops._DT[h.dtype],
+            int(ops._PERSISTENT_PLAIN), ops._PERSISTENT_MIN_T, int(ops._PERSISTENT_BY_SIZE), int(ops._PERSISTENT_GEMM),
+            ops._PERSISTENT_MIN_T_GATED, 0, cfg.k_scale, cfg.v_scale)
+        self.where = ctypes.c_int(0)
+
+
+def prefill_work(layer, h, batch, kv, cos_sin) -> PrefillWork | None:
+    """The shared part for layers like ``layer``, or None where the step is not one for native layers."""
+    if (not h.is_cuda or h.dtype not in (torch.bfloat16, torch.float16) or not h.is_contiguous() or h.data_ptr() % 16 or h.shape[0] == 0
+            or h.shape[1] % 8 or batch.is_decode or batch.lora_mapping is not None or batch.cu_q is None or batch.positions.dim() != 1
+            or batch.positions.dtype != torch.int32 or batch.slot_mapping.dtype != torch.int32 or pstate.tp_size() != 1
+            or ops._BOUNDS_CHECK or (PROFILER.stages and (PROFILER.enabled or PROFILER.nvtx))):
+        return None
+    k_cache, v_cache = kv
+    if reference.kv_mode(k_cache) >= 2 or not (k_cache.is_contiguous() and v_cache.is_contiguous() and batch.block_tables.is_contiguous()):
+        return None
+    at, mlp = layer.self_attn, layer.mlp
+    return PrefillWork(h, batch, cos_sin, (at.nh + 2 * at.nkv) * at.hd, at.nh * at.hd, mlp.gate_up_proj.out_features // 2, k_cache)
+
+
+def _pack(lin, cols: int, rows: int, dtype, T: int) -> bytes | None:
+    """A product's operands, or None where its module has to run it."""
+    if type(lin) is not LiteLinear or lin.tp != 1 or lin.act_limit or lin.in_features != cols or lin.out_features != rows:
+        return None
+    bias = lin.bias
+    if bias is not None and (bias.dtype != dtype or not bias.is_contiguous()):
+        return None
+    b = 0 if bias is None else bias.data_ptr()
+    if lin.quant_method is None:
+        w = lin.weight
+        if w.dtype != dtype or w.stride(1) != 1 or w.stride(0) % 8 or w.data_ptr() % 16 or cols % 8 or rows % 16:
+            return None
+        return _PRODUCT.pack(w.data_ptr(), 0, 0, b, rows, cols, w.stride(0), 0)
+    w = getattr(lin, "int4", None)
+    # longer steps may expand the weights into a copy of their own
+    if type(w) is not awq_ops.Int4Weight or w.qw is None or T >= awq_ops._EXPAND_MIN_T or w.scales_t.dtype != dtype or rows % 16:
+        return None
+    return _PRODUCT.pack(w.qw.data_ptr(), w.scales_t.data_ptr(), 0 if w.zeros_t is None else w.zeros_t.data_ptr(), b, rows, cols, 0, w.group)
+
+
+def run(layer, work: PrefillWork, h, kv, cos_sin) -> bool:
+    """The whole layer on ``h``, in place; False (and nothing done) where its modules have to run."""
+    if h is not work.h or cos_sin is not work.cos_sin:
+        return False
+    m = layer._modules
+    at, mlp, n1, n2 = m["self_attn"], m["mlp"], m["input_layernorm"], m["post_attention_layernorm"]
+    a, f = at._modules, mlp._modules
+    qkv, o, gu, down = a["qkv_proj"], a["o_proj"], f["gate_up_proj"], f["down_proj"]
+    if watched(at, mlp, n1, n2, qkv, o, gu, down):
+        return False
+    T, dtype = work.T, h.dtype
+    H, width, heads, inter = work.shape
+    k_cache, v_cache = kv
+    hd = at.hd
+    if ((at.nh + 2 * at.nkv) * hd, at.nh * hd) != (width, heads) or (k_cache.shape[0], k_cache.shape[2]) != (work.num_blocks, work.block_size) \
+            or (k_cache.dtype == torch.float8_e4m3fn) != work.fp8 or not (k_cache.is_contiguous() and v_cache.is_contiguous()):
+        return False
+    products = [_pack(qkv, H, width, dtype, T), _pack(o, heads, H, dtype, T), _pack(gu, H, 2 * inter, dtype, T), _pack(down, inter, H, dtype, T)]
+    if None in products or gu.gated_act is None or qkv.gated_act is not None or o.gated_act is not None or down.gated_act is not None:
+        return False
+    fused = layer.fused_norm and T <= 64
+    if fused and (qkv.quant_method is not None or gu.quant_method is not None):
+        return False
+    tensor = work.tensor_attention and hd in (64, 128) and k_cache.dtype == dtype and (work.block_size in (16, 32, 64) or work.block_size % 128 == 0)
+    qn, kn, qk_mode = (at.q_norm.weight.data_ptr(), at.k_norm.weight.data_ptr(), at.q_norm.w_mode) if at.qk_norm else (0, 0, -1)
+    packed = b"".join(products) + _REST.pack(
+        n1.weight.data_ptr(), n2.weight.data_ptr(), qn, kn, k_cache.data_ptr(), v_cache.data_ptr(), n1.eps, n2.eps, at.eps, at.sm_scale,
+        2 if n1.folded else n1.w_mode, 2 if n2.folded else n2.w_mode, qk_mode, int(fused), ops._ACT[gu.gated_act], at.nh, at.nkv, hd,
+        at.rot_dim, int(at.window or 0), int(tensor), 0)
+    rc = ops._lib.kernels().fi_dense_layer(packed, work.packed, ctypes.byref(work.where))
+    if rc != 0:
+        ops._lib.check(rc, f"fi_dense_layer (launch {work.where.value})")
+    ops._count(6 if fused else 8)
+    return True

@@ -15,7 +15,6 @@ from __future__ import annotations
 
 import torch
 from torch import nn
-from torch.nn.modules.module import _has_any_global_hook
 
 from .. import ops
 from ..layers.linear import LiteLinear
@@ -24,6 +23,7 @@ from ..ops import moe as moe_ops
 from ..ops import stream_norms as sn
 from ..ops.awq import Int4Weight, unpack_nibbles
 from ..parallel import state as pstate
+from ..utils.hooks import watched as _watched
 from ..utils.profiling import stage
 from .arch import ModelArch
 from .llama import RMSNormWeight
@@ -179,11 +179,6 @@ class Gemma4Experts(nn.Module):
 
 _NORMS_BEHIND_ATTENTION = ("post_attention_layernorm", "pre_feedforward_layernorm", "post_feedforward_layernorm",
                            "pre_feedforward_layernorm_2", "post_feedforward_layernorm_1", "post_feedforward_layernorm_2")
-
-
-def _watched(*modules) -> bool:
-    """Whether a hook or a replaced ``forward`` hangs on the call of one of the modules."""
-    return bool(_has_any_global_hook()) or any(m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__ for m in modules)
 
 
 def _plain_norm(m, eps: float) -> bool:

@@ -14,6 +14,7 @@ import torch
 from torch import nn
 
 from .. import ops
+from ..layers import dense_layer
 from ..layers.linear import LiteLinear
 from ..layers.rope import get_cos_sin
 from ..parallel import state as pstate
@@ -146,7 +147,10 @@ class LlamaDecoderLayer(nn.Module):
         self.input_layernorm.folded = self.post_attention_layernorm.folded = True
         self.fused_norm = True
 
-    def forward(self, h, batch, kv, cos_sin):
+    def forward(self, h, batch, kv, cos_sin, work=None):
+        """``work``: what the layers of a prefill step share when they run natively (``dense_layer.PrefillWork``)."""
+        if work is not None and dense_layer.run(self, work, h, kv, cos_sin):
+            return h
         # decode-sized batches: norms inside the GEMMs; prefill tiles are compute-bound and keep the norm kernel
         if self.fused_norm and h.is_cuda and batch.lora_mapping is None and h.shape[0] <= 64:
             h = self.self_attn(h, h, batch, kv, cos_sin, norm_eps=self.input_layernorm.eps)
@@ -207,8 +211,9 @@ class LlamaForCausalLM(nn.Module):
         cs = self.cos_sin(h.device)
         if self._sequence_parallel_ok(h, batch):
             return self._forward_sequence_parallel(h, batch, kv_caches, cs)
+        work = dense_layer.prefill_work(self.layers[0], h, batch, kv_caches[0], cs) if len(self.layers) and not batch.is_decode else None
         for i, layer in enumerate(self.layers):
-            h = layer(h, batch, kv_caches[i], cs)
+            h = layer(h, batch, kv_caches[i], cs, work)
         return self.compute_logits(h, batch)
 
     # ------------------------------------------------------------------ sequence-parallel prefill

@@ -1,0 +1,56 @@
+"""Prefill steps whose layers run in one native call: the same launches, so bit for bit the results of the layers' modules, and the modules
+wherever somebody listens to one of them."""
+import pytest
+import torch
+
+from litevllm_b200 import LLM, ops
+from litevllm_b200.layers import dense_layer
+
+pytestmark = pytest.mark.gpu
+
+
+def _logits(llm, lens, seed):
+    g = torch.Generator().manual_seed(seed)
+    vocab = llm.engine.model.arch.vocab_size
+    texts = [torch.randint(0, vocab, (n,), generator=g).tolist() for n in lens]
+    ids = [f"r{i}" for i in range(len(texts))]
+    llm.engine.replay_step([(r, t[:len(t) // 2], []) for r, t in zip(ids, texts)])           # cached, then the rest
+    out = llm.engine.replay_step([(r, t[len(t) // 2:], list(range(len(t) - len(t) // 2))) for r, t in zip(ids, texts)], ids).float().cpu()
+    ops.check_status(torch.device("cuda:0"))
+    return out
+
+
+@pytest.mark.parametrize("name,dtype,kv", [("tiny-llama-test", "bfloat16", None), ("tiny-llama-test", "float16", "fp8"), ("tiny-llama-awq-test", "float16", None),
+                                           ("tiny-llama-ct-test", "bfloat16", None), ("tiny-qwen3-test", "bfloat16", None)])
+@pytest.mark.parametrize("lens", [(1,), (37,), (64, 1), (65, 9, 30), (200, 129, 3)])
+def test_native_layers_equal_the_modules(name, dtype, kv, lens, monkeypatch):
+    kw = {} if kv is None else {"fastinference_config": {"kv_type": kv}}
+    llm = LLM(f"synthetic:{name}", dtype=dtype, device="cuda:0", max_num_seqs=4, max_model_len=256, **kw)
+    ran = []
+    run = dense_layer.run
+    monkeypatch.setattr(dense_layer, "run", lambda *a: ran.append(run(*a)) or ran[-1])
+    n0 = ops.launch_count()
+    native = _logits(llm, lens, 5)
+    n1 = ops.launch_count()
+    # int4 weights may be expanded into a copy from 129 tokens on, which the modules do
+    assert all(ran) if sum(lens) < 129 or llm.engine.model.layers[0].mlp.down_proj.quant_method is None else not any(ran)
+    monkeypatch.setattr(dense_layer, "run", lambda *a: False)
+    modules = _logits(llm, lens, 5)
+    assert ops.launch_count() - n1 == n1 - n0                # both count every launch
+    assert torch.equal(native, modules)
+
+
+def test_listeners_get_the_modules():
+    llm = LLM("synthetic:tiny-llama-test", dtype="bfloat16", device="cuda:0", max_num_seqs=2, max_model_len=128)
+    layer = llm.engine.model.layers[1]
+    plain = _logits(llm, (20,), 6)
+    for m in (layer, layer.self_attn, layer.mlp, layer.self_attn.qkv_proj, layer.self_attn.o_proj, layer.mlp.gate_up_proj, layer.mlp.down_proj):
+        seen = []
+        h = m.register_forward_hook(lambda mod, args, out: seen.append(out.shape))
+        again = _logits(llm, (20,), 6)
+        h.remove()
+        assert len(seen) == 2 and torch.equal(plain, again)        # both steps
+    h = layer.mlp.register_forward_hook(lambda mod, args, out: out + 1.0)
+    changed = _logits(llm, (20,), 6)
+    h.remove()
+    assert not torch.equal(plain, changed)
