@@ -456,6 +456,288 @@ __global__ void __launch_bounds__(128) paged_decode_kernel(const AttnParams p) {
   }
 }
 
+// What a decode CTA of 128 threads does with the shares of its warps: merged(row, channel, acc, l, m) gives their sum.  Whole rows are
+// finished, splits meet in the cluster, by tickets, or in a launch of their own.
+template <typename T, int HD, bool SIG, typename F>
+__device__ __forceinline__ void finish_decode(const AttnParams& p, uint8_t* smem_raw, int b, int head0, int heads_here, int split, int warp,
+                                              F merged) {
+  if (p.splits == 1 && p.x.maps == 2) {
+    for (int r = 2 * warp; r < heads_here; r += 8) store_map_pair<T, HD>(p, b, head0 + r, r, merged);
+    return;
+  }
+  for (int i = threadIdx.x; i < heads_here * HD; i += 128) {
+    const int r = i / HD, d = i % HD;
+    const int head = head0 + r;
+    if (p.splits == 1) {
+      finish_channel<T, HD, SIG>(p, b, head, r, d, merged);
+      continue;
+    }
+    float acc, l, m;
+    merged(r, d, acc, l, m);
+    if (p.cluster_off > 0) {
+      float* cO = reinterpret_cast<float*>(smem_raw + p.cluster_off);
+      cO[i] = acc;
+      if (d == 0) { cO[16 * HD + r * 2] = m; cO[16 * HD + r * 2 + 1] = l; }
+    } else {
+      const long base = (static_cast<long>(b) * p.nh + head) * p.splits + split;
+      p.ws_o[base * HD + d] = acc;
+      if (d == 0) { p.ws_ml[base * 2] = m; p.ws_ml[base * 2 + 1] = l; }
+    }
+  }
+  if (p.splits > 1 && p.cluster_off > 0) {
+    // the cluster's CTAs hold one partial each in their shared memory; every CTA finishes its share of
+    // the (head, channel) outputs from all of them and nobody leaves before the peers have read
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    float* cO = reinterpret_cast<float*>(smem_raw + p.cluster_off);
+    auto gathered = [&](int r, int d, float& acc, float& l, float& m) {
+      float ms[8];
+      m = -CUDART_INF_F;
+#pragma unroll
+      for (int sidx = 0; sidx < 8; ++sidx) {
+        if (sidx < p.splits) {
+          ms[sidx] = cluster.map_shared_rank(cO, sidx)[16 * HD + r * 2];
+          m = fmaxf(m, ms[sidx]);
+        }
+      }
+      acc = 0.f;
+      l = 0.f;
+#pragma unroll
+      for (int sidx = 0; sidx < 8; ++sidx) {
+        if (sidx < p.splits) {
+          const float* peer = cluster.map_shared_rank(cO, sidx);
+          const float f = ms[sidx] == -CUDART_INF_F ? 0.f : exp2f((ms[sidx] - m) * kLog2e);
+          acc += f * peer[r * HD + d];
+          l += f * peer[16 * HD + r * 2 + 1];
+        }
+      }
+    };
+    if (p.x.maps == 2) {
+      for (int r = 2 * (split * 4 + warp); r < heads_here; r += 8 * p.splits)
+        store_map_pair<T, HD>(p, b, head0 + r, r, gathered);
+    } else {
+      const int E = heads_here * HD;
+      const int per = (E + p.splits - 1) / p.splits;
+      const int i_end = min(E, (split + 1) * per);
+      for (int i = split * per + threadIdx.x; i < i_end; i += 128) {
+        finish_channel<T, HD, SIG>(p, b, head0 + i / HD, i / HD, i % HD, gathered);
+      }
+    }
+    cluster.sync();
+  } else if (p.splits > 1 && p.merge_tickets != nullptr) {
+    // last split CTA of this (sequence, head group) merges: every CTA publishes its partials, takes
+    // a ticket, and the one that draws the last ticket reads all of them back (L2) and finishes
+    __shared__ int is_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned int* ticket = p.merge_tickets + static_cast<long>(b) * gridDim.y + blockIdx.y;
+      const unsigned int prev = atomicAdd(ticket, 1u);
+      is_last = prev == static_cast<unsigned int>(p.splits) - 1u;
+      if (is_last) *ticket = 0u;
+    }
+    __syncthreads();
+    if (is_last) {
+      __threadfence();
+      auto gathered = [&](int r, int d, float& acc, float& l, float& m) {
+        const long base = (static_cast<long>(b) * p.nh + head0 + r) * p.splits;
+        m = -CUDART_INF_F;
+        for (int sidx = 0; sidx < p.splits; ++sidx) m = fmaxf(m, __ldcg(p.ws_ml + (base + sidx) * 2));
+        acc = 0.f;
+        l = 0.f;
+        for (int sidx = 0; sidx < p.splits; ++sidx) {
+          const float ms = __ldcg(p.ws_ml + (base + sidx) * 2);
+          const float f = ms == -CUDART_INF_F ? 0.f : exp2f((ms - m) * kLog2e);
+          acc += f * __ldcg(p.ws_o + (base + sidx) * HD + d);
+          l += f * __ldcg(p.ws_ml + (base + sidx) * 2 + 1);
+        }
+      };
+      if (p.x.maps == 2) {
+        for (int r = 2 * warp; r < heads_here; r += 8) store_map_pair<T, HD>(p, b, head0 + r, r, gathered);
+        return;
+      }
+      for (int i = threadIdx.x; i < heads_here * HD; i += 128) {
+        finish_channel<T, HD, SIG>(p, b, head0 + i / HD, i / HD, i % HD, gathered);
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------ decode, one or two query heads per KV head, e4m3 cache
+// grid as paged_decode_v2_kernel; 128 threads.  With one or two rows the 16-row products of that kernel are mostly padding, and its tiles of
+// expanded keys and values (136 KB at head size 256) leave one CTA to an SM, whose four warps wait for their own loads: 66 us
+// for 52 MB (32 sequences of 390 keys, 16 heads on 8 of size 256).  Here keys and values go from global memory into registers and through
+// fused multiply-adds in 32 bits (no rounding of the weights), 16 KB of shared memory for the merge, three CTAs to an SM: 26 us, and 18 % less error.
+//   * HD / 16 lanes share a key, 16 channels each; a warp reads 32 * 16 / HD keys at a time, a page of 16 in IT turns
+//   * the partial products of a page (IT keys x 2 heads per group of lanes) are added up crosswise, so that every lane ends with the score of
+//     one (key, head): soft cap, maximum and exponential are computed once
+//   * the lanes of a group keep a running state of their own; all of them meet at the end
+// Bound by the issue of about 800 instructions per page and warp.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n.reg .b64 x, y, z, w;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %5};\nmov.b64 z, {%6, %7};\nfma.rn.f32x2 w, x, y, z;\nmov.b64 {%0, %1}, w;\n}\n"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+// Two e4m3 values as 32-bit numbers (exact).
+__device__ __forceinline__ float2 e4m3x2(uint32_t pair) {
+  uint32_t h;
+  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h) : "h"(static_cast<uint16_t>(pair)));
+  return __half22float2(*reinterpret_cast<const __half2*>(&h));
+}
+
+template <typename T, int HD>
+__global__ void __launch_bounds__(128, 3) paged_decode_few_kernel(const AttnParams p) {
+  constexpr int LPK = HD / 16;            // lanes per key
+  constexpr int KPI = 32 / LPK;           // keys that a warp reads at a time
+  constexpr int IT = 16 / KPI;            // turns per 16-token group; 2 IT = LPK
+  fi::pdl_launch_dependents();
+  fi::pdl_wait();
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / LPK, at = lane % LPK;
+  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  const int heads_here = p.nh / p.nkv, head0 = kvh * heads_here;        // 1 or 2
+  const int seq_len = p.seq_lens[b];
+  const int* bt = p.block_tables + static_cast<long>(b) * p.max_blocks;
+  const int lo = p.window > 0 ? max(0, seq_len - p.window) : 0;
+  // 16-token groups of this CTA: [g_begin, g_end), dealt round-robin to the four warps
+  const int first_g = lo / 16;
+  const int n_groups = (seq_len + 15) / 16 - first_g;
+  const int per = ((n_groups + p.splits - 1) / p.splits + 3) / 4 * 4;
+  const int g_begin = first_g + split * per;
+  const int g_end = min(first_g + n_groups, g_begin + per);
+  const int my_n = (g_end - g_begin - warp + 3) / 4;   // groups of this warp (may be <= 0)
+  const int bpb = p.block_size / 16;                   // 16-token groups per KV block
+
+  float2 q[2][8], o[2][8];
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    const T* src = reinterpret_cast<const T*>(p.q) + static_cast<long>(b) * p.q_stride + static_cast<long>(head0 + min(g, heads_here - 1)) * HD + at * 16;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      q[g][c] = g < heads_here ? make_float2(static_cast<float>(src[2 * c]), static_cast<float>(src[2 * c + 1])) : make_float2(0.f, 0.f);
+      o[g][c] = make_float2(0.f, 0.f);
+    }
+  }
+  const float scale = p.sm_scale * p.k_scale;
+  float m = -CUDART_INF_F, l = 0.f;                    // of head (lane & 1) over the keys of this group of lanes; l: this lane's share
+
+  int bt_reg = 0;
+  auto refill_bt = [&](int k0) {   // block ids of this warp's groups k0 .. k0+31
+    const int g = g_begin + warp + 4 * (k0 + lane);
+    bt_reg = (k0 + lane < my_n) ? bt[g / bpb] : 0;
+  };
+  auto group_at = [&](int k) -> long {                 // first byte of this lane's part of the k-th group
+    const int g = g_begin + warp + 4 * k;
+    const int blk = __shfl_sync(0xffffffffu, bt_reg, k & 31);
+    return ((static_cast<long>(blk) * p.nkv + kvh) * p.block_size + (g % bpb) * 16) * HD + sub * HD + at * 16;
+  };
+  const uint8_t* const kc = reinterpret_cast<const uint8_t*>(p.k_cache);
+  const uint8_t* const vc = reinterpret_cast<const uint8_t*>(p.v_cache);
+  uint4 kr[IT], vr[IT];
+  if (my_n > 0) {
+    refill_bt(0);
+    const long base = group_at(0);
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+      kr[i] = *reinterpret_cast<const uint4*>(kc + base + i * KPI * HD);
+      vr[i] = *reinterpret_cast<const uint4*>(vc + base + i * KPI * HD);
+    }
+  }
+  for (int k = 0; k < my_n; ++k) {
+    const bool more = k + 1 < my_n;
+    if (((k + 1) & 31) == 0 && more) refill_bt(k + 1);
+    const long next = more ? group_at(k + 1) : 0;
+    float acc[2 * IT];                                 // [turn][head]
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+      const uint32_t w[4] = {kr[i].x, kr[i].y, kr[i].z, kr[i].w};
+      float2 s0 = make_float2(0.f, 0.f), s1 = s0;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float2 x = e4m3x2((c & 1) ? w[c >> 1] >> 16 : w[c >> 1] & 0xffffu);
+        s0 = fma2(x, q[0][c], s0);
+        s1 = fma2(x, q[1][c], s1);
+      }
+      acc[2 * i] = s0.x + s0.y;
+      acc[2 * i + 1] = s1.x + s1.y;
+      if (more) kr[i] = *reinterpret_cast<const uint4*>(kc + next + i * KPI * HD);
+    }
+    // 2 IT sums over LPK = 2 IT lanes: either half of the lanes keeps half of them; lane `at` ends with sum number `at`
+#pragma unroll
+    for (int n = IT; n >= 1; n >>= 1) {
+      const bool up = (at & n) != 0;
+#pragma unroll
+      for (int v = 0; v < n; ++v) {
+        const float give = up ? acc[v] : acc[v + n], keep = up ? acc[v + n] : acc[v];
+        acc[v] = keep + __shfl_xor_sync(0xffffffffu, give, n);
+      }
+    }
+    const int tok = (g_begin + warp + 4 * k) * 16 + (at >> 1) * KPI + sub;
+    float s = softcap_f(acc[0] * scale, p.softcap);
+    if (tok >= seq_len || tok < lo) s = -CUDART_INF_F;
+    float nm = s;
+#pragma unroll
+    for (int n = 2; n < LPK; n <<= 1) nm = fmaxf(nm, __shfl_xor_sync(0xffffffffu, nm, n));
+    nm = fmaxf(nm, m);
+    const float a = nm == -CUDART_INF_F ? 1.f : exp2f((m - nm) * kLog2e);
+    const float w = nm == -CUDART_INF_F ? 0.f : exp2f((s - nm) * kLog2e);
+    l = l * a + w;
+    m = nm;
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      const float f = __shfl_sync(0xffffffffu, a, sub * LPK + g);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) { o[g][c].x *= f; o[g][c].y *= f; }
+    }
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+      const float w0 = __shfl_sync(0xffffffffu, w, sub * LPK + 2 * i), w1 = __shfl_sync(0xffffffffu, w, sub * LPK + 2 * i + 1);
+      const uint32_t r[4] = {vr[i].x, vr[i].y, vr[i].z, vr[i].w};
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float2 x = e4m3x2((c & 1) ? r[c >> 1] >> 16 : r[c >> 1] & 0xffffu);
+        o[0][c] = fma2(x, make_float2(w0, w0), o[0][c]);
+        o[1][c] = fma2(x, make_float2(w1, w1), o[1][c]);
+      }
+      if (more) vr[i] = *reinterpret_cast<const uint4*>(vc + next + i * KPI * HD);
+    }
+  }
+#pragma unroll
+  for (int n = 2; n < LPK; n <<= 1) l += __shfl_xor_sync(0xffffffffu, l, n);
+
+  constexpr int STATES = 4 * KPI;
+  float* mO = reinterpret_cast<float*>(smem_raw);                 // [STATES][2][HD]
+  float* mML = mO + STATES * 2 * HD;                              // [STATES][2][2]
+  const int state = warp * KPI + sub;
+#pragma unroll
+  for (int g = 0; g < 2; ++g)
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      *reinterpret_cast<float4*>(mO + (state * 2 + g) * HD + at * 16 + c * 4) = make_float4(o[g][2 * c].x, o[g][2 * c].y, o[g][2 * c + 1].x, o[g][2 * c + 1].y);
+  if (at < 2) {
+    mML[(state * 2 + at) * 2] = m;
+    mML[(state * 2 + at) * 2 + 1] = l;
+  }
+  __syncthreads();
+  auto merged = [&](int r, int d, float& acc, float& sum, float& top) {     // the states' shares of one channel
+    top = -CUDART_INF_F;
+#pragma unroll
+    for (int i = 0; i < STATES; ++i) top = fmaxf(top, mML[(i * 2 + r) * 2]);
+    acc = 0.f;
+    sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < STATES; ++i) {
+      const float mi = mML[(i * 2 + r) * 2];
+      const float f = mi == -CUDART_INF_F ? 0.f : exp2f((mi - top) * kLog2e);
+      acc += f * mO[(i * 2 + r) * HD + d];
+      sum += f * mML[(i * 2 + r) * 2 + 1];
+    }
+  };
+  finish_decode<T, HD, false>(p, smem_raw, b, head0, heads_here, split, warp, merged);
+}
+
 // ------------------------------------------------------------------------------ decode, v2
 // Same math and grid as paged_decode_kernel, different data movement: every warp runs its OWN
 // multi-stage cp.async pipeline over 16-token groups (one KV block slice each), so the main loop has
@@ -709,107 +991,7 @@ __global__ void __launch_bounds__(128) paged_decode_v2_kernel(const AttnParams p
       l += f * mML[(w * 16 + r) * 2 + 1];
     }
   };
-  if (p.splits == 1 && p.x.maps == 2) {
-    for (int r = 2 * warp; r < heads_here; r += 8) store_map_pair<T, HD>(p, b, head0 + r, r, merged);
-    return;
-  }
-  for (int i = threadIdx.x; i < heads_here * HD; i += 128) {
-    const int r = i / HD, d = i % HD;
-    const int head = head0 + r;
-    if (p.splits == 1) {
-      finish_channel<T, HD, SIG>(p, b, head, r, d, merged);
-      continue;
-    }
-    float acc, l, m;
-    merged(r, d, acc, l, m);
-    if (p.cluster_off > 0) {
-      float* cO = reinterpret_cast<float*>(smem_raw + p.cluster_off);
-      cO[i] = acc;
-      if (d == 0) { cO[16 * HD + r * 2] = m; cO[16 * HD + r * 2 + 1] = l; }
-    } else {
-      const long base = (static_cast<long>(b) * p.nh + head) * p.splits + split;
-      p.ws_o[base * HD + d] = acc;
-      if (d == 0) { p.ws_ml[base * 2] = m; p.ws_ml[base * 2 + 1] = l; }
-    }
-  }
-  if (p.splits > 1 && p.cluster_off > 0) {
-    // the cluster's CTAs hold one partial each in their shared memory; every CTA finishes its share of
-    // the (head, channel) outputs from all of them and nobody leaves before the peers have read
-    namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
-    cluster.sync();
-    float* cO = reinterpret_cast<float*>(smem_raw + p.cluster_off);
-    auto gathered = [&](int r, int d, float& acc, float& l, float& m) {
-      float ms[8];
-      m = -CUDART_INF_F;
-#pragma unroll
-      for (int sidx = 0; sidx < 8; ++sidx) {
-        if (sidx < p.splits) {
-          ms[sidx] = cluster.map_shared_rank(cO, sidx)[16 * HD + r * 2];
-          m = fmaxf(m, ms[sidx]);
-        }
-      }
-      acc = 0.f;
-      l = 0.f;
-#pragma unroll
-      for (int sidx = 0; sidx < 8; ++sidx) {
-        if (sidx < p.splits) {
-          const float* peer = cluster.map_shared_rank(cO, sidx);
-          const float f = ms[sidx] == -CUDART_INF_F ? 0.f : exp2f((ms[sidx] - m) * kLog2e);
-          acc += f * peer[r * HD + d];
-          l += f * peer[16 * HD + r * 2 + 1];
-        }
-      }
-    };
-    if (p.x.maps == 2) {
-      for (int r = 2 * (split * 4 + warp); r < heads_here; r += 8 * p.splits)
-        store_map_pair<T, HD>(p, b, head0 + r, r, gathered);
-    } else {
-      const int E = heads_here * HD;
-      const int per = (E + p.splits - 1) / p.splits;
-      const int i_end = min(E, (split + 1) * per);
-      for (int i = split * per + threadIdx.x; i < i_end; i += 128) {
-        finish_channel<T, HD, SIG>(p, b, head0 + i / HD, i / HD, i % HD, gathered);
-      }
-    }
-    cluster.sync();
-  } else if (p.splits > 1 && p.merge_tickets != nullptr) {
-    // last split CTA of this (sequence, head group) merges: every CTA publishes its partials, takes
-    // a ticket, and the one that draws the last ticket reads all of them back (L2) and finishes
-    __shared__ int is_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned int* ticket = p.merge_tickets + static_cast<long>(b) * gridDim.y + blockIdx.y;
-      const unsigned int prev = atomicAdd(ticket, 1u);
-      is_last = prev == static_cast<unsigned int>(p.splits) - 1u;
-      if (is_last) *ticket = 0u;
-    }
-    __syncthreads();
-    if (is_last) {
-      __threadfence();
-      auto gathered = [&](int r, int d, float& acc, float& l, float& m) {
-        const long base = (static_cast<long>(b) * p.nh + head0 + r) * p.splits;
-        m = -CUDART_INF_F;
-        for (int sidx = 0; sidx < p.splits; ++sidx) m = fmaxf(m, __ldcg(p.ws_ml + (base + sidx) * 2));
-        acc = 0.f;
-        l = 0.f;
-        for (int sidx = 0; sidx < p.splits; ++sidx) {
-          const float ms = __ldcg(p.ws_ml + (base + sidx) * 2);
-          const float f = ms == -CUDART_INF_F ? 0.f : exp2f((ms - m) * kLog2e);
-          acc += f * __ldcg(p.ws_o + (base + sidx) * HD + d);
-          l += f * __ldcg(p.ws_ml + (base + sidx) * 2 + 1);
-        }
-      };
-      if (p.x.maps == 2) {
-        for (int r = 2 * warp; r < heads_here; r += 8) store_map_pair<T, HD>(p, b, head0 + r, r, gathered);
-        return;
-      }
-      for (int i = threadIdx.x; i < heads_here * HD; i += 128) {
-        finish_channel<T, HD, SIG>(p, b, head0 + i / HD, i / HD, i % HD, gathered);
-      }
-    }
-  }
+  finish_decode<T, HD, SIG>(p, smem_raw, b, head0, heads_here, split, warp, merged);
 }
 
 template <typename T, int HD, bool SIG>
@@ -1063,11 +1245,30 @@ __global__ void __launch_bounds__(128) paged_prefill_kernel(const AttnParams p) 
   }
 }
 
+inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 template <typename T, int HD, bool SIG>
 int launch_decode_as(const AttnParams& p, int B, cudaStream_t s) {
   const int G = p.nh / p.nkv;
   const int groups = (G + 15) / 16;
-  if (p.block_size % 16 == 0 && p.kv_fp8 <= 1) {
+  if (!SIG && p.block_size % 16 == 0 && p.kv_fp8 == 1 && G <= 2 && p.x.maps == 1 && aligned16(p.k_cache) && aligned16(p.v_cache)) {
+    constexpr int states = 4 * (512 / HD);
+    AttnParams pc = p;
+    int smem = (states * 2 * HD + states * 4) * 4;
+    pc.cluster_off = 0;
+    if (p.cluster_off != 0 && p.splits > 1 && p.splits <= 8) {   // cluster of the split CTAs merges through DSMEM
+      pc.cluster_off = (smem + 127) & ~127;
+      smem = pc.cluster_off + (16 * HD + 32) * 4;
+    }
+    auto kern = paged_decode_few_kernel<T, HD>;
+    cudaError_t ce = fi::ensure_dynamic_smem(kern, smem);
+    if (ce != cudaSuccess) return static_cast<int>(ce);
+    if (pc.cluster_off > 0) {
+      ce = fi::launch_kernel_cluster(kern, dim3(p.splits, p.nkv, B), dim3(128), smem, s, dim3(p.splits, 1, 1), pc);
+      return static_cast<int>(ce != cudaSuccess ? ce : cudaGetLastError());
+    }
+    fi::launch_kernel(kern, dim3(p.splits, p.nkv, B), dim3(128), smem, s, 0, pc);
+  } else if (p.block_size % 16 == 0 && p.kv_fp8 <= 1) {
     constexpr int NST = HD <= 64 ? 4 : HD <= 128 ? 3 : 2;
     const int tile = 16 * HD;
     const int raw = p.kv_fp8 ? tile : tile * 2;
