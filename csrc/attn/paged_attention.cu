@@ -1247,6 +1247,33 @@ __global__ void __launch_bounds__(128) paged_prefill_kernel(const AttnParams p) 
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+// Clusters of `splits` CTAs (single CTAs for one) of the decode kernel for 16-bit caches, or of the one for e4m3 caches with few heads, that
+// the chip holds at a time.
+template <typename T, int HD>
+int decode_clusters(bool few, int splits) {
+  constexpr int NST = HD <= 64 ? 4 : HD <= 128 ? 3 : 2, states = 4 * (512 / HD);
+  const int pipe = 4 * NST * 2 * 16 * HD * 2, merge = (4 * 16 * HD + 4 * 16 * 2) * 4;
+  int smem = few ? (states * 2 * HD + states * 4) * 4 : 16 * HD * 2 + (pipe > merge ? pipe : merge);
+  if (splits > 1) smem = ((smem + 127) & ~127) + (16 * HD + 32) * 4;
+  auto kern = few ? paged_decode_few_kernel<T, HD> : paged_decode_v2_kernel<T, HD, NST, false, true>;
+  if (fi::ensure_dynamic_smem(kern, smem) != cudaSuccess) return 0;
+  int dev = 0, sms = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  if (splits == 1) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, 128, smem) != cudaSuccess) return 0;
+    return n * sms;
+  }
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(splits, sms);
+  c.blockDim = dim3(128);
+  c.dynamicSmemBytes = smem;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = splits; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  c.attrs = at; c.numAttrs = 1;
+  return cudaOccupancyMaxActiveClusters(&n, kern, &c) == cudaSuccess ? n : 0;
+}
+
 template <typename T, int HD, bool SIG>
 int launch_decode_as(const AttnParams& p, int B, cudaStream_t s) {
   const int G = p.nh / p.nkv;
@@ -1281,8 +1308,8 @@ int launch_decode_as(const AttnParams& p, int B, cudaStream_t s) {
       pc.cluster_off = (smem + 127) & ~127;
       smem = pc.cluster_off + (16 * HD + 32) * 4;
     }
-    // few sequences: the calls that take eight splits in one cluster where they would fill the chip with many (pick_decode_splits)
-    const bool own = !SIG && pc.cluster_off > 0 && B * p.nkv <= (HD <= 128 ? 16 : 8);
+    // fewer splits than two CTAs per SM would take (pick_decode_splits): a warp has more groups, each exact in its largest weight
+    const bool own = !SIG && p.splits <= 8 && p.splits * B * p.nkv * groups < 2 * 148 && (pc.cluster_off > 0 || p.splits == 1);
     auto kern = own ? paged_decode_v2_kernel<T, HD, NST, SIG, !SIG> : paged_decode_v2_kernel<T, HD, NST, SIG, false>;
     cudaError_t ce = fi::ensure_dynamic_smem(kern, smem);
     if (ce != cudaSuccess) return static_cast<int>(ce);
@@ -1326,6 +1353,15 @@ int launch_prefill(const AttnParams& p, int B, int max_q_len, cudaStream_t s) {
 }
 
 }  // namespace
+
+// See decode_clusters; 0 where it is not known.
+extern "C" int fi_decode_clusters(int hd, int few, int splits) {
+  if (splits < 1 || splits > 8) return 0;
+  if (hd == 64) return decode_clusters<__nv_bfloat16, 64>(few != 0, splits);
+  if (hd == 128) return decode_clusters<__nv_bfloat16, 128>(few != 0, splits);
+  if (hd == 256) return decode_clusters<__nv_bfloat16, 256>(few != 0, splits);
+  return 0;
+}
 
 // Decode scratch: ws_o needs B*nh*splits*hd floats, ws_ml B*nh*splits*2 floats (splits > 1 only).  extra: see
 // attn_extra.h, or null.

@@ -436,12 +436,28 @@ _PREFILL_TC = os.environ.get("FI_PREFILL_TC", "auto")
 _PREFILL_TC_MIN_Q = int(os.environ.get("FI_PREFILL_TC_MIN_Q", "64"))
 
 
-def pick_decode_splits(B: int, nkv: int, max_kv_len: int, sm_count: int = 148, cluster_head: int = 0) -> int:
-    """``cluster_head``: head size of a call whose splits can form one cluster (up to eight, merged in the same launch)."""
+@functools.lru_cache(maxsize=256)
+def _decode_clusters(device: int, hd: int, few: bool) -> tuple[int, ...]:
+    """How many clusters of 1 to 8 decode CTAs the device holds at a time (groups of SMs are no multiples of all sizes)."""
+    return tuple(_lib.kernels().fi_decode_clusters(hd, int(few), n) for n in range(1, 9))
+
+
+def pick_decode_splits(B: int, nkv: int, max_kv_len: int, sm_count: int = 148, cluster_head: int = 0,
+                       room: tuple[int, ...] = ()) -> int:
+    """``cluster_head``: head size of a call whose splits can form one cluster (up to eight, merged in the same launch);
+    ``room``: how many such clusters of 1 to 8 splits fit the device, where known."""
     if _DECODE_SPLITS > 0:
         return _DECODE_SPLITS
     chunks = max(1, (max_kv_len + 63) // 64)
     ctas = max(1, B * nkv)
+    if cluster_head > 0 and room:
+        # The most splits whose clusters all run at a time: a few more fill a second round with little.  us with the splits below / these:
+        # 32 heads on 8 of size 128, 16 sequences 3 / 2: 13.1 / 7.2 at 100 keys, 19.4 / 13.0 at 700, 36.6 / 27.6 at 2000; 8 sequences 5
+        # / 4: 11.6 / 6.8, 16.9 / 9.5, 24.9 / 15.2; 4 sequences 10 / 8 (and one launch): 10.7 / 7.5, 11.8 / 8.8, 13.9 / 11.3.
+        # (Clusters of five and seven lose: 32 heads on 4 of size 64, 20 sequences of 700 keys 4 / 5 8.2 / 9.3, 14 with 6 / 7 7.8 / 9.4.)
+        fit = max((n for n in (1, 2, 3, 4, 6, 8) if room[n - 1] >= ctas), default=1)
+        if fit < 8 or max_kv_len <= 8 * 320:
+            return int(max(1, min(fit, chunks)))
     want = max(1, (2 * sm_count + ctas - 1) // ctas)
     # Few sequences: eight splits of a few more keys cost less than a second launch per layer.  us per step, more splits and a
     # merge kernel / eight (contexts of 100 to 2040 tokens): TinyLlama 1 sequence 1161 / 932 to 1170 / 1021, 4 (19 wanted) 1126 / 1074
@@ -532,8 +548,12 @@ def paged_attention_decode(q, k_cache, v_cache, block_tables, seq_lens, nh, nkv,
         eff = min(max_kv_len, window) if window and window > 0 else max_kv_len
         if sigmoid is not None and sigmoid.chunk > 0:
             eff = min(eff, sigmoid.chunk)
-        splits = pick_decode_splits(B, nkv, eff, cluster_head=hd if _DECODE_MERGE == "cluster" and k_cache.shape[2] % 16 == 0
-                                    and reference.kv_mode(k_cache) < 2 else 0)
+        clustered = _DECODE_MERGE == "cluster" and k_cache.shape[2] % 16 == 0 and reference.kv_mode(k_cache) < 2
+        few = reference.kv_mode(k_cache) == 1 and nh // nkv <= 2
+        room = ()
+        if clustered and (few or (reference.kv_mode(k_cache) == 0 and hd <= 128)) and diff is None and sigmoid is None and nh // nkv <= 16:
+            room = _decode_clusters(q.device.index or 0, hd, few)
+        splits = pick_decode_splits(B, nkv, eff, cluster_head=hd if clustered else 0, room=room)
     mode = reference.kv_mode(k_cache)
     assert mode < 2 or plain, "row-scaled caches take no sinks, gates, narrow outputs or two maps"
     if mode >= 2:

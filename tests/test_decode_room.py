@@ -1,0 +1,54 @@
+"""Splits of decode attention by the room for their clusters, and the decode kernel of one or two query heads per KV head."""
+import pytest
+import torch
+
+from litevllm_b200 import ops
+
+DEV = "cuda"
+ROOM = (296, 148, 93, 71, 56, 45, 37, 33)
+
+
+@pytest.mark.parametrize("B,nkv,context,want", [(16, 8, 2112, 2), (12, 8, 2112, 2), (8, 8, 2112, 4), (5, 8, 2112, 6), (4, 8, 2112, 8), (37, 8, 2112, 1),
+                                                (60, 8, 2112, 1), (16, 8, 9000, 2), (16, 8, 64, 1), (1, 8, 9000, 32), (1, 8, 200, 4)])
+def test_rule_with_room(B, nkv, context, want):
+    assert ops.pick_decode_splits(B, nkv, context, cluster_head=128, room=ROOM) == want
+
+
+# one and two heads per KV head, every head size, pages of several groups, windows, soft caps, sinks, gates and narrow outputs, sequences of one
+# key and of many, every number of splits with and without a cluster
+@pytest.mark.gpu
+@pytest.mark.parametrize("nh,nkv,hd,bs,window,softcap,dtype,extra", [
+    (16, 8, 256, 16, 0, 50.0, torch.bfloat16, ""), (8, 8, 256, 64, 100, 0.0, torch.float16, "sinks"), (12, 6, 128, 32, 0, 0.0, torch.bfloat16, "gate"),
+    (5, 5, 128, 16, 33, 20.0, torch.float16, "head gate"), (4, 2, 64, 128, 0, 0.0, torch.float16, "narrow"), (3, 3, 64, 16, 17, 0.0, torch.bfloat16, "")])
+@pytest.mark.parametrize("splits", [0, 1, 2, 3, 8, 13])
+def test_few_heads_per_kv_head(nh, nkv, hd, bs, window, softcap, dtype, extra, splits):
+    g = torch.Generator(device=DEV).manual_seed(nh * hd + splits)
+    lens = [1, 15, 16, 130, 700, 333]
+    per = (max(lens) + bs - 1) // bs
+    kc, vc = (torch.randn(len(lens) * per + 1, nkv, bs, hd, generator=g, device=DEV).to(torch.float8_e4m3fn) for _ in range(2))
+    bt = (torch.randperm(len(lens) * per, generator=g, device=DEV) + 1).view(len(lens), per).int()
+    sl = torch.tensor(lens, device=DEV, dtype=torch.int32)
+    q = torch.randn(len(lens), (nh + 2 * nkv) * hd, generator=g, device=DEV).to(dtype)
+    od = hd - 16 if extra == "narrow" else hd
+    sinks = torch.randn(nh, generator=g, device=DEV) if extra == "sinks" else None
+    gate = {"gate": torch.randn(len(lens), nh * od, generator=g, device=DEV).to(dtype),
+            "head gate": torch.randn(len(lens), nh, generator=g, device=DEV).to(dtype)}.get(extra)
+    ks, vs, scale = 0.7, 1.3, hd ** -0.5
+    got = ops.paged_attention_decode(q, kc, vc, bt, sl, nh, nkv, hd, scale, window, softcap, ks, vs, splits=splits, sinks=sinks,
+                                     v_dim=od if od != hd else None, gate=gate).double().view(len(lens), nh, od)
+    eps = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)            # half a unit in the last of 8 or 11 places
+    for b, n in enumerate(lens):
+        lo = max(0, n - window) if window else 0
+        k, v = (c[bt[b].long()].permute(1, 0, 2, 3).reshape(nkv, per * bs, hd)[:, lo:n].double() * f for c, f in ((kc, ks), (vc, vs)))
+        s = torch.einsum("kgd,ksd->kgs", q[b, :nh * hd].view(nkv, nh // nkv, hd).double(), k) * scale
+        if softcap:
+            s = torch.tanh(s / softcap) * softcap
+        if sinks is not None:
+            s = torch.cat([s, sinks.double().view(nkv, -1, 1)], -1)
+        w = s.softmax(-1)[..., :n - lo]
+        ref, size = (torch.einsum("kgs,ksd->kgd", w, t).reshape(nh, hd)[:, :od] for t in (v, v.abs()))
+        if gate is not None:
+            f = torch.sigmoid(gate[b].double()).view(nh, -1)
+            ref, size = ref * f, size * f
+        # one rounding of the result; scores, weights and sums are 32-bit
+        assert ((got[b] - ref).abs() <= eps * ref.abs() + 2e-5 * size + 1e-7).all()
