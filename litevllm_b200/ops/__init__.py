@@ -434,6 +434,11 @@ _DECODE_SPLITS = int(os.environ.get("FI_DECODE_SPLITS", "0"))
 # chunk has at least _PREFILL_TC_MIN_Q tokens, else the 64-row mma.sync kernel; "on" / "off" force one.
 _PREFILL_TC = os.environ.get("FI_PREFILL_TC", "auto")
 _PREFILL_TC_MIN_Q = int(os.environ.get("FI_PREFILL_TC_MIN_Q", "64"))
+# Heads of 256 channels on an e4m3 cache: their own tensor-core kernel (csrc/attn/prefill_fp8.cu), whose CTA of 128 rows costs an SM at least
+# 6 us.  Two prompts of 384 tokens, 16 heads on 8: 19.5 against 74.5 us; 8 tokens after 500: 21 against 82; one token: 7 against 9.  Only
+# chunks of no more than one 32-key step of the general kernel lose when there are more of them than SMs: 100 chunks of 16, 79 against
+# 59 us; 100 of 40, 80 against 102.
+_PREFILL_FP8_STEP, _SMS = 32, 148
 
 
 @functools.lru_cache(maxsize=256)
@@ -693,6 +698,17 @@ def paged_attention_prefill(q, k_cache, v_cache, block_tables, seq_lens, cu_q, m
             sm_scale, float(softcap or 0.0), extra, _DT[q.dtype], _p(status_word(q.device)), _stream())
         if rc != -12:       # -12: outside what the tensor-core kernel covers, take the general one
             _lib.check(rc, "fi_paged_prefill_tc")
+            _count()
+            return out
+    if (plain and mode == 1 and hd == 256 and _PREFILL_TC != "off" and q.dtype in (torch.bfloat16, torch.float16)
+            and k_cache.is_contiguous() and v_cache.is_contiguous()
+            and (_PREFILL_TC == "on" or int(max_q_len) > _PREFILL_FP8_STEP or B * nh <= _SMS)):
+        rc = _lib.kernels().fi_paged_prefill_fp8(
+            _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(out), _p(block_tables), _p(seq_lens), _p(cu_q), B, T,
+            int(max_q_len), nh, nkv, hd, k_cache.shape[0], block_tables.shape[1], k_cache.shape[2], int(window or 0),
+            sm_scale, float(softcap or 0.0), k_scale, v_scale, _DT[q.dtype], _p(status_word(q.device)), _stream())
+        if rc != -12:
+            _lib.check(rc, "fi_paged_prefill_fp8")
             _count()
             return out
     rc = _lib.kernels().fi_paged_prefill(
