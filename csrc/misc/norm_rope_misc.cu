@@ -280,6 +280,112 @@ __global__ void rope_cache_vec_kernel(T* __restrict__ qkv, const int* __restrict
   }
 }
 
+// The same with per-head norms or an e4m3 cache, for full-width rotary on heads of 32 to 512 channels (a power of two): hd / 16 neighbouring
+// lanes hold a head, each 8 channels of the low half and the 8 that turn with them, so that one pass with 16-byte accesses reads, norms,
+// turns and stores it.  Bound by its three dependent loads (slot, position, table) at few tokens and by L2 at many: 768 tokens, 16 heads
+// on 8 of 256 channels with norms and an e4m3 cache, 9.0 us (general kernel 20.5); 32 tokens, 2.4 us (4.7).  Values are rounded where
+// the general kernel rounds them; a head's sum of squares is added in another order.
+template <typename T>
+__global__ void rope_cache_heads_kernel(T* __restrict__ qkv, const int* __restrict__ positions, const float* __restrict__ cos_sin,
+                                        const int* __restrict__ slot_mapping, void* __restrict__ k_cache, void* __restrict__ v_cache,
+                                        const T* __restrict__ qw, const T* __restrict__ kw, int nh, int nkv, int hd, int block_size,
+                                        int kv_fp8, float k_scale, float v_scale, float eps, int qk_norm_mode, int v_norm) {
+  fi::pdl_launch_dependents();
+  fi::pdl_wait();
+  const int t = blockIdx.x, total = nh + 2 * nkv, half = hd >> 1;
+  const int lanes = hd >> 4, heads = blockDim.x / lanes;      // lanes of a head, heads of a pass
+  const int c = (threadIdx.x & (lanes - 1)) * 8;
+  const int slot = slot_mapping ? slot_mapping[t] : -1;
+  const float* cs = cos_sin + static_cast<long>(positions[t]) * hd + c;
+  for (int h0 = blockIdx.y * heads; h0 < total; h0 += heads * gridDim.y) {      // the same for the whole CTA: its lanes shuffle
+    const int h = h0 + static_cast<int>(threadIdx.x) / lanes;
+    const bool on = h < total, is_q = h < nh, is_v = h >= nh + nkv;
+    T* x = qkv + (static_cast<long>(t) * total + h) * hd + c;
+    uint4 raw[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)}, wraw[2] = {raw[0], raw[0]};
+    const T* nw = is_v || qk_norm_mode < 0 ? nullptr : is_q ? qw : kw;
+    float tab[2][8];      // cosines, sines
+    if (on) {
+      raw[0] = *reinterpret_cast<const uint4*>(x);
+      raw[1] = *reinterpret_cast<const uint4*>(x + half);
+      if (nw != nullptr) {
+        wraw[0] = *reinterpret_cast<const uint4*>(nw + c);
+        wraw[1] = *reinterpret_cast<const uint4*>(nw + half + c);
+      }
+      if (!is_v) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          *reinterpret_cast<float4*>(tab[i]) = *reinterpret_cast<const float4*>(cs + i * half);
+          *reinterpret_cast<float4*>(tab[i] + 4) = *reinterpret_cast<const float4*>(cs + i * half + 4);
+        }
+      }
+    }
+    float v[2][8], ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v[i][j] = Cvt<T>::to_f(reinterpret_cast<const T*>(&raw[i])[j]);
+        ss += v[i][j] * v[i][j];
+      }
+    }
+    const bool norm = is_v ? v_norm != 0 : qk_norm_mode >= 0;
+    if (qk_norm_mode >= 0 || v_norm) {
+      for (int o = lanes >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (norm) {
+        const float inv = rsqrtf(ss / static_cast<float>(hd) + eps);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            float f = Cvt<T>::to_f(Cvt<T>::from_f(v[i][j] * inv));
+            if (nw != nullptr) {
+              const float g = Cvt<T>::to_f(reinterpret_cast<const T*>(&wraw[i])[j]);
+              f *= qk_norm_mode == 1 ? 1.f + g : g;
+            }
+            v[i][j] = Cvt<T>::to_f(Cvt<T>::from_f(f));
+          }
+        }
+      }
+    }
+    if (!on) continue;
+    if (!is_v) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float a = v[0][j], b = v[1][j];
+        v[0][j] = Cvt<T>::to_f(Cvt<T>::from_f(a * tab[0][j] - b * tab[1][j]));
+        v[1][j] = Cvt<T>::to_f(Cvt<T>::from_f(b * tab[0][j] + a * tab[1][j]));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) reinterpret_cast<T*>(&raw[i])[j] = Cvt<T>::from_f(v[i][j]);
+    }
+    if (!is_v || norm) {
+      *reinterpret_cast<uint4*>(x) = raw[0];
+      *reinterpret_cast<uint4*>(x + half) = raw[1];
+    }
+    if (is_q || slot < 0) continue;
+    const long at = ((static_cast<long>(slot / block_size) * nkv + (is_v ? h - nh - nkv : h - nh)) * block_size + slot % block_size) * hd + c;
+    void* cache = is_v ? v_cache : k_cache;
+    if (kv_fp8) {
+      const float scale = 1.f / (is_v ? v_scale : k_scale);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        uint2 packed;
+        __nv_fp8x2_storage_t* e = reinterpret_cast<__nv_fp8x2_storage_t*>(&packed);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          e[j] = __nv_cvt_float2_to_fp8x2(make_float2(v[i][2 * j] * scale, v[i][2 * j + 1] * scale), __NV_SATFINITE, __NV_E4M3);
+        *reinterpret_cast<uint2*>(reinterpret_cast<uint8_t*>(cache) + at + i * half) = packed;
+      }
+    } else {
+      *reinterpret_cast<uint4*>(reinterpret_cast<T*>(cache) + at) = raw[0];
+      *reinterpret_cast<uint4*>(reinterpret_cast<T*>(cache) + at + half) = raw[1];
+    }
+  }
+}
+
 // Plain cache write (no rotation): k/v rows [T, nkv, hd] with row pitch ld -> paged cache.
 template <typename T>
 __global__ void reshape_and_cache_kernel(const T* __restrict__ k, const T* __restrict__ v,
@@ -644,6 +750,16 @@ extern "C" int fi_rope_cache(void* qkv, const int* positions, const float* cos_s
       const int threads = items >= 256 ? 256 : (items >= 128 ? 128 : 64);
       fi::launch_kernel(rope_cache_vec_kernel<Tt>, dim3(T), dim3(threads), 0, FI_STREAM(stream), 0, (Tt*)qkv, positions,
                         cos_sin, slot_mapping, (Tt*)k_cache, (Tt*)v_cache, nh, nkv, hd, block_size);
+      return static_cast<int>(cudaGetLastError());
+    }
+    const uintptr_t ends = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(cos_sin) | reinterpret_cast<uintptr_t>(qw) |
+                           reinterpret_cast<uintptr_t>(kw) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache);
+    if (rot_dim == hd && freq_stream == nullptr && hd >= 32 && hd <= 512 && (hd & (hd - 1)) == 0 && (ends & 15) == 0) {
+      // as many CTAs of 128 threads as there are heads to hold: whatever the number of tokens, no head waits for another
+      const int heads = 128 / (hd / 16);
+      fi::launch_kernel(rope_cache_heads_kernel<Tt>, dim3(T, (nh + 2 * nkv + heads - 1) / heads), dim3(128), 0, FI_STREAM(stream), 0, (Tt*)qkv,
+                        positions, cos_sin, slot_mapping, k_cache, v_cache, (const Tt*)qw, (const Tt*)kw, nh, nkv, hd, block_size, kv_fp8,
+                        k_scale, v_scale, eps, qk_norm_mode, v_norm);
       return static_cast<int>(cudaGetLastError());
     }
     int warps = nh + 2 * nkv;

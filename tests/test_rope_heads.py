@@ -1,0 +1,42 @@
+"""Rotary embedding, head norms and cache write in one pass (csrc/misc/norm_rope_misc.cu) against its general kernel's forms."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("T,nh,nkv,hd,dtype,fp8,mode,v_norm", [
+    (1, 1, 1, 32, torch.bfloat16, True, -1, False), (37, 5, 3, 64, torch.float16, True, 0, False), (19, 32, 8, 128, torch.bfloat16, False, 1, True),
+    (33, 16, 8, 256, torch.bfloat16, True, 0, True), (3, 7, 1, 512, torch.float16, False, 2, False), (5, 3, 2, 256, torch.bfloat16, False, -1, True)])
+def test_one_pass_and_general_kernel(T, nh, nkv, hd, dtype, fp8, mode, v_norm):
+    from litevllm_b200 import ops
+    from litevllm_b200.ops import reference as ref
+    g = torch.Generator(device=DEV).manual_seed(T + hd)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    bs, nb = 16, 6
+    qkv = rnd(T, (nh + 2 * nkv) * hd).to(dtype)
+    pos = torch.randint(0, 500, (T,), generator=g, device=DEV).int()
+    cs = ref.build_cos_sin(hd, 512, 10000.0).to(DEV)
+    slots = (torch.randperm((nb - 1) * bs, generator=g, device=DEV)[:T] + bs).int()
+    slots[T // 2] = -1 if T > 1 else slots[0]
+    qw, kw = ((rnd(hd) * 0.1 + 1).to(dtype) if mode in (0, 1) else None for _ in range(2))
+    outs = []
+    for stream in (None, torch.zeros(hd // 2, device=DEV, dtype=torch.int32)):      # a table of position streams: the general kernel
+        a = qkv.clone()
+        kc, vc = (torch.zeros(nb, nkv, bs, hd, device=DEV, dtype=torch.float8_e4m3fn if fp8 else dtype) for _ in range(2))
+        ops.rope_and_cache(a, pos, cs, slots, kc, vc, nh, nkv, hd, hd, freq_stream=stream, q_norm_w=qw, k_norm_w=kw, qk_norm_mode=mode,
+                           v_norm=v_norm, eps=1e-6, k_scale=0.5, v_scale=0.25)
+        outs.append([x.float() for x in (a, kc, vc)])
+    # the order of a sum of squares may move a normed value by one ulp, which the turning and its rounding pass on twice
+    # (a value is at most a quarter of sqrt(hd), its partner too); in e4m3 by one of its steps
+    ulp = 2.0 ** (-7 if dtype == torch.bfloat16 else -10)
+    moved = mode >= 0 or v_norm
+    for i, (one, two) in enumerate(zip(*outs)):
+        if not moved:
+            assert torch.equal(one, two)
+        else:
+            step = 2.0 ** -3 if fp8 and i else ulp
+            top = one.abs().max() * ulp * (4 if fp8 and i else 1)
+            assert ((one - two).abs() <= step * two.abs() + 2 * top).all()
+            assert (one != two).float().mean() < 0.01
