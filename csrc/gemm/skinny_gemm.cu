@@ -34,6 +34,7 @@
 // slots, ALU 45 to 51 %), the 16-bit forms of large matrices by memory, small ones by the latencies of one CTA's life.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <math.h>
 
 #include "../common/launch.cuh"
 #include "epilogue.cuh"
@@ -512,12 +513,28 @@ int launch(const SkinnyParams& p, int tiles, cudaStream_t s) {
 //   K = 2816 0.89, 1.16, 1.12), with K of 8192 and more less or not at all (0.74, 0.92, 1.00), with K up to 1024 everywhere.  For 9 to
 //   16 tokens, whose accumulators leave one CTA per SM either way, two tiles are 0 to 45 % faster at nearly every size (K = 704 to
 //   12288, 192 to 1536 tiles), up to 10 % slower at 128 tiles.
-//   Experts have short K and many tiles: two warps per tile (128 experts of 2816 x 704, 32 tokens: 153; four warps 202).
+//   Experts of up to 8 rows: about as many warps per tile as there are warps on the chip for the tiles of the experts that occur when
+//   routes fall evenly.  Fewer lengthen the chain of a warp, the more the longer K is; more cost rounds of CTAs with their table reads,
+//   tokens and sums (us with one warp for two tiles / one / two / four / eight for one): 240 tiles of K = 5120 - / 22 / 15 / 10 / 9, 512 of 4096
+//   27 / 18 / 13 / 11 / 14, 684 of 2816 21 / 15 / 13 / 16 / 18, 1365 of 704 9.8 / 9.5 / 12 / 15 / 21, 3600 of 768 12 / 16 / 21 / 27 / 37.
+//   The line between one and two warps is where a decode step crosses (1365 tiles of 704 in a step of one token: two warps 1 % faster).
+//   The layer's products, two warps always / by this: 128 experts of 2816 x 704, 8 per token, 1 / 2 / 4 / 6 tokens 30 / 43 / 64 / 77 -> 30 / 40 /
+//   58 / 64; 60 of 2048 x 1408 at 32 routes 65 -> 52; 256 of 2048 x 1024 at 32 routes 63 -> 44; 8 of 4096 x 2048 at 2 routes 28 -> 22.
+//   Experts of 9 to 16 rows have many tiles: two warps per tile (128 experts of 2816 x 704, 32 tokens: 153; four warps 202).
 template <typename T, bool POST>
 int int4_by_size(const SkinnyParams& p, cudaStream_t s) {
   const int tiles = p.dual_rows > 0 ? (p.dual_rows + 7) / 8 : (p.N + 15) / 16;
-  if (p.tile_expert != nullptr)
-    return p.tile_tokens <= 8 ? launch<T, true, POST, false, 2, 1, 1, 4>(p, tiles, s) : launch<T, true, POST, false, 2, 1, 2, 4>(p, tiles, s);
+  if (p.tile_expert != nullptr) {
+    if (p.tile_tokens > 8) return launch<T, true, POST, false, 2, 1, 2, 4>(p, tiles, s);
+    const float experts = static_cast<float>(p.rows_total / p.expert_rows);
+    const float n = tiles * fminf(static_cast<float>(p.max_tiles), experts * (1.f - expf(-p.T / experts)));
+    const float warps = 2.f * kWarps * sm_count();
+    if (8.f * n <= warps) return launch<T, true, POST, false, 8, 1, 1, 2>(p, tiles, s);
+    if (4.f * n <= warps) return launch<T, true, POST, false, 4, 1, 1, 4>(p, tiles, s);
+    if (2.f * n <= fmaxf(1.25f * warps, (POST ? 0.6f : 0.875f) * p.K)) return launch<T, true, POST, false, 2, 1, 1, 4>(p, tiles, s);
+    if (n <= fmaxf(warps, 1.25f * p.K)) return launch<T, true, POST, false, 1, 1, 1, 4>(p, tiles, s);
+    return launch<T, true, POST, false, 1, 2, 1, 2>(p, tiles, s);
+  }
   if (p.T > 8) return launch<T, true, POST, false, 8, 2, 2, 2>(p, tiles, s);
   return tiles >= 320 ? launch<T, true, POST, false, 8, 2, 1, 2>(p, tiles, s) : launch<T, true, POST, false, 8, 1, 1, 4>(p, tiles, s);
 }

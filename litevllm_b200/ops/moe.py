@@ -275,11 +275,10 @@ def _tmem_takes(w_gate_up: Int4Weight, w_down: Int4Weight, H: int, inter: int) -
 
 def _tmem_pays(routes: int, experts: int) -> bool:
     """Whether the routed rows take int4_tmem.cu rather than skinny_gemm.cu, which spreads the rows of few experts over all SMs.  us of the
-    layer there / in int4_tmem.cu: 128 experts of 2816 x 704 with 8 of them per token 30 / 35 at 8 routes, 52 / 43 at 24, 63 / 63 at 32
-    (and 1 % of a decode step more there: its start does not hide behind the kernel in front), 79 / 70 at 48, 154 / 136 at 256; 8 of 4096
-    x 1408 27 / 44 at 2, 47 / 50 at 24, 60 / 50 at 32; 16 of 4096 x 4096 111 / 134 at 16, 143 / 154 at 24, 146 / 133 at 32; 256 of 2048
-    x 1024 54 / 55 at 24, 69 / 57 at 32; 32 of 1024 x 512 18 / 24 at 24, 26 / 25 at 32."""
-    return routes >= 32 + experts // 32
+    layer there / in int4_tmem.cu: 128 experts of 2816 x 704 with 8 of them per token 28 / 38 at 8 routes, 59 / 65 at 32, 70 / 74 at 64, 95 / 88
+    at 72; 256 of 2048 x 1024 45 / 57 at 32, 100 / 115 at 120; 60 of 2048 x 1408 49 / 59 at 32, 63 / 70 at 48; 32 of 1024 x 512 21 / 25 at
+    32, 25 / 25 at 48; 16 of 4096 x 4096 109 / 127 at 24, 133 / 149 at 32; 8 of 4096 x 2048 45 / 53 at 24, of 4096 x 1408 51 / 49."""
+    return routes >= 28 + experts * 5 // 16
 
 
 def _tmem_tile(mean: int) -> int:

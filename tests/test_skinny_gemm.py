@@ -105,3 +105,32 @@ def test_experts_of_few_rows(T, E, K, H, inter):
     got = moe.fused_experts(x, gu, dn, ids, wts, E, 0, "gelu_tanh")
     ref = moe._reference_experts(x, gu, dn, ids, wts, E, 0, E, "gelu_tanh").float()
     _close(got, ref, torch.bfloat16, 6.0)
+
+
+# experts of few rows: eight, four, two warps and one per tile of their up products, one for two tiles; groups of a chunk and shorter ones
+@pytest.mark.gpu
+@pytest.mark.parametrize("group", [32, 128])
+@pytest.mark.parametrize("T,E,K", [(1, 4, 2), (1, 8, 8), (2, 32, 8), (3, 32, 8), (5, 64, 8)])
+def test_warps_of_an_experts_tile(T, E, K, group):
+    from litevllm_b200 import ops
+    from litevllm_b200.ops import moe
+    from litevllm_b200.ops.awq import Int4Weight
+    H, inter, dtype = 256, 768, torch.bfloat16
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+
+    def weight(rows, cols):
+        nib = torch.randint(0, 16, (rows, cols), generator=g, device="cuda", dtype=torch.uint8)
+        s = (torch.rand(rows, cols // group, generator=g, device="cuda") + 0.5).mul_(0.2 * cols ** -0.5).to(dtype)
+        z = torch.randint(4, 12, (rows, cols // group), generator=g, device="cuda", dtype=torch.uint8)
+        return Int4Weight(nib, s, z, group, dtype)
+    gu, dn = weight(E * 2 * inter, H), weight(E * H, inter)
+    x = torch.randn(T, H, generator=g, device="cuda").to(dtype)
+    ids = torch.rand(T, E, generator=g, device="cuda").topk(K).indices.int()
+    wts = torch.rand(T, K, generator=g, device="cuda")
+    assert not moe._tmem_pays(T * K, E)
+    got = moe.fused_experts(x, gu, dn, ids, wts, E, 0, "gelu_tanh").float()
+    ops.check_status(x.device)
+    ref = moe._reference_experts(x, gu, dn, ids, wts, E, 0, E, "gelu_tanh").float()
+    # weights, gated activations, rows and the sum are rounded to 16 bits, half an ulp each
+    assert (got - ref).norm() <= 2 * 2.0 ** -8 * ref.norm()
+    assert (got - ref).abs().max() <= 8 * 2.0 ** -8 * ref.abs().max()
