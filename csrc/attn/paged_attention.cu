@@ -6,7 +6,8 @@
 // KV cache layout: [num_blocks, n_kv_heads, block_size, head_dim]; block id 0 is the null block.
 //
 // These are bandwidth-bound (decode) or a small share of prefill FLOPs for the served shapes, so
-// they use register-level mma.sync tiles with cp.async double buffering rather than TMEM.
+// they use register-level mma.sync tiles with cp.async double buffering rather than TMEM.  Prefill of heads of 64 and 128
+// channels on 16-bit caches is in prefill_tc.cu, of 256 on e4m3 caches in prefill_fp8.cu.
 //
 // Counterpart in the reference: vllm/kernels/triton/paged_attention.py:306-759 (one program per
 // (sequence, query head), also used for prefill by expanding every query token into its own row,

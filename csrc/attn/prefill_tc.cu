@@ -17,6 +17,9 @@
 //            then fold PV of the previous tile into the row's fp32 output registers
 //            (o = o * alpha + PV) so TMEM never has to be rescaled
 //
+// Where there are more such tiles than SMs a CTA takes two of them (prefill_pair_kernel below), so that one tile's softmax fills the
+// other's waits.
+//
 // With two maps per head (MAPS = 2) the 128 rows are 64 tokens times the two maps of one head, side by side: query rows
 // [q1 | 0] and [0 | q2] against key rows [k1 | k2] share every K and V tile, and the epilogue takes the difference of
 // neighbouring rows, its norm over the head's channels and the scale before it stores.
