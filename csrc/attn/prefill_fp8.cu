@@ -371,6 +371,7 @@ extern "C" int fi_paged_prefill_fp8(const void* q, long q_stride, const void* k_
   if (B <= 0 || max_q_len <= 0 || T_total <= 0) return 0;
   if (nkv <= 0 || nh <= 0 || nh % nkv != 0) return -10;
   if (hd != kHd || (dtype != 0 && dtype != 1)) return -12;
+  if (!(sm_scale * k_scale > 0.f)) return -12;      // the largest raw product is taken for the largest score
   if (block_size != 16 && block_size != 32 && block_size % 64 != 0) return -12;
   if ((reinterpret_cast<uintptr_t>(q) & 15) != 0 || (q_stride * 2) % 16 != 0 || (reinterpret_cast<uintptr_t>(out) & 15) != 0) return -12;
   CUtensorMap qm, km, vm;
